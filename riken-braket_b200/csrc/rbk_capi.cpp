@@ -38,6 +38,8 @@ struct rbk_state {
   float* d_tc_w = nullptr;   // W_hi, W_lo of the tensor-core unitaries (largest k), kept between calls
   int* d_tc_flag = nullptr;  // set by a tensor-core unitary whose bounded wait ran out (sticky)
   int* h_tc_flag = nullptr;  // pinned copy, read at every bounded_sync
+  double* d_sample = nullptr;  // workspace of the sampling calls (sample_workspace)
+  size_t sample_bytes = 0;
   std::vector<int> perm, inv;
   std::vector<hgate> queue;
   bool deferred = true;
@@ -514,6 +516,7 @@ int rbk_state_destroy(rbk_state* s)
   if (s->d_partials) cudaFree(s->d_partials);
   if (s->d_out) cudaFree(s->d_out);
   if (s->h_out) cudaFreeHost(s->h_out);
+  if (s->d_sample) cudaFree(s->d_sample);
   if (s->d_tc_w) cudaFree(s->d_tc_w);
   if (s->d_tc_flag) cudaFree(s->d_tc_flag);
   if (s->h_tc_flag) cudaFreeHost(s->h_tc_flag);
@@ -1958,21 +1961,27 @@ double random_upto(std::mt19937_64& g, double maximum)
   return d(g);
 }
 
-// Inclusive prefix sums of |a_i|^2 in logical order, plus the total.
-int prob_prefix(rbk_state* s, device_buffer& prefix, device_buffer& scratch, double* total)
+// Device workspace of the sampling calls: kept in the state up to
+// kSampleKeptBytes (29 qubits), so that repeated calls allocate nothing;
+// above that the call's own, since a state that large leaves little room.
+constexpr size_t kSampleKeptBytes = size_t(40) << 20;
+
+int sample_workspace(rbk_state* s, size_t doubles, device_buffer& own, double** out)
 {
-  if (int rc = canonicalize(s)) return rc;
-  device_guard g(s->device);
-  const uint64_t size = 1ull << s->n;
-  RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&prefix.p), sizeof(double) * size));
-  RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&scratch.p), sizeof(double) * rbk::scan_scratch_doubles(size)));
-  const cudaError_t e = s->precision == RBK_C128 ? rbk::launch_prob_scan<double>(s->amps, size, prefix.p, scratch.p, s->stream)
-                                                : rbk::launch_prob_scan<float>(s->amps, size, prefix.p, scratch.p, s->stream);
-  if (e != cudaSuccess) return cuda_fail(e, "probability scan");
-  s->stats.kernel_launches += 2;
-  RBK_CUDA(cudaMemcpyAsync(s->h_out, prefix.p + (size - 1), sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-  if (int rc = bounded_sync(s)) return rc;
-  *total = s->h_out[0];
+  const size_t bytes = sizeof(double) * doubles;
+  if (bytes > kSampleKeptBytes) {
+    RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&own.p), bytes));
+    *out = own.p;
+    return RBK_OK;
+  }
+  if (s->sample_bytes < bytes) {
+    if (s->d_sample) cudaFree(s->d_sample);
+    s->d_sample = nullptr;
+    s->sample_bytes = 0;
+    RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&s->d_sample), bytes));
+    s->sample_bytes = bytes;
+  }
+  *out = s->d_sample;
   return RBK_OK;
 }
 
@@ -1980,22 +1989,30 @@ int prob_prefix(rbk_state* s, device_buffer& prefix, device_buffer& scratch, dou
 template <typename Draw>
 int sample_indices(rbk_state* s, Draw&& draw, int num, uint64_t* out)
 {
-  device_buffer prefix, scratch, rbuf;
-  double total = 0;
-  if (int rc = prob_prefix(s, prefix, scratch, &total)) return rc;
+  if (int rc = canonicalize(s)) return rc;
+  device_guard g(s->device);
+  device_buffer own;
+  double* work = nullptr;
+  const size_t sums = rbk::sample_scratch_doubles(s->n);
+  if (int rc = sample_workspace(s, sums + 2 * static_cast<size_t>(num), own, &work)) return rc;
+  const bool c128 = s->precision == RBK_C128;
+  const double* d_total = nullptr;
+  RBK_CUDA(c128 ? rbk::launch_sample_sums<double>(s->amps, s->n, work, &d_total, s->stream)
+                : rbk::launch_sample_sums<float>(s->amps, s->n, work, &d_total, s->stream));
+  s->stats.kernel_launches += s->n > 12 ? 2 : 1;
+  RBK_CUDA(cudaMemcpyAsync(s->h_out, d_total, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+  if (int rc = bounded_sync(s)) return rc;
+  const double total = s->h_out[0];
   std::vector<double> r(num);
   for (auto& x : r) x = draw(total);
-  RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&rbuf.p), sizeof(double) * 2 * num));
-  uint64_t* ev = reinterpret_cast<uint64_t*>(rbuf.p + num);
-  RBK_CUDA(cudaMemcpyAsync(rbuf.p, r.data(), sizeof(double) * num, cudaMemcpyHostToDevice, s->stream));
-  RBK_CUDA(rbk::launch_upper_bound(prefix.p, 1ull << s->n, rbuf.p, num, ev, s->stream));
+  double* d_r = work + sums;
+  uint64_t* ev = reinterpret_cast<uint64_t*>(d_r + num);
+  RBK_CUDA(cudaMemcpyAsync(d_r, r.data(), sizeof(double) * num, cudaMemcpyHostToDevice, s->stream));
+  RBK_CUDA(c128 ? rbk::launch_sample<double>(s->amps, s->n, work, d_r, num, ev, s->stream)
+                : rbk::launch_sample<float>(s->amps, s->n, work, d_r, num, ev, s->stream));
   ++s->stats.kernel_launches;
   RBK_CUDA(cudaMemcpyAsync(out, ev, sizeof(uint64_t) * num, cudaMemcpyDeviceToHost, s->stream));
-  if (int rc = bounded_sync(s)) return rc;
-  // upper_bound can land past the end only when r reaches the total (rounding); clamp like the last bin.
-  const uint64_t last = (1ull << s->n) - 1;
-  for (int k = 0; k < num; ++k) if (out[k] > last) out[k] = last;
-  return RBK_OK;
+  return bounded_sync(s);
 }
 
 }  // namespace

@@ -1643,38 +1643,78 @@ template cudaError_t launch_overlap<float>(const void*, const void*, int, uint64
 namespace rbk {
 
 // ---------------------------------------------------------------------------
-// Sampling: inclusive prefix sums of |a_i|^2 and upper_bound searches
-// (the device form of ket::generate_events, ket/include/ket/generate_events.hpp:18-51)
+// Sampling: the device form of ket::generate_events
+// (ket/include/ket/generate_events.hpp:18-51), the upper_bound of a random
+// value among the inclusive prefix sums of |a_i|^2.
+//
+// The prefix sums are kept at two levels only: one sum per block of
+// 2^kSampleBlockLog amplitudes and the scanned sums of chunks of
+// 2^kSampleChunkLog amplitudes.  A sample searches the chunks, then the 32
+// block sums of its chunk, then re-reads the 128 amplitudes of its block.  The
+// state is read once and 8 bytes are written per 128 amplitudes, so the call
+// is bound by that read; a prefix value per amplitude wrote and re-read 24
+// bytes for each and needed half the state's size of scratch (26 qubits
+// complex<double>: 0.74 ms of scans, 0.4 to 3 ms more for allocating and
+// freeing 512 MB; now 0.2 ms).
 // ---------------------------------------------------------------------------
-constexpr int kScanThreads = 256;
-constexpr int kScanPerThread = 16;
-constexpr int kScanChunk = kScanThreads * kScanPerThread;  // values per block
+constexpr int kSampleBlockLog = 7;   // 32 lanes x 4 amplitudes
+constexpr int kSampleChunkLog = 12;  // 32 blocks: one per lane
+constexpr int kSampleWarps = 4;
 
-// One block scans kScanChunk consecutive values: out[i] = sum_{j<=i in chunk} v[j],
-// and writes the chunk total to sums[block].  v = |a_i|^2 when amps != nullptr,
-// else v = in[i].
+// One warp per chunk: sums[b] = sum of |a|^2 over block b (0 for blocks past the
+// end of a state smaller than a chunk), chunk_sums[c] = their sum.
 template <typename Real>
-__global__ void __launch_bounds__(kScanThreads)
-chunk_scan_kernel(const typename ctype<Real>::c* __restrict__ amps, const double* __restrict__ in, uint64_t count,
-                  double* __restrict__ out, double* __restrict__ sums)
+__global__ void __launch_bounds__(kSampleWarps * 32)
+sample_sums_kernel(const typename ctype<Real>::c* __restrict__ a, uint64_t size, uint64_t chunks, double* __restrict__ sums,
+                   double* __restrict__ chunk_sums)
 {
-  __shared__ double warp_tot[kScanThreads / 32];
-  const uint64_t base = uint64_t(blockIdx.x) * kScanChunk + uint64_t(threadIdx.x) * kScanPerThread;
-  double v[kScanPerThread];
-  double run = 0;
+  using C = typename ctype<Real>::c;
+  constexpr int kGroup = 4;  // blocks whose loads are in flight together
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t c = uint64_t(blockIdx.x) * kSampleWarps + (threadIdx.x >> 5);
+  if (c >= chunks) return;
+  const uint64_t base = c << kSampleChunkLog;
+  double mine = 0.0;  // lane l: the sum of block l
+  for (int g = 0; g < 32; g += kGroup) {
+    C v[kGroup][4];
 #pragma unroll
-  for (int k = 0; k < kScanPerThread; ++k) {
-    const uint64_t i = base + k;
-    double x = 0;
-    if (i < count) {
-      if (amps) { const auto a = amps[i]; x = double(a.x) * double(a.x) + double(a.y) * double(a.y); }
-      else x = in[i];
+    for (int b = 0; b < kGroup; ++b)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint64_t i = base + (uint64_t(g + b) << kSampleBlockLog) + uint64_t(k * 32) + lane;
+        v[b][k] = i < size ? __ldcs(a + i) : C{Real(0), Real(0)};
+      }
+#pragma unroll
+    for (int b = 0; b < kGroup; ++b) {
+      double p = 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) p += double(v[b][k].x) * double(v[b][k].x) + double(v[b][k].y) * double(v[b][k].y);
+      p = warp_sum(p);
+      if (lane == uint32_t(g + b)) mine = p;
     }
-    run += x;
-    v[k] = run;
   }
-  // exclusive scan of the per-thread totals over the block
+  sums[(c << (kSampleChunkLog - kSampleBlockLog)) + lane] = mine;
+  // The chunk's sum as the inclusive scan that sample_kernel forms: its last lane.
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, mine, o);
+    if (lane >= uint32_t(o)) mine += y;
+  }
+  if (lane == 31) chunk_sums[c] = mine;
+}
+
+// Inclusive scan of v[0..count) in place by one block: thread t sums and then
+// rewrites its own run of consecutive values.  At most 2^21 chunks (33 qubits).
+constexpr int kSampleScanThreads = 1024;
+__global__ void __launch_bounds__(kSampleScanThreads) sample_scan_kernel(double* __restrict__ v, uint64_t count)
+{
+  __shared__ double warp_tot[kSampleScanThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t per = (count + kSampleScanThreads - 1) / kSampleScanThreads;
+  const uint64_t lo = min(count, threadIdx.x * per), hi = min(count, lo + per);
+  double run = 0.0;
+#pragma unroll 8
+  for (uint64_t i = lo; i < hi; ++i) run += v[i];
   double incl = run;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -1683,100 +1723,132 @@ chunk_scan_kernel(const typename ctype<Real>::c* __restrict__ amps, const double
   }
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
-  double warp_off = 0, block_tot = 0;
-  for (int w = 0; w < kScanThreads / 32; ++w) {
-    if (w < warp) warp_off += warp_tot[w];
-    block_tot += warp_tot[w];
-  }
-  const double off = warp_off + (incl - run);
-#pragma unroll
-  for (int k = 0; k < kScanPerThread; ++k) {
-    const uint64_t i = base + k;
-    if (i < count) out[i] = v[k] + off;
-  }
-  if (threadIdx.x == 0 && sums) sums[blockIdx.x] = block_tot;
-}
-
-// out[i] += offsets[block of i - 1] (offsets = inclusive scan of the chunk totals)
-__global__ void add_offsets_kernel(double* __restrict__ out, uint64_t count, const double* __restrict__ offsets)
-{
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < count; i += stride) {
-    const uint64_t chunk = i / kScanChunk;
-    if (chunk > 0) out[i] += offsets[chunk - 1];
+  double off = 0.0;
+  for (int w = 0; w < warp; ++w) off += warp_tot[w];
+  // The start of a run is the end of the one before it, bit for bit, so that the
+  // scanned values never decrease from one thread's run to the next.
+  double before = __shfl_up_sync(0xffffffffu, incl, 1);
+  if (lane == 0) before = 0.0;
+  double acc = off + before;
+  const double end = off + incl;
+#pragma unroll 8
+  for (uint64_t i = lo; i < hi; ++i) {
+    acc += v[i];
+    v[i] = i + 1 == hi ? end : min(acc, end);
   }
 }
 
-// events[k] = first index i with prefix[i] > r[k]  (std::upper_bound)
-__global__ void upper_bound_kernel(const double* __restrict__ prefix, uint64_t count, const double* __restrict__ r,
-                                   int num, uint64_t* __restrict__ events)
+// One warp per sample: events[k] = first index whose prefix sum exceeds r[k].
+// Where rounding between the levels leaves no such entry inside the chunk or
+// block that a search chose, its last entry of non-zero weight is taken, so an
+// amplitude of weight zero is never drawn.  r[k] at or above the last prefix
+// sum (rounding) gives the last index, as does a state whose sums are NaN.
+template <typename Real>
+__global__ void __launch_bounds__(kSampleWarps * 32)
+sample_kernel(const typename ctype<Real>::c* __restrict__ a, uint64_t size, uint64_t chunks, const double* __restrict__ sums,
+              const double* __restrict__ prefix, const double* __restrict__ r, int num, uint64_t* __restrict__ events)
 {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int k = blockIdx.x * kSampleWarps + (threadIdx.x >> 5);
   if (k >= num) return;
   const double x = r[k];
-  uint64_t lo = 0, hi = count;
-  while (lo < hi) {
-    const uint64_t mid = lo + ((hi - lo) >> 1);
-    if (prefix[mid] > x) hi = mid;
-    else lo = mid + 1;
+  // First chunk whose prefix exceeds x, by a 32-way search: lane l looks at the end of the l-th part.
+  uint64_t lo = 0, hi = chunks;
+  while (hi - lo > 1) {
+    const uint64_t step = (hi - lo + 31) / 32;
+    const uint64_t end = min(hi, lo + uint64_t(lane + 1) * step);
+    const uint32_t over = __ballot_sync(0xffffffffu, prefix[end - 1] > x);
+    const uint64_t part = over ? uint64_t(__ffs(static_cast<int>(over)) - 1) : 31;
+    const uint64_t nlo = min(hi - 1, lo + part * step);
+    hi = min(hi, nlo + step);
+    lo = nlo;
   }
-  events[k] = lo;
+  if (!(prefix[lo] > x)) {
+    if (lane == 0) events[k] = size - 1;
+    return;
+  }
+  // The block of the chunk: lane l holds block l.
+  double base = lo > 0 ? prefix[lo - 1] : 0.0;
+  const double s = sums[(lo << (kSampleChunkLog - kSampleBlockLog)) + uint64_t(lane)];
+  double incl = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  uint32_t over = __ballot_sync(0xffffffffu, base + incl > x && s > 0.0);
+  uint32_t some = __ballot_sync(0xffffffffu, s > 0.0);
+  const int blk = over ? __ffs(static_cast<int>(over)) - 1 : some ? 31 - __clz(static_cast<int>(some)) : 0;
+  const double upto = __shfl_sync(0xffffffffu, incl, blk > 0 ? blk - 1 : 0);
+  if (blk > 0) base += upto;
+  // The amplitude: lane l holds the four consecutive ones from 4 l.
+  const uint64_t first = (lo << kSampleChunkLog) + (uint64_t(blk) << kSampleBlockLog) + uint64_t(4 * lane);
+  double p[4], tot = 0.0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    p[j] = 0.0;
+    if (first + j < size) {
+      const auto v = a[first + j];
+      p[j] = double(v.x) * double(v.x) + double(v.y) * double(v.y);
+    }
+    tot += p[j];
+  }
+  incl = tot;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  double run = __shfl_up_sync(0xffffffffu, incl, 1);
+  run = base + (lane > 0 ? run : 0.0);
+  int hit = -1, last = -1;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    run += p[j];
+    if (p[j] > 0.0) {
+      last = j;
+      if (hit < 0 && run > x) hit = j;
+    }
+  }
+  over = __ballot_sync(0xffffffffu, hit >= 0);
+  some = __ballot_sync(0xffffffffu, last >= 0);
+  const int src = over ? __ffs(static_cast<int>(over)) - 1 : some ? 31 - __clz(static_cast<int>(some)) : 0;
+  if (lane == src) events[k] = min(size - 1, first + uint64_t(over ? hit : some ? last : 0));
 }
 
-size_t scan_scratch_doubles(uint64_t count)
-{
-  size_t total = 0;
-  uint64_t m = count;
-  while (m > 1) {
-    m = (m + kScanChunk - 1) / kScanChunk;
-    total += m;
-  }
-  return total + 1;
-}
+static uint64_t sample_chunks(int n) { return n > kSampleChunkLog ? 1ull << (n - kSampleChunkLog) : 1; }
 
-// Inclusive scan of |a|^2 (level 0) with the chunk totals scanned recursively in `scratch`.
+// Block sums, then chunk prefixes.
+size_t sample_scratch_doubles(int n) { return sample_chunks(n) * ((1u << (kSampleChunkLog - kSampleBlockLog)) + 1); }
+
+// scratch: sample_scratch_doubles(n) doubles; *total points at the sum of |a|^2 in it.
 template <typename Real>
-cudaError_t launch_prob_scan(const void* amps, uint64_t count, double* prefix, double* scratch, cudaStream_t stream)
+cudaError_t launch_sample_sums(const void* amps, int n, double* scratch, const double** total, cudaStream_t stream)
 {
-  // level list: (values, count, out, sums)
-  const double* in = nullptr;
-  const void* a = amps;
-  double* out = prefix;
-  uint64_t m = count;
-  double* level_out[64];
-  uint64_t level_count[64];
-  int levels = 0;
-  double* s = scratch;
-  while (true) {
-    const uint64_t blocks = (m + kScanChunk - 1) / kScanChunk;
-    double* sums = blocks > 1 ? s : nullptr;
-    if (a) chunk_scan_kernel<Real><<<(unsigned)blocks, kScanThreads, 0, stream>>>(static_cast<const typename ctype<Real>::c*>(a), nullptr, m, out, sums);
-    else chunk_scan_kernel<double><<<(unsigned)blocks, kScanThreads, 0, stream>>>(nullptr, in, m, out, sums);
-    level_out[levels] = out;
-    level_count[levels] = m;
-    ++levels;
-    if (blocks <= 1) break;
-    // scan the chunk totals in place: next level reads `sums`, writes into the same array
-    in = sums;
-    a = nullptr;
-    out = sums;
-    m = blocks;
-    s += blocks;
-  }
-  for (int l = levels - 2; l >= 0; --l) {
-    add_offsets_kernel<<<grid_for(level_count[l], 256), 256, 0, stream>>>(level_out[l], level_count[l], level_out[l + 1]);
-  }
+  const uint64_t chunks = sample_chunks(n);
+  double* prefix = scratch + (chunks << (kSampleChunkLog - kSampleBlockLog));
+  sample_sums_kernel<Real><<<(unsigned)((chunks + kSampleWarps - 1) / kSampleWarps), kSampleWarps * 32, 0, stream>>>(
+    static_cast<const typename ctype<Real>::c*>(amps), 1ull << n, chunks, scratch, prefix);
+  if (chunks > 1) sample_scan_kernel<<<1, kSampleScanThreads, 0, stream>>>(prefix, chunks);
+  *total = prefix + (chunks - 1);
   return cudaGetLastError();
 }
 
-cudaError_t launch_upper_bound(const double* prefix, uint64_t count, const double* r, int num, uint64_t* events, cudaStream_t stream)
+template <typename Real>
+cudaError_t launch_sample(const void* amps, int n, const double* scratch, const double* r, int num, uint64_t* events,
+                          cudaStream_t stream)
 {
-  upper_bound_kernel<<<(num + 255) / 256, 256, 0, stream>>>(prefix, count, r, num, events);
+  const uint64_t chunks = sample_chunks(n);
+  sample_kernel<Real><<<(num + kSampleWarps - 1) / kSampleWarps, kSampleWarps * 32, 0, stream>>>(
+    static_cast<const typename ctype<Real>::c*>(amps), 1ull << n, chunks, scratch,
+    scratch + (chunks << (kSampleChunkLog - kSampleBlockLog)), r, num, events);
   return cudaGetLastError();
 }
 
-template cudaError_t launch_prob_scan<double>(const void*, uint64_t, double*, double*, cudaStream_t);
-template cudaError_t launch_prob_scan<float>(const void*, uint64_t, double*, double*, cudaStream_t);
+template cudaError_t launch_sample_sums<double>(const void*, int, double*, const double**, cudaStream_t);
+template cudaError_t launch_sample_sums<float>(const void*, int, double*, const double**, cudaStream_t);
+template cudaError_t launch_sample<double>(const void*, int, const double*, const double*, int, uint64_t*, cudaStream_t);
+template cudaError_t launch_sample<float>(const void*, int, const double*, const double*, int, uint64_t*, cudaStream_t);
 
 }  // namespace rbk
 

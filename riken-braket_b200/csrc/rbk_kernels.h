@@ -190,13 +190,14 @@ template <typename Real> cudaError_t launch_zsum2(const void* lam, const void* p
 template <typename Real> cudaError_t launch_pair_overlaps(const void* lam, const void* psi, int n, const pair_overlap_set& set,
                                                           double* partials, double* out, cudaStream_t stream);
 
-// Sampling: prefix = inclusive scan of |a_i|^2 (scratch: scan_scratch_doubles(count)
-// doubles); events[k] = upper_bound(prefix, r[k]).
-size_t scan_scratch_doubles(uint64_t count);
-template <typename Real> cudaError_t launch_prob_scan(const void* amps, uint64_t count, double* prefix, double* scratch,
-                                                      cudaStream_t stream);
-cudaError_t launch_upper_bound(const double* prefix, uint64_t count, const double* r, int num, uint64_t* events,
-                               cudaStream_t stream);
+// Sampling: block sums and chunk prefixes of |a_i|^2 in scratch
+// (sample_scratch_doubles(n) doubles; *total: device address of the sum over the
+// state), then events[k] = upper_bound of r[k] among the prefix sums.
+size_t sample_scratch_doubles(int n);
+template <typename Real> cudaError_t launch_sample_sums(const void* amps, int n, double* scratch, const double** total,
+                                                        cudaStream_t stream);
+template <typename Real> cudaError_t launch_sample(const void* amps, int n, const double* scratch, const double* r, int num,
+                                                   uint64_t* events, cudaStream_t stream);
 
 // Dense k-qubit unitaries.
 // Tensor cores (complex<float>, k = 5 or 6, n >= k + 7): w_split holds W_hi then
