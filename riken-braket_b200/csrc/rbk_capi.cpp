@@ -428,6 +428,180 @@ int group_pauli_terms(const rbk_state* s, int num_terms, const char* strings, co
   return RBK_OK;
 }
 
+// Sums read from the state by observe_all: x[b] = sum over the pairs of physical
+// bit b of conj(a0) a1 for the bits asked for; with z, sum |a|^2 in all and over
+// each bit set; diag = sum |a|^2 W of the Z-type strings given.
+struct observed {
+  double x[rbk::kMaxQubits][2] = {};
+  double total = 0.0, z[rbk::kMaxQubits] = {};
+  double diag = 0.0;
+};
+
+// A Z-type string on physical bits with its real weight.
+struct diag_term { uint64_t sign; double w; };
+
+// The tile layout over `bits` (ascending) as the run-by-run deposit of the other bits.
+template <typename Group>
+void fill_tile(Group& g, const std::vector<int>& bits, int n)
+{
+  uint64_t mask = 0;
+  g.K = static_cast<int>(bits.size());
+  for (size_t b = 0; b < bits.size(); ++b) {
+    g.tile_phys[b] = static_cast<uint8_t>(bits[b]);
+    mask |= 1ull << bits[b];
+  }
+  int runs = 0, src = 0;
+  for (int q = 0; q < n;) {
+    if ((mask >> q) & 1) { ++q; continue; }
+    int len = 0;
+    while (q + len < n && !((mask >> (q + len)) & 1)) ++len;
+    g.run_src[runs] = static_cast<uint8_t>(src);
+    g.run_len[runs] = static_cast<uint8_t>(len);
+    g.run_dst[runs] = static_cast<uint8_t>(q);
+    ++runs;
+    src += len;
+    q += len;
+  }
+  g.num_runs = runs;
+}
+
+// The diagonal strings [first, first + count) as classes of one weight and one
+// pattern on the layout's register bits.
+void fill_diag(rbk::observe_group& g, int reg_bits, const std::vector<diag_term>& terms, size_t first, size_t count)
+{
+  g.diag_terms = static_cast<int>(count);
+  struct cls { int pattern; double w; uint64_t mask; };
+  std::vector<cls> classes;
+  for (size_t k = 0; k < count; ++k) {
+    const diag_term& t = terms[first + k];
+    g.sign[k] = t.sign;
+    int pattern = 0;
+    for (int b = 0; b < reg_bits; ++b) pattern |= static_cast<int>((t.sign >> g.tile_phys[8 + b]) & 1) << b;
+    g.sign[k] = t.sign;
+    bool found = false;
+    for (cls& c : classes)
+      if (c.pattern == pattern && c.w == t.w) { c.mask |= 1ull << k; found = true; break; }
+    if (!found) classes.push_back({pattern, t.w, 1ull << k});
+  }
+  std::stable_sort(classes.begin(), classes.end(), [](const cls& a, const cls& b) { return a.pattern < b.pattern; });
+  g.diag_classes = static_cast<int>(classes.size());
+  for (size_t c = 0; c < classes.size(); ++c) {
+    g.class_mask[c] = classes[c].mask;
+    g.class_w[c] = classes[c].w;
+  }
+  size_t at = 0;
+  for (int p = 0; p <= (1 << reg_bits); ++p) {
+    while (at < classes.size() && classes[at].pattern < p) ++at;
+    g.class_begin[p] = static_cast<uint8_t>(at);
+  }
+}
+
+// flips: the physical bits whose x is wanted.  Few tiled reads of the state
+// (rbk::launch_observe) and one read-back: the first layout holds the low bits
+// and takes the sums of |a|^2, the further ones the coalescing bits (128-byte
+// runs) and as many flipped bits as the tile has left.  z or diag, not both.
+int observe_all(rbk_state* s, uint64_t flips, bool z, const std::vector<diag_term>& diag, observed& out)
+{
+  if (int rc = flush(s)) return rc;  // the layout map is final only after the queued gates ran
+  const bool c128 = s->precision == RBK_C128;
+  const int n = s->n, RB = rbk::kObserveRegBits, KT = rbk::kObserveTileBits;
+  if (n < KT) {
+    for (size_t first = 0; first == 0 || first < diag.size(); first += rbk::kMaxPauliTerms) {
+      rbk::pauli_terms t{};
+      for (size_t k = first; k < diag.size() && t.count < rbk::kMaxPauliTerms; ++k) {
+        t.sign[t.count] = diag[k].sign;
+        t.w[t.count++][0] = diag[k].w;
+      }
+      int rc = launch_reduction(s, [&] {
+        return c128 ? rbk::launch_observe_small<double>(s->amps, n, t, s->d_out, s->stream)
+                    : rbk::launch_observe_small<float>(s->amps, n, t, s->d_out, s->stream);
+      });
+      if (rc) return rc;
+      if ((rc = read_out(s, 3 * n + 2))) return rc;
+      for (int b = 0; b < n; ++b) {
+        out.x[b][0] = s->h_out[2 * b];
+        out.x[b][1] = s->h_out[2 * b + 1];
+        out.z[b] = s->h_out[2 * n + 1 + b];
+      }
+      out.total = s->h_out[2 * n];
+      out.diag += s->h_out[3 * n + 1];
+    }
+    return RBK_OK;
+  }
+  const int low = c128 ? 3 : 4;
+  std::vector<rbk::observe_group> groups;
+  auto add = [&](const std::vector<int>& bits, uint64_t wanted) {
+    rbk::observe_group g{};
+    fill_tile(g, bits, n);
+    for (int b = 0; b < KT; ++b)
+      if ((wanted >> g.tile_phys[b]) & 1) g.flip_mask |= 1 << b;
+    groups.push_back(g);
+  };
+  const uint64_t first_bits = (1ull << KT) - 1;
+  if (z || !diag.empty() || (flips & first_bits)) {
+    std::vector<int> bits;
+    for (int b = 0; b < KT; ++b) bits.push_back(b);
+    add(bits, flips & first_bits);
+    groups.back().zsums = z ? 1 : 0;
+  }
+  std::vector<int> high;
+  for (int b = KT; b < n; ++b)
+    if ((flips >> b) & 1) high.push_back(b);
+  for (size_t h = 0; h < high.size(); h += static_cast<size_t>(KT - low)) {
+    std::vector<int> bits;
+    uint64_t wanted = 0;
+    for (int b = 0; b < low; ++b) bits.push_back(b);
+    for (size_t k = h; k < high.size() && k < h + static_cast<size_t>(KT - low); ++k) {
+      bits.push_back(high[k]);
+      wanted |= 1ull << high[k];
+    }
+    for (int b = low; static_cast<int>(bits.size()) < KT; ++b)  // fillers: the bits after the coalescing ones
+      if (!((wanted >> b) & 1)) bits.push_back(b);
+    std::sort(bits.begin(), bits.end());
+    add(bits, wanted);
+  }
+  // More strings than one launch takes: further diagonal-only reads of the first layout.
+  for (size_t first = 0; first < diag.size(); first += rbk::kObserveTerms) {
+    if (first > 0) {
+      std::vector<int> bits;
+      for (int b = 0; b < KT; ++b) bits.push_back(b);
+      add(bits, 0);
+    }
+    fill_diag(first > 0 ? groups.back() : groups.front(), RB, diag, first, std::min<size_t>(rbk::kObserveTerms, diag.size() - first));
+  }
+  constexpr int kOut = 4 * (rbk::kMaxQubits + 8);
+  for (size_t g0 = 0; g0 < groups.size();) {
+    int width = 0;
+    size_t g1 = g0;
+    for (; g1 < groups.size() && width + rbk::observe_width(groups[g1], n) <= kOut; ++g1) {
+      int rc = launch_reduction(s, [&] {
+        return c128 ? rbk::launch_observe<double>(s->amps, n, groups[g1], s->d_partials, s->d_out + width, s->stream)
+                    : rbk::launch_observe<float>(s->amps, n, groups[g1], s->d_partials, s->d_out + width, s->stream);
+      });
+      if (rc) return rc;
+      width += rbk::observe_width(groups[g1], n);
+    }
+    if (int rc = read_out(s, width)) return rc;
+    int at = 0;
+    for (; g0 < g1; ++g0) {
+      const rbk::observe_group& g = groups[g0];
+      for (int b = 0; b < KT; ++b) {
+        if (!((g.flip_mask >> b) & 1)) continue;
+        out.x[g.tile_phys[b]][0] = s->h_out[at];
+        out.x[g.tile_phys[b]][1] = s->h_out[at + 1];
+        at += 2;
+      }
+      if (g.zsums) {
+        out.total = s->h_out[at];
+        for (int b = 0; b < n; ++b) out.z[b] = s->h_out[at + 1 + b];
+        at += 1 + n;
+      }
+      if (g.diag_classes > 0) out.diag += s->h_out[at++];
+    }
+  }
+  return RBK_OK;
+}
+
 // sum over one flip-mask group of Pauli terms (physical masks).
 int pauli_group(rbk_state* s, uint64_t flip, const rbk::pauli_terms& t, double* out2)
 {
@@ -962,124 +1136,13 @@ int rbk_spin_expectation_values(rbk_state* s, double* out)
   return guarded([&]() -> int {
     if (int rc = check_state(s)) return rc;
     if (!out) return fail(RBK_ERR_INVALID, "null output pointer");
-    if (int rc = flush(s)) return rc;  // the layout map is final only after the queued gates ran
-    const bool c128 = s->precision == RBK_C128;
-    const int n = s->n, RB = rbk::spin_register_bits(c128 ? 0 : 1), KT = 8 + RB;
-    if (n < KT) {
-      // Small states: one Z-sum pass and one pair-sum pass per qubit.
-      int rc = launch_reduction(s, [&] {
-        return c128 ? rbk::launch_zsum<double>(s->amps, n, s->d_partials, s->d_out, s->stream)
-                    : rbk::launch_zsum<float>(s->amps, n, s->d_partials, s->d_out, s->stream);
-      });
-      if (rc) return rc;
-      if ((rc = read_out(s, n + 1))) return rc;
-      const double total = s->h_out[0];
-      std::vector<double> ones(static_cast<size_t>(n));
-      for (int p = 0; p < n; ++p) ones[static_cast<size_t>(p)] = s->h_out[1 + p];
-      for (int q = 0; q < n; ++q) {
-        const double one = ones[static_cast<size_t>(s->perm[q])];
-        out[3 * q + 2] = 0.5 * ((total - one) - one);
-        rbk::pauli_terms t{};
-        t.count = 1;
-        t.w[0][0] = 1.0;
-        t.one_sided = 1;  // <S_x> + i <S_y> = sum over pairs with the qubit clear of conj(a0) a1
-        double r[2];
-        if ((rc = pauli_group(s, 1ull << s->perm[q], t, r))) return rc;
-        out[3 * q + 0] = r[0];
-        out[3 * q + 1] = r[1];
-      }
-      return RBK_OK;
-    }
-    // Tile layouts of KT bits whose flips cover every physical bit once: the
-    // low KT bits, then the coalescing bits 0..LOW-1 with up to KT - LOW
-    // further bits (filled up with other bits when fewer remain).  Each layout
-    // is one read of the state (spins_kernel) for all its flips.
-    const int LOW = c128 ? rbk::precision_traits<double>::LOW : rbk::precision_traits<float>::LOW;
-    std::vector<rbk::spin_group> groups;
-    std::vector<std::vector<int>> group_flips;  // physical bits flipped by each group, in flip order
-    auto add_group = [&](const std::vector<int>& tile_bits, const std::vector<int>& flips_local) {
-      rbk::spin_group g{};
-      g.K = KT;
-      uint64_t mask = 0;
-      for (int b = 0; b < KT; ++b) { g.tile_phys[b] = static_cast<uint8_t>(tile_bits[b]); mask |= 1ull << tile_bits[b]; }
-      g.nflips = static_cast<int>(flips_local.size());
-      g.nphases = (g.nflips + RB - 1) / RB;
-      std::vector<int> phys;
-      for (int p = 0; p < g.nphases; ++p) {
-        std::vector<int> regs;
-        for (int k = 0; k < RB; ++k) {
-          const int f = p * RB + k;
-          if (f < g.nflips) regs.push_back(flips_local[static_cast<size_t>(f)]);
-        }
-        for (int b = 0; static_cast<int>(regs.size()) < RB; ++b)  // fillers: other tile bits
-          if (std::find(regs.begin(), regs.end(), b) == regs.end()) regs.push_back(b);
-        int nt = 0;
-        for (int b = 0; b < KT; ++b)
-          if (std::find(regs.begin(), regs.end(), b) == regs.end()) g.phase_thr[p][nt++] = static_cast<uint8_t>(b);
-        for (int k = 0; k < RB; ++k) g.phase_reg[p][k] = static_cast<uint8_t>(regs[static_cast<size_t>(k)]);
-      }
-      for (int f : flips_local) phys.push_back(tile_bits[static_cast<size_t>(f)]);
-      int runs = 0, src = 0;
-      for (int q = 0; q < n;) {
-        if ((mask >> q) & 1) { ++q; continue; }
-        int len = 0;
-        while (q + len < n && !((mask >> (q + len)) & 1)) ++len;
-        g.run_src[runs] = static_cast<uint8_t>(src);
-        g.run_len[runs] = static_cast<uint8_t>(len);
-        g.run_dst[runs] = static_cast<uint8_t>(q);
-        ++runs;
-        src += len;
-        q += len;
-      }
-      g.num_runs = runs;
-      groups.push_back(g);
-      group_flips.push_back(phys);
-    };
-    {
-      std::vector<int> bits, flips;
-      for (int b = 0; b < KT; ++b) { bits.push_back(b); flips.push_back(b); }
-      add_group(bits, flips);
-      for (int b = KT; b < n; b += KT - LOW) {
-        std::vector<int> tile_bits, local;
-        for (int l = 0; l < LOW; ++l) tile_bits.push_back(l);
-        for (int c = b; c < std::min(n, b + KT - LOW); ++c) {
-          local.push_back(static_cast<int>(tile_bits.size()));
-          tile_bits.push_back(c);
-        }
-        for (int c = KT - 1; static_cast<int>(tile_bits.size()) < KT; --c) tile_bits.push_back(c);  // fillers
-        std::vector<int> order(tile_bits);  // tile bits ascending keeps the 512-byte runs of the low bits
-        std::sort(order.begin(), order.end());
-        std::vector<int> flips;
-        for (int f : local) flips.push_back(static_cast<int>(std::find(order.begin(), order.end(), tile_bits[static_cast<size_t>(f)]) - order.begin()));
-        add_group(order, flips);
-      }
-    }
-    std::vector<int> slot_of_bit(static_cast<size_t>(n), -1);  // d_out offset of a physical bit's (x, y, z)
-    int width = 0;
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-      for (int f = 0; f < groups[gi].nflips; ++f) slot_of_bit[static_cast<size_t>(group_flips[gi][static_cast<size_t>(f)])] = width + 3 * f;
-      width += 3 * groups[gi].nflips + 1;
-    }
-    if (width > 4 * (rbk::kMaxQubits + 8)) return fail(RBK_ERR_INVALID, "too many qubits for the spin layouts");
-    for (int q = 0; q < n; ++q)
-      if (slot_of_bit[static_cast<size_t>(q)] < 0) return fail(RBK_ERR_STATE, "spin layouts miss a qubit");
-    int offset = 0;
-    for (const auto& g : groups) {
-      int rc = launch_reduction(s, [&] {
-        return c128 ? rbk::launch_spins<double>(s->amps, n, g, s->d_partials, s->d_out + offset, s->stream)
-                    : rbk::launch_spins<float>(s->amps, n, g, s->d_partials, s->d_out + offset, s->stream);
-      });
-      if (rc) return rc;
-      offset += 3 * g.nflips + 1;
-    }
-    if (int rc = read_out(s, width)) return rc;
-    const double total = s->h_out[3 * groups.front().nflips];  // sum |a|^2 of the first layout
-    for (int q = 0; q < n; ++q) {
-      const int k = slot_of_bit[static_cast<size_t>(s->perm[q])];
-      const double one = s->h_out[k + 2];
-      out[3 * q + 0] = s->h_out[k];      // <S_x> = Re sum conj(a0) a1
-      out[3 * q + 1] = s->h_out[k + 1];  // <S_y> = Im sum conj(a0) a1
-      out[3 * q + 2] = 0.5 * ((total - one) - one);
+    observed o;
+    if (int rc = observe_all(s, (1ull << s->n) - 1, true, {}, o)) return rc;
+    for (int q = 0; q < s->n; ++q) {
+      const int b = s->perm[q];
+      out[3 * q + 0] = o.x[b][0];  // <S_x> = Re sum conj(a0) a1
+      out[3 * q + 1] = o.x[b][1];  // <S_y> = Im sum conj(a0) a1
+      out[3 * q + 2] = 0.5 * ((o.total - o.z[b]) - o.z[b]);
     }
     return RBK_OK;
   });
@@ -1096,12 +1159,60 @@ int rbk_expectation_pauli(rbk_state* s, int num_terms, const char* strings, cons
     if (int rc = flush(s)) return rc;
     std::vector<pauli_group_terms> groups;
     if (int rc = group_pauli_terms(s, num_terms, strings, coeffs, groups)) return rc;
-    double acc_re = 0, acc_im = 0;
+    // Strings without flips (real weights) and X_q, Y_q come from the one-qubit
+    // reads of the whole state, all in one go; every other flip mask takes a read
+    // of its own.
+    std::vector<diag_term> diag;
+    std::vector<const pauli_group_terms*> singles, others;
+    uint64_t flips = 0;
     for (const auto& g : groups) {
-      double r[2];
-      if (int rc = pauli_group(s, g.flip, g.terms, r)) return rc;
-      acc_re += r[0];
-      acc_im += r[1];
+      bool single = __builtin_popcountll(g.flip) == 1, real = g.flip == 0;
+      for (int t = 0; t < g.terms.count; ++t) {
+        if (g.terms.sign[t] != 0 && g.terms.sign[t] != g.flip) single = false;
+        if (g.terms.w[t][1] != 0.0) real = false;
+      }
+      if (real) {
+        for (int t = 0; t < g.terms.count; ++t) diag.push_back({g.terms.sign[t], g.terms.w[t][0]});
+      } else if (single) {
+        singles.push_back(&g);
+        flips |= g.flip;
+      } else {
+        others.push_back(&g);
+      }
+    }
+    double acc_re = 0, acc_im = 0;
+    if (!diag.empty() || flips) {
+      observed o;
+      if (int rc = observe_all(s, flips, false, diag, o)) return rc;
+      acc_re += o.diag;
+      for (const pauli_group_terms* g : singles) {
+        const int b = __builtin_ctzll(g->flip);
+        for (int t = 0; t < g->terms.count; ++t) {
+          // X: w (c + conj c) = 2 w Re c.  Y: its w holds -i, w (c - conj c) = 2 i w Im c.
+          const cplx w{g->terms.w[t][0], g->terms.w[t][1]};
+          const cplx v = g->terms.sign[t] == 0 ? 2.0 * o.x[b][0] * w : cplx{0.0, 2.0 * o.x[b][1]} * w;
+          acc_re += v.real();
+          acc_im += v.imag();
+        }
+      }
+    }
+    constexpr size_t kPerRead = 2 * (rbk::kMaxQubits + 8);  // results that one read-back holds
+    for (size_t g0 = 0; g0 < others.size(); g0 += kPerRead) {
+      const size_t count = std::min(kPerRead, others.size() - g0);
+      for (size_t k = 0; k < count; ++k) {
+        const pauli_group_terms& g = *others[g0 + k];
+        int rc = launch_reduction(s, [&] {
+          double* to = s->d_out + 2 * k;
+          return s->precision == RBK_C128 ? rbk::launch_pauli<double>(s->amps, s->n, g.flip, g.terms, s->d_partials, to, s->stream)
+                                          : rbk::launch_pauli<float>(s->amps, s->n, g.flip, g.terms, s->d_partials, to, s->stream);
+        });
+        if (rc) return rc;
+      }
+      if (int rc = read_out(s, static_cast<int>(2 * count))) return rc;
+      for (size_t k = 0; k < count; ++k) {
+        acc_re += s->h_out[2 * k];
+        acc_im += s->h_out[2 * k + 1];
+      }
     }
     out[0] = acc_re;
     out[1] = acc_im;

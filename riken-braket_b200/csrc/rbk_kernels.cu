@@ -232,107 +232,275 @@ pauli_kernel(const typename ctype<Real>::c* __restrict__ a, int n, uint64_t flip
   block_sum_store<2>(vals, 2, partials + size_t(blockIdx.x) * 2);
 }
 
-// spin_group (rbk_kernels.h): persistent CTAs, one tile at a time, two CTAs
-// per SM (one loads while the other sums).  Element j = it * 256 + tid of a
-// tile sits at shared-memory slot smem_slot(j) (the fused pass's XOR swizzle,
-// linear, so a thread composes slots with XORs and every phase reads without
-// bank conflicts).
-template <typename Real>
-__global__ void __launch_bounds__(kRedThreads, 2)
-spins_kernel(const typename ctype<Real>::c* __restrict__ a, const __grid_constant__ spin_group S, uint64_t num_tiles,
-             double* partials)
-{
-  using C = typename ctype<Real>::c;
-  constexpr int VB = precision_traits<Real>::VB;
-  constexpr int RB = sizeof(Real) == 8 ? 3 : 4, NE = 1 << RB;  // 256 threads x NE = 2^(8 + RB) = the tile
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* tile = reinterpret_cast<C*>(smem_raw);
-  const uint32_t tid = threadIdx.x;
-  // The thread's parts of addresses, the same for every tile.
-  uint64_t tphys = 0;
-  for (int b = 0; b < 8; ++b) tphys |= uint64_t((tid >> b) & 1u) << S.tile_phys[b];
-  const uint32_t st = smem_slot<VB>(tid);
-  uint32_t sbase[kSpinPhases];
-#pragma unroll
-  for (int p = 0; p < kSpinPhases; ++p) {
-    uint32_t j = 0;
-    if (p < S.nphases)
-      for (int b = 0; b < 8; ++b) j |= ((tid >> b) & 1u) << S.phase_thr[p][b];
-    sbase[p] = smem_slot<VB>(j);
+// observe_group (rbk_kernels.h).  Persistent CTAs, two per SM; a thread loads
+// the 2^RB amplitudes of a tile that vary in the top RB tile bits, so the flips
+// of those bits and every sum of |a|^2 come straight from the loaded registers;
+// the other flips are read back from shared memory (slots smem_slot, conflict
+// free) in register phases of RB bits.  The next tile's loads are issued before
+// the phases, so that they are in flight while the phases run.
+//   Bounds: HBM (one read) against 2 FP64 multiply-adds per amplitude and flip
+// and (phases + 1) shared-memory moves of the tile.  Sums of |a|^2 cost one
+// square per amplitude for all bits: the bits above the tile take a warp's
+// total once per tile (lane l keeps the sum of bit l of the tile index).
+//   27 qubits complex<double> (2 GiB): energy of 27 ZZ and 27 X strings with all
+// spins 19.1 -> 3.5 ms; before, 28 reads of 0.45 ms, one per flip mask and each
+// waited for, and four spin reads of 0.59 ms.
+// A tile is 2^11 amplitudes for both precisions: with 16 amplitudes a thread
+// (complex<float>) the sums of 12 bits and the two register copies spilled.
+// Phase p's registers and thread bits, one hexadecimal digit per tile bit,
+// lowest first (lanes 0-2 of every layout reach distinct bank groups of the
+// swizzled slots for complex<double>); own: how many of its registers' flips
+// belong to the phase.
+struct observe_shape {
+  static constexpr int RB = kObserveRegBits, K = 8 + RB, NE = 1 << RB, PHASES = 4;
+  static __host__ __device__ constexpr int reg(int p, int k) { return ((p == 0 ? 0xA98 : p == 1 ? 0x210 : p == 2 ? 0x043 : 0x765) >> (4 * k)) & 15; }
+  static __host__ __device__ constexpr int own(int p) { return p == 2 ? 2 : 3; }
+  static __host__ __device__ constexpr int thr(int p, int b)
+  {
+    return ((p == 0 ? 0x76543210u : p == 1 ? 0x765A9843u : p == 2 ? 0x765A8921u : 0xA9843210u) >> (4 * b)) & 15;
   }
-  double xr[kMaxSpinFlips], xi[kMaxSpinFlips], z[kMaxSpinFlips];
+};
+
+// The flips that belong to phase P from a thread's registers.
+template <typename Real, int P>
+__device__ __forceinline__ void observe_flips(const typename ctype<Real>::c (&e)[observe_shape::NE], int mask,
+                                              double (&xr)[observe_shape::K], double (&xi)[observe_shape::K])
+{
+  using SH = observe_shape;
 #pragma unroll
-  for (int f = 0; f < kMaxSpinFlips; ++f) xr[f] = xi[f] = z[f] = 0.0;
-  double total = 0.0;
-  for (uint64_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-    uint64_t base = tphys;
-    for (int r = 0; r < S.num_runs; ++r) base |= ((t >> S.run_src[r]) & ((1ull << S.run_len[r]) - 1)) << S.run_dst[r];
-    C v[NE];
+  for (int k = 0; k < SH::own(P); ++k) {
+    const int f = SH::reg(P, k);
+    if ((mask >> f) & 1) {
 #pragma unroll
-    for (int it = 0; it < NE; ++it) {
-      uint64_t p = base;
-#pragma unroll
-      for (int b = 0; b < RB; ++b)
-        if ((it >> b) & 1) p |= 1ull << S.tile_phys[8 + b];
-      v[it] = __ldcs(a + p);
-    }
-    __syncthreads();  // the previous tile is no longer read
-#pragma unroll
-    for (int it = 0; it < NE; ++it) {
-      tile[st ^ smem_slot<VB>(uint32_t(it) << 8)] = v[it];
-      total += double(v[it].x) * double(v[it].x) + double(v[it].y) * double(v[it].y);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < kSpinPhases; ++p) {
-      if (p < S.nphases) {
-        uint32_t rs[RB];
-#pragma unroll
-        for (int k = 0; k < RB; ++k) rs[k] = smem_slot<VB>(1u << S.phase_reg[p][k]);
-        C e[NE];
-#pragma unroll
-        for (int i = 0; i < NE; ++i) {
-          uint32_t sidx = sbase[p];
-#pragma unroll
-          for (int k = 0; k < RB; ++k)
-            if ((i >> k) & 1) sidx ^= rs[k];
-          e[i] = tile[sidx];
-        }
-#pragma unroll
-        for (int k = 0; k < RB; ++k) {
-          const int f = p * RB + k;
-          if (f < kMaxSpinFlips && f < S.nflips) {
-#pragma unroll
-            for (int i = 0; i < NE; ++i) {
-              if ((i >> k) & 1) continue;
-              const C u = e[i], w = e[i | (1 << k)];
-              xr[f] += double(u.x) * double(w.x) + double(u.y) * double(w.y);
-              xi[f] += double(u.x) * double(w.y) - double(u.y) * double(w.x);
-              z[f] += double(w.x) * double(w.x) + double(w.y) * double(w.y);
-            }
-          }
-        }
+      for (int i = 0; i < (1 << SH::RB); ++i) {
+        if ((i >> k) & 1) continue;
+        const auto u = e[i], w = e[i | (1 << k)];
+        xr[f] = __fma_rn(double(u.x), double(w.x), __fma_rn(double(u.y), double(w.y), xr[f]));
+        xi[f] = __fma_rn(double(u.x), double(w.y), __fma_rn(-double(u.y), double(w.x), xi[f]));
       }
     }
   }
-  // Block sums, in a fixed order, of 3 nflips + 1 values.
-  __shared__ double red[kRedThreads / 32][3 * kMaxSpinFlips + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+}
+
+// Phase P and those after it, each reading the tile in its layout.
+template <typename Real, int P>
+__device__ __forceinline__ void observe_phases(const typename ctype<Real>::c* tile, int mask, double (&xr)[observe_shape::K],
+                                               double (&xi)[observe_shape::K])
+{
+  using SH = observe_shape;
+  constexpr int VB = precision_traits<Real>::VB, RB = SH::RB, NE = 1 << RB;
+  if constexpr (P < SH::PHASES) {
+    int mine = 0;
 #pragma unroll
-  for (int f = 0; f < kMaxSpinFlips; ++f) {
-    if (f < S.nflips) {
-      const double a0 = warp_sum(xr[f]), a1 = warp_sum(xi[f]), a2 = warp_sum(z[f]);
-      if (lane == 0) { red[warp][3 * f] = a0; red[warp][3 * f + 1] = a1; red[warp][3 * f + 2] = a2; }
+    for (int k = 0; k < SH::own(P); ++k) mine |= 1 << SH::reg(P, k);
+    if (mask & mine) {
+      uint32_t j = 0;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) j |= ((threadIdx.x >> b) & 1u) << SH::thr(P, b);
+      const uint32_t sb = smem_slot<VB>(j);
+      typename ctype<Real>::c e[NE];
+#pragma unroll
+      for (int i = 0; i < NE; ++i) {
+        uint32_t sidx = sb;
+#pragma unroll
+        for (int k = 0; k < RB; ++k)
+          if ((i >> k) & 1) sidx ^= smem_slot<VB>(1u << SH::reg(P, k));
+        e[i] = tile[sidx];
+      }
+      observe_flips<Real, P>(e, mask, xr, xi);
+    }
+    observe_phases<Real, P + 1>(tile, mask, xr, xi);
+  }
+}
+
+template <typename Real, bool ZSUMS, bool DIAG>
+__global__ void __launch_bounds__(kRedThreads, 2)
+observe_kernel(const typename ctype<Real>::c* __restrict__ a, int n, const __grid_constant__ observe_group S, uint64_t num_tiles,
+               double* partials)
+{
+  using C = typename ctype<Real>::c;
+  using SH = observe_shape;
+  constexpr int VB = precision_traits<Real>::VB, RB = SH::RB, NE = 1 << RB, K = 8 + RB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* tile = reinterpret_cast<C*>(smem_raw);
+  const uint32_t tid = threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t tphys = 0;
+  for (int b = 0; b < 8; ++b) tphys |= uint64_t((tid >> b) & 1u) << S.tile_phys[b];
+  auto tile_base = [&](uint64_t t) {
+    uint64_t base = 0;
+    for (int r = 0; r < S.num_runs; ++r) base |= ((t >> S.run_src[r]) & ((1ull << S.run_len[r]) - 1)) << S.run_dst[r];
+    return base;
+  };
+  auto load = [&](uint64_t t, C (&v)[NE]) {
+    const uint64_t base = tile_base(t) | tphys;
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+      uint64_t p = base;
+#pragma unroll
+      for (int b = 0; b < RB; ++b)
+        if ((i >> b) & 1) p |= 1ull << S.tile_phys[8 + b];
+      v[i] = __ldcs(a + p);
+    }
+  };
+  // Parity of every diagonal string on this thread's tile bits, one bit per string.
+  uint64_t tpar = 0;
+  for (int k = 0; DIAG && k < S.diag_terms; ++k) tpar |= uint64_t(__popcll(tphys & S.sign[k]) & 1) << k;
+  const bool flips_any = S.flip_mask != 0;
+  double xr[K], xi[K];
+#pragma unroll
+  for (int f = 0; f < K; ++f) xr[f] = xi[f] = 0.0;
+  double total = 0.0, zreg[RB], zout = 0.0, dsum = 0.0;
+#pragma unroll
+  for (int b = 0; b < RB; ++b) zreg[b] = 0.0;
+
+  C v[NE];
+  if (blockIdx.x < num_tiles) load(blockIdx.x, v);
+  for (uint64_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+    if constexpr (ZSUMS || DIAG) {
+      double c[NE];
+      if constexpr (DIAG) {
+        // Parities of the strings on the bits outside the tile, lane k string k (and k + 32), then
+        // per register pattern the classes' weights; a Walsh transform turns the patterns into W.
+        const uint64_t base = tile_base(t);
+        const uint32_t p0 = __ballot_sync(0xffffffffu, lane < S.diag_terms && (__popcll(base & S.sign[lane]) & 1));
+        const uint32_t p1 = __ballot_sync(0xffffffffu, lane + 32 < S.diag_terms && (__popcll(base & S.sign[lane + 32]) & 1));
+        const uint64_t par = tpar ^ ((uint64_t(p1) << 32) | p0);
+#pragma unroll
+        for (int p = 0; p < NE; ++p) {
+          double w = 0.0;
+          for (int k = S.class_begin[p]; k < S.class_begin[p + 1]; ++k)
+            w = __fma_rn(S.class_w[k], double(__popcll(S.class_mask[k]) - 2 * __popcll(par & S.class_mask[k])), w);
+          c[p] = w;
+        }
+#pragma unroll
+        for (int b = 0; b < RB; ++b)
+#pragma unroll
+          for (int i = 0; i < NE; ++i) {
+            if ((i >> b) & 1) continue;
+            const double s0 = c[i], s1 = c[i | (1 << b)];
+            c[i] = s0 + s1;
+            c[i | (1 << b)] = s0 - s1;
+          }
+      }
+      double tot = 0.0;
+#pragma unroll
+      for (int i = 0; i < NE; ++i) {
+        const double p = double(v[i].x) * double(v[i].x) + double(v[i].y) * double(v[i].y);
+        if constexpr (DIAG) dsum = __fma_rn(p, c[i], dsum);
+        if constexpr (ZSUMS) {
+          tot += p;
+#pragma unroll
+          for (int b = 0; b < RB; ++b)
+            if ((i >> b) & 1) zreg[b] += p;
+        }
+      }
+      if constexpr (ZSUMS) {
+        total += tot;
+        const double w = warp_sum(tot);
+        if ((t >> lane) & 1) zout += w;
+      }
+    }
+    observe_flips<Real, 0>(v, S.flip_mask, xr, xi);
+    const bool more = t + gridDim.x < num_tiles;
+    if (flips_any) {
+      __syncthreads();  // the previous tile is no longer read
+#pragma unroll
+      for (int i = 0; i < NE; ++i) tile[smem_slot<VB>(tid) ^ smem_slot<VB>(uint32_t(i) << 8)] = v[i];
+      __syncthreads();
+    }
+    if (more) load(t + gridDim.x, v);
+    observe_phases<Real, 1>(tile, S.flip_mask, xr, xi);
+  }
+  // Block sums in a fixed order, one output column after the other.
+  constexpr int COLS = 2 * K + 1 + kMaxQubits + 1;
+  __shared__ double red[kRedThreads / 32][COLS];
+  int col = 0;
+#pragma unroll
+  for (int f = 0; f < K; ++f) {
+    if ((S.flip_mask >> f) & 1) {
+      const double a0 = warp_sum(xr[f]), a1 = warp_sum(xi[f]);
+      if (lane == 0) { red[warp][col] = a0; red[warp][col + 1] = a1; }
+      col += 2;
     }
   }
-  const double tt = warp_sum(total);
-  if (lane == 0) red[warp][3 * S.nflips] = tt;
+  if constexpr (ZSUMS) {
+    // Column 1 + q: the physical bit q of thread bits, register bits, then tile-index bits.
+    const double tt = warp_sum(total);
+    if (lane == 0) red[warp][col] = tt;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const double z = warp_sum(((tid >> b) & 1u) ? total : 0.0);
+      if (lane == 0) red[warp][col + 1 + S.tile_phys[b]] = z;
+    }
+#pragma unroll
+    for (int b = 0; b < RB; ++b) {
+      const double z = warp_sum(zreg[b]);
+      if (lane == 0) red[warp][col + 1 + S.tile_phys[8 + b]] = z;
+    }
+    for (int r = 0; r < S.num_runs; ++r)
+      if (lane >= S.run_src[r] && lane < S.run_src[r] + S.run_len[r])
+        red[warp][col + 1 + S.run_dst[r] + (lane - S.run_src[r])] = zout;
+    col += 1 + n;
+  }
+  if constexpr (DIAG) {
+    const double d = warp_sum(dsum);
+    if (lane == 0) red[warp][col] = d;
+    col += 1;
+  }
   __syncthreads();
-  const int width = 3 * S.nflips + 1;
-  for (int k = threadIdx.x; k < width; k += blockDim.x) {
+  for (int k = threadIdx.x; k < col; k += blockDim.x) {
     double acc = 0.0;
     for (int w = 0; w < kRedThreads / 32; ++w) acc += red[w][k];
-    partials[size_t(blockIdx.x) * width + k] = acc;
+    partials[size_t(blockIdx.x) * col + k] = acc;
+  }
+}
+
+// launch_observe_small: the state in shared memory, one warp per output, no
+// partial sums and no second launch.
+constexpr int kSmallThreads = 512;
+template <typename Real>
+__global__ void __launch_bounds__(kSmallThreads)
+observe_small_kernel(const typename ctype<Real>::c* __restrict__ a, int n, const __grid_constant__ pauli_terms T,
+                     double* __restrict__ out)
+{
+  using C = typename ctype<Real>::c;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* s = reinterpret_cast<C*>(smem_raw);
+  const uint32_t size = 1u << n;
+  for (uint32_t i = threadIdx.x; i < size; i += blockDim.x) s[i] = a[i];
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31;
+  const int warps = kSmallThreads / 32;
+  // Work items: x_b of bit b (item b), the plain sum (item n), the sum over bit b set (n + 1 + b), the diagonal strings.
+  for (int w = threadIdx.x >> 5; w < 2 * n + 2; w += warps) {
+    double re = 0.0, im = 0.0;
+    if (w < n) {
+      for (uint32_t v = lane; v < size / 2; v += 32) {
+        const uint32_t i = uint32_t(insert_zero(v, w));
+        const C x = s[i], y = s[i | (1u << w)];
+        re += double(x.x) * double(y.x) + double(x.y) * double(y.y);
+        im += double(x.x) * double(y.y) - double(x.y) * double(y.x);
+      }
+    } else {
+      const uint32_t need = w > n && w <= 2 * n ? 1u << (w - n - 1) : 0u;
+      for (uint32_t i = lane; i < size; i += 32) {
+        if ((i & need) != need) continue;
+        const double p = double(s[i].x) * double(s[i].x) + double(s[i].y) * double(s[i].y);
+        double f = 1.0;
+        if (w == 2 * n + 1) {
+          f = 0.0;
+          for (int t = 0; t < T.count; ++t) f += (__popc(i & uint32_t(T.sign[t])) & 1) ? -T.w[t][0] : T.w[t][0];
+        }
+        re += p * f;
+      }
+    }
+    re = warp_sum(re);
+    im = warp_sum(im);
+    if (lane == 0) {
+      if (w < n) { out[2 * w] = re; out[2 * w + 1] = im; }
+      else out[n + w] = re;
+    }
   }
 }
 
@@ -419,13 +587,15 @@ cudaError_t launch_pauli(const void* state, int n, uint64_t flip, const pauli_te
   return cudaGetLastError();
 }
 
-template <typename Real>
-cudaError_t launch_spins(const void* state, int n, const spin_group& g, double* partials, double* out, cudaStream_t stream)
+int observe_width(const observe_group& g, int n)
 {
-  const int rb = sizeof(Real) == 8 ? 3 : 4;
-  if (g.K != 8 + rb || g.K > n || g.nflips < 1 || g.nflips > kMaxSpinFlips || g.nphases < 1 ||
-      g.nphases > kSpinPhases || g.nphases * rb < g.nflips)
-    return cudaErrorInvalidValue;
+  return 2 * __builtin_popcount(static_cast<unsigned>(g.flip_mask)) + (g.zsums ? 1 + n : 0) + (g.diag_classes > 0 ? 1 : 0);
+}
+
+template <typename Real, bool ZSUMS, bool DIAG>
+static cudaError_t launch_observe_form(const typename ctype<Real>::c* state, int n, const observe_group& g, uint64_t tiles,
+                                       int blocks, double* partials, cudaStream_t stream)
+{
   const size_t smem = sizeof(typename ctype<Real>::c) << g.K;
   static std::atomic<bool> configured[64] = {};
   int dev = 0;
@@ -433,14 +603,40 @@ cudaError_t launch_spins(const void* state, int n, const spin_group& g, double* 
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (!configured[dev].load(std::memory_order_acquire)) {
-    e = cudaFuncSetAttribute(spins_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 << 12);
+    e = cudaFuncSetAttribute(observe_kernel<Real, ZSUMS, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     configured[dev].store(true, std::memory_order_release);
   }
-  const uint64_t tiles = 1ull << (n - g.K);
+  observe_kernel<Real, ZSUMS, DIAG><<<blocks, kRedThreads, smem, stream>>>(state, n, g, tiles, partials);
+  return cudaGetLastError();
+}
+
+template <typename Real>
+cudaError_t launch_observe(const void* state, int n, const observe_group& g, double* partials, double* out, cudaStream_t stream)
+{
+  constexpr int K = 8 + observe_shape::RB;
+  const int width = observe_width(g, n);
+  if (g.K != K || K > n || n - K > 32 || n > kMaxQubits || (g.flip_mask >> K) != 0 || width < 1 ||
+      (g.zsums && g.diag_classes > 0) || g.diag_terms < 0 ||
+      g.diag_terms > kObserveTerms || g.diag_classes < 0 || g.diag_classes > kObserveTerms)
+    return cudaErrorInvalidValue;
+  const uint64_t tiles = 1ull << (n - K);
   const int blocks = static_cast<int>(std::min<uint64_t>(tiles, 148 * 2));
-  spins_kernel<Real><<<blocks, kRedThreads, smem, stream>>>(static_cast<const typename ctype<Real>::c*>(state), g, tiles, partials);
-  finish_partials_kernel<<<3 * g.nflips + 1, kFinishThreads, 0, stream>>>(partials, blocks, 3 * g.nflips + 1, out);
+  const auto* a = static_cast<const typename ctype<Real>::c*>(state);
+  const cudaError_t e = g.diag_classes > 0 ? launch_observe_form<Real, false, true>(a, n, g, tiles, blocks, partials, stream)
+                        : g.zsums          ? launch_observe_form<Real, true, false>(a, n, g, tiles, blocks, partials, stream)
+                                           : launch_observe_form<Real, false, false>(a, n, g, tiles, blocks, partials, stream);
+  if (e != cudaSuccess) return e;
+  finish_partials_kernel<<<width, kFinishThreads, 0, stream>>>(partials, blocks, width, out);
+  return cudaGetLastError();
+}
+
+template <typename Real>
+cudaError_t launch_observe_small(const void* state, int n, const pauli_terms& terms, double* out, cudaStream_t stream)
+{
+  if (n < 1 || n >= 8 + observe_shape::RB || terms.count < 0 || terms.count > kMaxPauliTerms) return cudaErrorInvalidValue;
+  observe_small_kernel<Real><<<1, kSmallThreads, sizeof(typename ctype<Real>::c) << n, stream>>>(
+    static_cast<const typename ctype<Real>::c*>(state), n, terms, out);
   return cudaGetLastError();
 }
 
@@ -476,8 +672,10 @@ template cudaError_t launch_zsum<double>(const void*, int, double*, double*, cud
 template cudaError_t launch_zsum<float>(const void*, int, double*, double*, cudaStream_t);
 template cudaError_t launch_pauli<double>(const void*, int, uint64_t, const pauli_terms&, double*, double*, cudaStream_t);
 template cudaError_t launch_pauli<float>(const void*, int, uint64_t, const pauli_terms&, double*, double*, cudaStream_t);
-template cudaError_t launch_spins<double>(const void*, int, const spin_group&, double*, double*, cudaStream_t);
-template cudaError_t launch_spins<float>(const void*, int, const spin_group&, double*, double*, cudaStream_t);
+template cudaError_t launch_observe<double>(const void*, int, const observe_group&, double*, double*, cudaStream_t);
+template cudaError_t launch_observe<float>(const void*, int, const observe_group&, double*, double*, cudaStream_t);
+template cudaError_t launch_observe_small<double>(const void*, int, const pauli_terms&, double*, cudaStream_t);
+template cudaError_t launch_observe_small<float>(const void*, int, const pauli_terms&, double*, cudaStream_t);
 template cudaError_t launch_pauli2<double>(const void*, const void*, int, uint64_t, const pauli_terms&, double*, double*, cudaStream_t);
 template cudaError_t launch_pauli2<float>(const void*, const void*, int, uint64_t, const pauli_terms&, double*, double*, cudaStream_t);
 template cudaError_t launch_inner<double>(const void*, const void*, int, double*, double*, cudaStream_t);

@@ -94,18 +94,12 @@ size_t tile_overlaps_partials_doubles(int n, int K);
 template <typename Real> cudaError_t launch_tile_overlaps(const void* lam, const void* psi, int n, const tile_overlap_set& set,
                                                           double* partials, double* out, cudaStream_t stream);
 
-// All spins of the flip bits of one tile layout in one read of the state.
-// Tile t (its bits outside tile_phys spell t, deposited run by run) of 2^K
-// amplitudes, K = 8 + RB (RB = 3 for complex<double>, 4 for complex<float>;
-// 256 threads), is staged in shared memory; for each flip f the CTAs sum
-//   x_f = sum over j with tile bit b_f clear of conj(a_j) a_{j | b_f}   (complex)
-//   z_f = sum over j with tile bit b_f set of |a_j|^2
-// and the total of |a|^2.  The flips are read in register phases: in phase p
-// a thread holds the 2^RB amplitudes whose tile bits phase_reg[p][0..RB-1]
-// vary, at the tile bits phase_thr[p][0..7] that its index gives; flip
-// f = p * RB + k is register bit k of phase p (entries past nflips are fillers).
-// out[3f], out[3f+1] = x_f; out[3f+2] = z_f; out[3 nflips] = total.
-constexpr int kMaxSpinFlips = 12;
+// The register phases of a tile of 2^(8 + RB) amplitudes held by 256 threads, and
+// where its other bits lie: tile t's bits outside tile_phys spell t, deposited
+// run by run; in phase p a thread holds the 2^RB amplitudes whose tile bits
+// phase_reg[p][0..RB-1] vary, at the tile bits phase_thr[p][0..7] that its
+// index gives; flip f = p * RB + k is register bit k of phase p (entries past
+// nflips are fillers).
 constexpr int kSpinPhases = 4;
 struct spin_group {
   int K, num_runs, nflips, nphases;
@@ -113,9 +107,36 @@ struct spin_group {
   uint8_t phase_reg[kSpinPhases][4];
   uint8_t phase_thr[kSpinPhases][8];
 };
-inline int spin_register_bits(int precision) { return precision == 0 ? 3 : 4; }
-template <typename Real> cudaError_t launch_spins(const void* state, int n, const spin_group& g, double* partials, double* out,
-                                                  cudaStream_t stream);
+
+// One-qubit sums of one tile layout in one read of the state.  Tile bits
+// tile_phys[0..K-1] (K = kObserveTileBits), the tile index deposited run by run
+// into the others.  For every tile bit b in flip_mask
+//   x_b = sum over j with tile bit b clear of conj(a_j) a_{j | b}   (complex);
+// with `zsums`, sum |a_j|^2 in all and over j with each physical bit set; with
+// diag_classes > 0, sum |a_j|^2 W(j), W(j) = sum_t w_t (-1)^popcount(j & sign_t)
+// over diag_terms real-weighted Z-type strings.  The strings come in classes of
+// one weight and one pattern on the thread's register bits (the top RB tile
+// bits), sorted by pattern: class c has the strings of bit mask class_mask[c].
+// out: (x_b re, im) for the bits of flip_mask in ascending order, then 1 + n
+// sums (zsums), then the diagonal sum (diag_classes > 0).
+constexpr int kObserveTerms = 64;
+constexpr int kObserveRegBits = 3;
+constexpr int kObserveTileBits = 8 + kObserveRegBits;
+struct observe_group {
+  int32_t K, num_runs, flip_mask, zsums, diag_terms, diag_classes;  // zsums or diag_classes > 0, not both
+  uint8_t tile_phys[16], run_src[16], run_len[16], run_dst[16];
+  uint64_t sign[kObserveTerms];
+  uint64_t class_mask[kObserveTerms];
+  double class_w[kObserveTerms];
+  uint8_t class_begin[(1 << kObserveRegBits) + 1];  // classes of register pattern p: [begin[p], begin[p + 1])
+};
+int observe_width(const observe_group& g, int n);
+template <typename Real> cudaError_t launch_observe(const void* state, int n, const observe_group& g, double* partials, double* out,
+                                                    cudaStream_t stream);
+// The same for a state smaller than the tile (n < kObserveTileBits), in one CTA: every x_b, the
+// 1 + n sums of |a_j|^2, and the diagonal sum of `terms` (real weights), in that order.
+template <typename Real> cudaError_t launch_observe_small(const void* state, int n, const pauli_terms& terms, double* out,
+                                                          cudaStream_t stream);
 
 // Overlaps of one-qubit Paulis in one read of both states (the adjoint sweep's
 // rotation runs).  Z type: S_q = sum_j (-1)^{j_q} conj(lam_j) psi_j for
