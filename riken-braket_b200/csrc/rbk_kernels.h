@@ -33,7 +33,9 @@ int reduction_blocks();
 // Records msg as the calling thread's rbk_last_error() and returns code.
 int set_last_error(int code, const char* msg);
 // Scratch needed by the reductions below, in doubles.
-inline size_t reduction_scratch_doubles() { return size_t(1 << 12) * (1 + kMaxQubits) + 64; }
+// The most is the Z sums' 512 blocks of 1 + n sums (1.3 MB of slack on top made
+// creating a state map fresh device memory more often than not).
+inline size_t reduction_scratch_doubles() { return size_t(1 << 9) * (1 + kMaxQubits) + 64; }
 
 template <typename Real> cudaError_t launch_zsum(const void* state, int n, double* partials, double* out, cudaStream_t stream);
 template <typename Real> cudaError_t launch_pauli(const void* state, int n, uint64_t flip, const pauli_terms& terms,
