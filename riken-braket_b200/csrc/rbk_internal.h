@@ -192,16 +192,28 @@ struct dev_pass {
   alignas(16) double tabs[kMaxLayerTabs * kTabDoubles];  // factored layers' diagonal factors (complex<double> or complex<float>)
 };
 
-// Per-gate (unfused) program record, used for states smaller than one tile
-// and by the unfused execution mode.  Bits are physical.
-struct alignas(8) gate_rec {
-  uint8_t kind;        // op_kind
-  uint8_t target;      // physical target bit (MAT/X/Y/DIAG)
-  uint8_t diag_one;
-  uint8_t pad;
+// Program of a state that fits one CTA's shared memory (n <= kSmallBits): the
+// queue as phases of 2^kSmallRegBits amplitudes per thread.  In a phase the
+// register bits are the physical bits reg[0] < reg[1] < reg[2]; a thread's other
+// bits give its base index.  Controls and diagonal bits are checked on the
+// register slot (creg, dreg) and on the base index (cbase, dbase).
+constexpr int kSmallBits = 12;    // 2^12 complex<double> = 64 KB
+constexpr int kSmallRegBits = 3;  // states of fewer qubits are padded to this
+constexpr int kSmallGates = 368;  // gates of one launch (32 KB of kernel parameters is the most)
+struct alignas(8) small_op {
+  uint8_t kind;      // op_kind
+  uint8_t treg;      // MAT/X/Y: target register bit
+  uint8_t real;      // MAT: every entry is real
+  uint8_t diag_one;  // DIAG: d0 == 1 exactly
+  uint8_t creg, dreg;
+  uint16_t cbase, dbase, pad;
   uint32_t pad1;
-  uint64_t cmask;      // physical control mask
   double m[8];
+};
+struct small_phase {
+  uint8_t reg[kSmallRegBits];
+  uint8_t pad;
+  uint16_t begin, end;
 };
 
 }  // namespace rbk

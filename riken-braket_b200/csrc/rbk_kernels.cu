@@ -21,37 +21,137 @@
 namespace rbk {
 
 // ---------------------------------------------------------------------------
-// Unfused gate straight on HBM
+// Whole circuits on states of one CTA
 // ---------------------------------------------------------------------------
 
-template <typename Real>
-__global__ void gate_kernel(typename ctype<Real>::c* __restrict__ a, uint64_t size, const gate_rec g)
+// A queue of gates on a state of up to kSmallBits qubits, in one CTA: the state
+// and the program are read into shared memory once, every phase (small_phase)
+// moves 8 amplitudes per thread into registers, applies its gates there and
+// writes them back, and the state goes back to HBM at the end.  Arithmetic is
+// complex<double> for both precisions (a complex<float> state is rounded once,
+// at the end).
+//   Bound by latency: a phase costs two shared-memory moves and a barrier, a
+// gate its dispatch and its FP64 work on one SM.  One launch per gate (below
+// one tile) took 2.7 us of device and 2.9 us of host time a gate; the tile
+// passes at 11 and 12 qubits put a pass of 12 gates on 1 or 2 CTAs of 4 warps.
+//   8 qubits, 200 random gates: 772 us of device and 468 us of host time with a
+// launch per gate, 126 and 31 us here.
+template <int CAP>
+struct small_params {
+  uint32_t num_ops, num_phases;
+  small_phase phases[CAP];
+  small_op ops[CAP];
+};
+
+template <int B>
+__device__ __forceinline__ void small_target(double2 (&a)[1 << kSmallRegBits], const small_op& o)
+{
+  const uint32_t creg = o.creg;
+#pragma unroll
+  for (int i = 0; i < (1 << kSmallRegBits); ++i) {
+    if (i & (1 << B)) continue;
+    if ((uint32_t(i) & creg) != creg) continue;
+    double2 &x = a[i], &y = a[i | (1 << B)];
+    const double2 a0 = x, a1 = y;
+    if (o.kind == OPK_X) {
+      x = a1;
+      y = a0;
+    } else if (o.kind == OPK_Y) {
+      x = double2{a1.y, -a1.x};
+      y = double2{-a0.y, a0.x};
+    } else if (o.real) {
+      x = rmac2(a0, a1, o.m[0], o.m[2]);
+      y = rmac2(a0, a1, o.m[4], o.m[6]);
+    } else {
+      x = cmac2(a0, a1, o.m[0], o.m[1], o.m[2], o.m[3]);
+      y = cmac2(a0, a1, o.m[4], o.m[5], o.m[6], o.m[7]);
+    }
+  }
+}
+
+constexpr int kSmallCircuitThreads = 512;  // 1024 (64 registers) spilled
+template <typename Real, int CAP>
+__global__ void __launch_bounds__(kSmallCircuitThreads, 1)
+small_circuit_kernel(typename ctype<Real>::c* __restrict__ state, int n, const __grid_constant__ small_params<CAP> P)
 {
   using C = typename ctype<Real>::c;
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  const uint64_t tmask = 1ull << g.target;
-  if (g.kind == OPK_MAT || g.kind == OPK_X || g.kind == OPK_Y) {
-    const Real m00r = (Real)g.m[0], m00i = (Real)g.m[1], m01r = (Real)g.m[2], m01i = (Real)g.m[3];
-    const Real m10r = (Real)g.m[4], m10i = (Real)g.m[5], m11r = (Real)g.m[6], m11i = (Real)g.m[7];
-    for (uint64_t v = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; v < (size >> 1); v += stride) {
-      const uint64_t i0 = insert_zero(v, g.target), i1 = i0 | tmask;
-      if ((i0 & g.cmask) != g.cmask) continue;
-      C a0 = a[i0], a1 = a[i1];
-      if (g.kind == OPK_X) { a[i0] = a1; a[i1] = a0; }
-      else if (g.kind == OPK_Y) { a[i0] = C{a1.y, -a1.x}; a[i1] = C{-a0.y, a0.x}; }
-      else {
-        a[i0] = cmac2(a0, a1, m00r, m00i, m01r, m01i);
-        a[i1] = cmac2(a0, a1, m10r, m10i, m11r, m11i);
+  constexpr int NR = 1 << kSmallRegBits;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* s = reinterpret_cast<double2*>(smem_raw);
+  const uint32_t size = 1u << n, padded = max(size, uint32_t(NR));
+  small_op* ops = reinterpret_cast<small_op*>(s + padded);
+  {
+    // Through a generic pointer: the threads read the parameter block side by side,
+    // where indexing it by the thread would go word by word through the constant cache.
+    const uint64_t* src = reinterpret_cast<const uint64_t*>(P.ops);
+    asm volatile("" : "+l"(src));
+    uint64_t* dst = reinterpret_cast<uint64_t*>(ops);
+    for (uint32_t i = threadIdx.x; i < P.num_ops * uint32_t(sizeof(small_op) / 8); i += blockDim.x) dst[i] = src[i];
+  }
+  // Slots are swizzled (smem_slot) so that the lanes of a phase reach distinct banks whichever bits it holds.
+  for (uint32_t i = threadIdx.x; i < padded; i += blockDim.x) {
+    double2 v{0.0, 0.0};
+    if (i < size) {
+      const C x = state[i];
+      v = double2{double(x.x), double(x.y)};
+    }
+    s[smem_slot<0>(i)] = v;
+  }
+  __syncthreads();
+  for (uint32_t p = 0; p < P.num_phases; ++p) {
+    const small_phase ph = P.phases[p];
+    uint32_t rs[kSmallRegBits];
+#pragma unroll
+    for (int k = 0; k < kSmallRegBits; ++k) rs[k] = smem_slot<0>(1u << ph.reg[k]);
+    for (uint32_t t = threadIdx.x; t < padded / NR; t += blockDim.x) {
+      uint32_t base = t;
+#pragma unroll
+      for (int k = 0; k < kSmallRegBits; ++k) base = uint32_t(insert_zero(base, ph.reg[k]));
+      const uint32_t sb = smem_slot<0>(base);
+      double2 a[NR];
+#pragma unroll
+      for (int i = 0; i < NR; ++i) {
+        uint32_t x = sb;
+#pragma unroll
+        for (int k = 0; k < kSmallRegBits; ++k)
+          if ((i >> k) & 1) x ^= rs[k];
+        a[i] = s[x];
+      }
+      for (uint32_t g = ph.begin; g < ph.end; ++g) {
+        const small_op& o = ops[g];
+        if ((base & o.cbase) != o.cbase) continue;
+        if (o.kind == OPK_DIAG || o.kind == OPK_NEG) {
+          const uint32_t creg = o.creg, dreg = o.dreg;
+          const bool hi = (base & o.dbase) != 0, neg = o.kind == OPK_NEG, one = o.diag_one;
+#pragma unroll
+          for (int i = 0; i < NR; ++i) {
+            if ((uint32_t(i) & creg) != creg) continue;
+            if (neg) a[i] = double2{-a[i].x, -a[i].y};
+            else if (hi || (uint32_t(i) & dreg)) a[i] = cmul(a[i], double2{o.m[2], o.m[3]});
+            else if (!one) a[i] = cmul(a[i], double2{o.m[0], o.m[1]});
+          }
+        } else if (o.treg == 0) {
+          small_target<0>(a, o);
+        } else if (o.treg == 1) {
+          small_target<1>(a, o);
+        } else {
+          small_target<2>(a, o);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < NR; ++i) {
+        uint32_t x = sb;
+#pragma unroll
+        for (int k = 0; k < kSmallRegBits; ++k)
+          if ((i >> k) & 1) x ^= rs[k];
+        s[x] = a[i];
       }
     }
-  } else {
-    const C d0{(Real)g.m[0], (Real)g.m[1]}, d1{(Real)g.m[2], (Real)g.m[3]};
-    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < size; i += stride) {
-      if ((i & g.cmask) != g.cmask) continue;
-      if (g.kind == OPK_NEG) { a[i].x = -a[i].x; a[i].y = -a[i].y; }
-      else if (i & tmask) a[i] = cmul(a[i], d1);
-      else if (!g.diag_one) a[i] = cmul(a[i], d0);
-    }
+    __syncthreads();
+  }
+  for (uint32_t i = threadIdx.x; i < size; i += blockDim.x) {
+    const double2 v = s[smem_slot<0>(i)];
+    state[i] = C{Real(v.x), Real(v.y)};
   }
 }
 
@@ -63,15 +163,49 @@ static unsigned grid_for(uint64_t work, int threads)
   return (unsigned)(b == 0 ? 1 : b);
 }
 
-template <typename Real>
-cudaError_t launch_gate(void* state, int n, const gate_rec& g, cudaStream_t stream)
+template <typename Real, int CAP>
+static cudaError_t launch_small_cap(typename ctype<Real>::c* state, int n, const small_op* ops, int num_ops,
+                                    const small_phase* phases, int num_phases, cudaStream_t stream)
 {
-  const uint64_t size = 1ull << n;
-  gate_kernel<Real><<<grid_for(size >> 1, 256), 256, 0, stream>>>(static_cast<typename ctype<Real>::c*>(state), size, g);
+  const uint32_t padded = std::max(1u << n, 1u << kSmallRegBits);
+  const size_t smem = sizeof(double2) * padded + sizeof(small_op) * size_t(num_ops);
+  constexpr size_t most = sizeof(double2) * (size_t(1) << kSmallBits) + sizeof(small_op) * CAP;
+  static std::atomic<bool> configured[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(small_circuit_kernel<Real, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess) return e;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  small_params<CAP> P;
+  P.num_ops = static_cast<uint32_t>(num_ops);
+  P.num_phases = static_cast<uint32_t>(num_phases);
+  std::copy(ops, ops + num_ops, P.ops);
+  std::copy(phases, phases + num_phases, P.phases);
+  const int threads = static_cast<int>(std::max(32u, std::min(uint32_t(kSmallCircuitThreads), padded >> kSmallRegBits)));
+  small_circuit_kernel<Real, CAP><<<1, threads, smem, stream>>>(state, n, P);
   return cudaGetLastError();
 }
-template cudaError_t launch_gate<double>(void*, int, const gate_rec&, cudaStream_t);
-template cudaError_t launch_gate<float>(void*, int, const gate_rec&, cudaStream_t);
+
+// The parameter block is copied at every launch whatever it holds, so short
+// programs take a short one (2.8, 11 and 32 KB).
+template <typename Real>
+cudaError_t launch_small(void* state, int n, const small_op* ops, int num_ops, const small_phase* phases, int num_phases,
+                         cudaStream_t stream)
+{
+  static_assert(sizeof(small_params<kSmallGates>) <= 32640, "parameter block");
+  if (n < 1 || n > kSmallBits || num_ops < 1 || num_ops > kSmallGates || num_phases < 1 || num_phases > num_ops)
+    return cudaErrorInvalidValue;
+  auto* a = static_cast<typename ctype<Real>::c*>(state);
+  if (num_ops <= 32) return launch_small_cap<Real, 32>(a, n, ops, num_ops, phases, num_phases, stream);
+  if (num_ops <= 128) return launch_small_cap<Real, 128>(a, n, ops, num_ops, phases, num_phases, stream);
+  return launch_small_cap<Real, kSmallGates>(a, n, ops, num_ops, phases, num_phases, stream);
+}
+template cudaError_t launch_small<double>(void*, int, const small_op*, int, const small_phase*, int, cudaStream_t);
+template cudaError_t launch_small<float>(void*, int, const small_op*, int, const small_phase*, int, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Basis-state initialisation

@@ -22,7 +22,9 @@ struct pauli_terms {
 
 // One fused pass with tile shape `shape` (see tile_shape in rbk_internal.h).
 template <typename Real> cudaError_t launch_tile_pass(void* state, int n, const dev_pass& pass, int shape, cudaStream_t stream);
-template <typename Real> cudaError_t launch_gate(void* state, int n, const gate_rec& g, cudaStream_t stream);
+// One small-state program (plan_small) on a state of n <= kSmallBits qubits.
+template <typename Real> cudaError_t launch_small(void* state, int n, const small_op* ops, int num_ops, const small_phase* phases,
+                                                  int num_phases, cudaStream_t stream);
 template <typename Real> cudaError_t launch_set_basis(void* state, int n, uint64_t index, cudaStream_t stream);
 // ket::shor_box on a zeroed state: 2^nx amplitudes of value coeff (divisor, base < 2^32).
 template <typename Real>

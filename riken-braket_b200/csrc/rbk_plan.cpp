@@ -892,15 +892,77 @@ void apply_relabel(const plan_params& p, const int* tile_phys, const int* new_ph
 
 }  // namespace
 
-gate_rec to_physical(const hgate& g, const std::vector<int>& perm)
+void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv,
+                std::vector<small_program>& out)
 {
-  gate_rec r{};
-  r.kind = g.kind;
-  r.diag_one = g.diag_one;
-  r.target = static_cast<uint8_t>(g.target >= 0 ? perm[g.target] : 0);
-  r.cmask = map_mask(g.cmask, perm);
-  std::memcpy(r.m, g.m, sizeof(r.m));
-  return r;
+  std::vector<char> taken(gates.size(), 0);
+  const uint64_t all = bit(n) - 1;
+  size_t first = 0;
+  while (true) {
+    while (first < gates.size() && taken[first]) ++first;
+    if (first >= gates.size()) break;
+    uint64_t blockN = 0, blockZ = 0, regs = 0;
+    std::vector<size_t> mine;
+    for (size_t i = first; i < gates.size() && mine.size() < static_cast<size_t>(kSmallGates); ++i) {
+      if (taken[i]) continue;
+      const hgate& g = gates[i];
+      if (g.kind == HK_SWAP) {
+        const uint64_t m = bit(perm[g.target]) | bit(perm[g.target2]);
+        if ((blockN | blockZ) & m) { blockN |= m; continue; }
+        if (!mine.empty()) { blockN |= m; continue; }  // gates taken so far name physical bits of the present map
+        const int pa = perm[g.target], pb = perm[g.target2];
+        perm[g.target] = pb; perm[g.target2] = pa;
+        inv[pa] = g.target2; inv[pb] = g.target;
+        taken[i] = 1;
+        continue;
+      }
+      const uint64_t t = is_target_kind(g.kind) ? bit(perm[g.target]) : 0;
+      const uint64_t z = map_mask(g.cmask, perm) | (g.kind == OPK_DIAG ? bit(perm[g.target]) : 0);
+      if ((t & (blockN | blockZ)) || (z & blockN) || (t && !(regs & t) && popc(regs) >= kSmallRegBits)) {
+        blockN |= t;
+        blockZ |= z;
+        if (((blockN | blockZ) & all) == all) break;
+        continue;
+      }
+      regs |= t;
+      mine.push_back(i);
+      taken[i] = 1;
+    }
+    if (mine.empty()) continue;  // only swaps were taken
+    small_phase ph{};
+    for (int q = 0; popc(regs) < kSmallRegBits; ++q) regs |= bit(q);  // fillers (bits past n are padding)
+    for (int k = 0, q = 0; k < kSmallRegBits; ++q)
+      if (regs & bit(q)) ph.reg[k++] = static_cast<uint8_t>(q);
+    auto reg_mask = [&](uint64_t m) {
+      uint8_t r = 0;
+      for (int k = 0; k < kSmallRegBits; ++k) r |= static_cast<uint8_t>(((m >> ph.reg[k]) & 1) << k);
+      return r;
+    };
+    if (out.empty() || out.back().ops.size() + mine.size() > static_cast<size_t>(kSmallGates)) out.emplace_back();
+    small_program& prog = out.back();
+    ph.begin = static_cast<uint16_t>(prog.ops.size());
+    for (size_t i : mine) {
+      const hgate& g = gates[i];
+      small_op o{};
+      o.kind = g.kind;
+      o.diag_one = g.diag_one;
+      std::memcpy(o.m, g.m, sizeof(o.m));
+      const uint64_t c = map_mask(g.cmask, perm);
+      o.creg = reg_mask(c);
+      o.cbase = static_cast<uint16_t>(c & ~regs);
+      if (is_target_kind(g.kind)) {
+        const uint8_t tm = reg_mask(bit(perm[g.target]));
+        o.treg = static_cast<uint8_t>(__builtin_ctz(tm));
+        o.real = g.m[1] == 0.0 && g.m[3] == 0.0 && g.m[5] == 0.0 && g.m[7] == 0.0;
+      } else if (g.kind == OPK_DIAG) {
+        o.dreg = reg_mask(bit(perm[g.target]));
+        o.dbase = static_cast<uint16_t>(bit(perm[g.target]) & ~regs);
+      }
+      prog.ops.push_back(o);
+    }
+    ph.end = static_cast<uint16_t>(prog.ops.size());
+    prog.phases.push_back(ph);
+  }
 }
 
 void plan_passes(const plan_params& p, const std::vector<hgate>& gates, std::vector<int>& perm,

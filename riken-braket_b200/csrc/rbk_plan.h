@@ -53,7 +53,17 @@ void plan_layout(const plan_params& p, std::vector<int>& perm, std::vector<int>&
 void plan_canonicalize(const plan_params& p, std::vector<int>& perm, std::vector<int>& inv,
                        std::vector<dev_pass>& out);
 
-// Physical form of a gate for the unfused path (states smaller than a tile).
-gate_rec to_physical(const hgate& g, const std::vector<int>& perm);
+// A small state's launch: at most kSmallGates gates in register phases.
+struct small_program {
+  std::vector<small_op> ops;
+  std::vector<small_phase> phases;
+};
+
+// The queue as launches of the small-state kernel (n <= kSmallBits), gates in
+// physical bits; SWAPs only update the layout map.  A phase takes, in order,
+// every gate that commutes with those it leaves behind and whose target is, or
+// can still join, its register bits.
+void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv,
+                std::vector<small_program>& out);
 
 }  // namespace rbk
