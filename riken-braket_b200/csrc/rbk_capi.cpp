@@ -38,6 +38,7 @@ struct rbk_state {
   float* d_tc_w = nullptr;   // W_hi, W_lo of the tensor-core unitaries (largest k), kept between calls
   int* d_tc_flag = nullptr;  // set by a tensor-core unitary whose bounded wait ran out (sticky)
   int* h_tc_flag = nullptr;  // pinned copy, read at every bounded_sync
+  double* d_block_u = nullptr;  // U of the CUDA-core block unitaries (largest k), kept between calls
   double* d_sample = nullptr;  // workspace of the sampling calls (sample_workspace)
   size_t sample_bytes = 0;
   std::vector<int> perm, inv;
@@ -703,6 +704,7 @@ int rbk_state_destroy(rbk_state* s)
   if (s->d_out) cudaFree(s->d_out);
   if (s->h_out) cudaFreeHost(s->h_out);
   if (s->d_sample) cudaFree(s->d_sample);
+  if (s->d_block_u) cudaFree(s->d_block_u);
   if (s->d_tc_w) cudaFree(s->d_tc_w);
   if (s->d_tc_flag) cudaFree(s->d_tc_flag);
   if (s->h_tc_flag) cudaFreeHost(s->h_tc_flag);
@@ -2601,7 +2603,8 @@ int apply_unitary(rbk_state* s, const std::vector<cplx>& U, const uint32_t* q, i
 {
   device_guard g(s->device);
   const bool tensor = s->precision == RBK_C64 && (k == 5 || k == 6) && s->n >= k + 7;
-  if (tensor) {
+  const bool block = !tensor && k <= rbk::kBlockMaxBits;
+  if (tensor || block) {
     if (int rc = flush(s)) return rc;
   } else if (int rc = move_to_low(s, q, k)) {
     return rc;
@@ -2653,6 +2656,48 @@ int apply_unitary(rbk_state* s, const std::vector<cplx>& U, const uint32_t* q, i
     // No wait here: the flag reaches the pinned copy in stream order and the next
     // bounded_sync (every read of the state) reports a wait that ran out.
     RBK_CUDA(cudaMemcpyAsync(s->h_tc_flag, s->d_tc_flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  } else if (block) {
+    // Tile bits: the targets and the lowest others, ascending; the kernel gathers
+    // them where they lie.
+    rbk::block_layout lay{};
+    const int T = std::min(s->n, rbk::kBlockTileBits), LR = rbk::kBlockTileBits - k;
+    std::vector<int> target_of(static_cast<size_t>(s->n), -1);
+    uint64_t mask = 0;
+    for (int i = 0; i < k; ++i) {
+      target_of[static_cast<size_t>(s->perm[q[i]])] = i;
+      mask |= 1ull << s->perm[q[i]];
+    }
+    for (int b = 0; b < s->n && __builtin_popcountll(mask) < T; ++b) mask |= 1ull << b;
+    int at = 0, row = 0, src = 0;
+    for (int b = 0; b < s->n; ++b) {
+      if (!((mask >> b) & 1)) continue;
+      const int i = target_of[static_cast<size_t>(b)];
+      lay.tile_phys[at] = static_cast<uint8_t>(b);
+      lay.tile_local[at++] = static_cast<uint16_t>(1u << (i >= 0 ? LR + i : row++));
+    }
+    lay.elems = 1u << T;
+    for (int b = 0; b < s->n;) {
+      if ((mask >> b) & 1) { ++b; continue; }
+      int len = 0;
+      while (b + len < s->n && !((mask >> (b + len)) & 1)) ++len;
+      lay.run_src[lay.num_runs] = static_cast<uint8_t>(src);
+      lay.run_len[lay.num_runs] = static_cast<uint8_t>(len);
+      lay.run_dst[lay.num_runs] = static_cast<uint8_t>(b);
+      ++lay.num_runs;
+      src += len;
+      b += len;
+    }
+    if (!s->d_block_u)
+      RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&s->d_block_u), sizeof(cplx) << (2 * rbk::kBlockMaxBits)));
+    // Stream order keeps this copy behind the previous unitary's reads of the buffer; the
+    // pageable source is staged by the copy call.
+    RBK_CUDA(cudaMemcpyAsync(s->d_block_u, U.data(), sizeof(cplx) * U.size(), cudaMemcpyHostToDevice, s->stream));
+    const cudaError_t e = s->precision == RBK_C128
+      ? rbk::launch_block_unitary<double>(s->amps, s->n, k, s->d_block_u, lay, s->stream)
+      : rbk::launch_block_unitary<float>(s->amps, s->n, k, s->d_block_u, lay, s->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "block unitary");
+    ++s->stats.kernel_launches;
+    ++s->stats.passes;
   } else {
     device_buffer du;
     const size_t count = 2 * U.size();

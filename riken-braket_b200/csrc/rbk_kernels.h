@@ -241,8 +241,22 @@ size_t tc_w_split_floats(int k);
 size_t tc_shared_bytes(int k);
 cudaError_t launch_unitary_tf32x3(void* state, int n, int k, const float* w_split, int* error_flag, int grid,
                                   const tc_layout& layout, cudaStream_t stream);
-// CUDA cores, any precision, k <= 10, targets on the low k physical bits: U is 2^k x 2^k
-// complex (re, im) in row-major order on the device.
+// CUDA cores, any precision.  U is 2^k x 2^k complex (re, im) in row-major order
+// on the device.  k <= kBlockMaxBits: tiles of 2^kBlockTileBits amplitudes (the
+// whole state where n is smaller; elems amplitudes) over tile_phys, ascending;
+// tile_local[b] is 1 << (kBlockTileBits - k + i) where tile bit b is target i,
+// and 1 << r where it is row bit r.
+constexpr int kBlockMaxBits = 6;
+constexpr int kBlockTileBits = 11;
+struct block_layout {
+  uint32_t elems;
+  uint16_t tile_local[kBlockTileBits];
+  uint8_t tile_phys[kBlockTileBits];
+  uint8_t num_runs, run_src[16], run_len[16], run_dst[16];
+};
+template <typename Real> cudaError_t launch_block_unitary(void* state, int n, int k, const double* U, const block_layout& layout,
+                                                          cudaStream_t stream);
+// k <= 10, targets on the low k physical bits.
 template <typename Real> cudaError_t launch_dense_rows(void* state, int n, int k, const double* U, cudaStream_t stream);
 
 }  // namespace rbk

@@ -374,8 +374,120 @@ unitary_tf32x3_kernel(float2* __restrict__ state, uint64_t rows, const float4* _
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOLS));
 }
 
-// Dense k-qubit unitary on CUDA cores (any precision; the targets on the low k
-// physical bits): one CTA per row of 2^k amplitudes, thread b computes output b.
+// Dense k-qubit unitary, k <= kBlockMaxBits, on CUDA cores with FP64 products
+// and sums for both precisions.  A tile is the targets' bits with the lowest
+// other bits, 2^kBlockTileBits amplitudes (512-byte or longer runs), held in
+// shared memory as [target index e][row] with U beside it; thread t computes 4
+// outputs (2 for k = 1) of 2 (4) rows, so that 6 shared-memory loads feed 32
+// FP64 multiply-adds.  Persistent CTAs, two per SM; the next tile's loads are
+// issued before the products.  Row slots are XORed with the low bits of e, so
+// that both the coalesced side (lanes on target bits) and the product side
+// (lanes along rows) reach distinct banks.
+//   Bound: 2^(k+2) FP64 multiply-adds an amplitude against one read and one
+// write; the two meet near k = 4 (complex<double>).  The targets are gathered
+// where they lie: no relabelling passes.
+constexpr int kBlockThreads = 256;
+
+template <typename Real, int KB>
+__global__ void __launch_bounds__(kBlockThreads, 2)
+block_unitary_kernel(typename ctype<Real>::c* __restrict__ state, uint64_t tiles, const __grid_constant__ block_layout L,
+                     const double2* __restrict__ U)
+{
+  using C = typename ctype<Real>::c;
+  constexpr int DIM = 1 << KB, LR = kBlockTileBits - KB, ROWS = 1 << LR, LD = DIM + 1;
+  constexpr int TO = KB >= 2 ? 4 : 2, TR = 8 / TO;  // outputs and rows per thread
+  constexpr int RG = ROWS / TR;                     // row groups; rows of a thread are RG apart
+  constexpr int NE = (1 << kBlockTileBits) / kBlockThreads;
+  static_assert(NE == TO * TR && (DIM / TO) * RG == kBlockThreads, "each thread owns as many outputs as loads");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* x = reinterpret_cast<double2*>(smem_raw);
+  double2* u = x + (1 << kBlockTileBits);
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t i = tid; i < DIM * DIM; i += kBlockThreads) u[(i >> KB) * LD + (i & (DIM - 1))] = U[i];
+  // This thread's tile elements j = tid + 256 it: physical offset and shared-memory slot, both sums over j's bits.
+  auto slot = [](uint32_t e, uint32_t row) { return (e << LR) | (row ^ (e & 7u)); };
+  const bool active = tid < L.elems;  // a state smaller than a tile
+  uint64_t tphys = 0;
+  uint32_t tloc = 0;  // (e << LR) | row
+  for (int b = 0; b < 8; ++b)
+    if ((tid >> b) & 1u) { tphys |= 1ull << L.tile_phys[b]; tloc |= L.tile_local[b]; }
+  auto tile_base = [&](uint64_t t) {
+    uint64_t v = 0;
+    for (int r = 0; r < L.num_runs; ++r) v |= ((t >> L.run_src[r]) & ((1ull << L.run_len[r]) - 1)) << L.run_dst[r];
+    return v;
+  };
+  auto elem = [&](int it, uint64_t base, uint64_t& phys, uint32_t& s) {
+    phys = base | tphys;
+    uint32_t loc = tloc;
+#pragma unroll
+    for (int b = 8; b < kBlockTileBits; ++b)
+      if ((it >> (b - 8)) & 1) { phys |= 1ull << L.tile_phys[b]; loc |= L.tile_local[b]; }
+    s = slot(loc >> LR, loc & (ROWS - 1));
+    return active && tid + uint32_t(it) * kBlockThreads < L.elems;
+  };
+  C v[NE];
+  auto load = [&](uint64_t t) {
+    const uint64_t base = tile_base(t);
+#pragma unroll
+    for (int it = 0; it < NE; ++it) {
+      uint64_t p;
+      uint32_t s;
+      v[it] = elem(it, base, p, s) ? __ldcs(state + p) : C{Real(0), Real(0)};
+    }
+  };
+  const uint32_t rg = tid % RG, og = tid / RG;
+  if (blockIdx.x < tiles) load(blockIdx.x);
+  for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const uint64_t base = tile_base(t);
+#pragma unroll
+    for (int it = 0; it < NE; ++it) {
+      uint64_t p;
+      uint32_t s;
+      if (elem(it, base, p, s)) x[s] = double2{double(v[it].x), double(v[it].y)};
+    }
+    __syncthreads();
+    if (t + gridDim.x < tiles) load(t + gridDim.x);
+    double2 acc[TO][TR];
+#pragma unroll
+    for (int o = 0; o < TO; ++o)
+#pragma unroll
+      for (int r = 0; r < TR; ++r) acc[o][r] = double2{0.0, 0.0};
+#pragma unroll 2
+    for (int a = 0; a < DIM; ++a) {
+      double2 xv[TR];
+#pragma unroll
+      for (int r = 0; r < TR; ++r) xv[r] = x[slot(a, rg + r * RG)];
+#pragma unroll
+      for (int o = 0; o < TO; ++o) {
+        const double2 w = u[(og * TO + o) * LD + a];
+#pragma unroll
+        for (int r = 0; r < TR; ++r) {
+          acc[o][r].x = __fma_rn(-w.y, xv[r].y, __fma_rn(w.x, xv[r].x, acc[o][r].x));
+          acc[o][r].y = __fma_rn(w.y, xv[r].x, __fma_rn(w.x, xv[r].y, acc[o][r].y));
+        }
+      }
+    }
+    __syncthreads();  // every input of the tile has been read
+#pragma unroll
+    for (int o = 0; o < TO; ++o)
+#pragma unroll
+      for (int r = 0; r < TR; ++r) x[slot(og * TO + o, rg + r * RG)] = acc[o][r];
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < NE; ++it) {
+      uint64_t p;
+      uint32_t s;
+      if (elem(it, base, p, s)) {
+        const double2 y = x[s];
+        __stcs(state + p, C{Real(y.x), Real(y.y)});
+      }
+    }
+    __syncthreads();  // the stores have read the tile
+  }
+}
+
+// The same for k > kBlockMaxBits, where U no longer fits beside a tile (the
+// targets on the low k physical bits): one CTA per row of 2^k amplitudes, thread b computes output b.
 template <typename Real>
 __global__ void dense_rows_kernel(typename ctype<Real>::c* __restrict__ state, uint64_t rows, int k,
                                   const double* __restrict__ U)
@@ -433,6 +545,37 @@ cudaError_t launch_unitary_tf32x3(void* state, int n, int k, const float* w_spli
   }
   return cudaGetLastError();
 }
+
+namespace {
+template <typename Real, int KB>
+cudaError_t launch_block(void* state, int n, const double* U, const block_layout& layout, cudaStream_t stream)
+{
+  constexpr size_t smem = sizeof(double2) * ((size_t(1) << kBlockTileBits) + (size_t(1) << KB) * ((size_t(1) << KB) + 1));
+  cudaError_t e = cudaFuncSetAttribute(block_unitary_kernel<Real, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (e != cudaSuccess) return e;
+  const uint64_t tiles = n > kBlockTileBits ? 1ull << (n - kBlockTileBits) : 1;
+  block_unitary_kernel<Real, KB><<<unsigned(tiles < 148 * 2 ? tiles : 148 * 2), kBlockThreads, smem, stream>>>(
+    static_cast<typename ctype<Real>::c*>(state), tiles, layout, reinterpret_cast<const double2*>(U));
+  return cudaGetLastError();
+}
+}  // namespace
+
+template <typename Real>
+cudaError_t launch_block_unitary(void* state, int n, int k, const double* U, const block_layout& layout, cudaStream_t stream)
+{
+  if (k > n || layout.elems != (1u << (n < kBlockTileBits ? n : kBlockTileBits))) return cudaErrorInvalidValue;
+  switch (k) {
+    case 1: return launch_block<Real, 1>(state, n, U, layout, stream);
+    case 2: return launch_block<Real, 2>(state, n, U, layout, stream);
+    case 3: return launch_block<Real, 3>(state, n, U, layout, stream);
+    case 4: return launch_block<Real, 4>(state, n, U, layout, stream);
+    case 5: return launch_block<Real, 5>(state, n, U, layout, stream);
+    case 6: return launch_block<Real, 6>(state, n, U, layout, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+template cudaError_t launch_block_unitary<double>(void*, int, int, const double*, const block_layout&, cudaStream_t);
+template cudaError_t launch_block_unitary<float>(void*, int, int, const double*, const block_layout&, cudaStream_t);
 
 template <typename Real>
 cudaError_t launch_dense_rows(void* state, int n, int k, const double* U, cudaStream_t stream)
