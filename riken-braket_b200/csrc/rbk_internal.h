@@ -206,8 +206,9 @@ struct alignas(8) small_op {
   uint8_t real;      // MAT: every entry is real
   uint8_t diag_one;  // DIAG: d0 == 1 exactly
   uint8_t creg, dreg;
-  uint16_t cbase, dbase, pad;
-  uint32_t pad1;
+  uint16_t cbase, dbase;
+  uint16_t rot;      // adjoint sweeps: 1, 2, 3 = a rotation of X, Y, Z type whose overlap is taken, 0 = none
+  int32_t slot;      // ... and the overlap's number
   double m[8];
 };
 struct small_phase {

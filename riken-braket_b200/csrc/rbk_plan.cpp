@@ -892,24 +892,26 @@ void apply_relabel(const plan_params& p, const int* tile_phys, const int* new_ph
 
 }  // namespace
 
-void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv,
-                std::vector<small_program>& out)
+void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv, size_t max_ops,
+                       const std::function<void(const std::vector<small_op>&, const std::vector<size_t>&, const small_phase&)>& emit)
 {
   std::vector<char> taken(gates.size(), 0);
   const uint64_t all = bit(n) - 1;
   size_t first = 0;
+  std::vector<size_t> mine;
+  std::vector<small_op> ops;
   while (true) {
     while (first < gates.size() && taken[first]) ++first;
     if (first >= gates.size()) break;
     uint64_t blockN = 0, blockZ = 0, regs = 0;
-    std::vector<size_t> mine;
-    for (size_t i = first; i < gates.size() && mine.size() < static_cast<size_t>(kSmallGates); ++i) {
+    mine.clear();
+    for (size_t i = first; i < gates.size() && mine.size() < max_ops; ++i) {
       if (taken[i]) continue;
       const hgate& g = gates[i];
       if (g.kind == HK_SWAP) {
         const uint64_t m = bit(perm[g.target]) | bit(perm[g.target2]);
-        if ((blockN | blockZ) & m) { blockN |= m; continue; }
-        if (!mine.empty()) { blockN |= m; continue; }  // gates taken so far name physical bits of the present map
+        // gates taken so far name physical bits of the present map
+        if (((blockN | blockZ) & m) || !mine.empty()) { blockN |= m; continue; }
         const int pa = perm[g.target], pb = perm[g.target2];
         perm[g.target] = pb; perm[g.target2] = pa;
         inv[pa] = g.target2; inv[pb] = g.target;
@@ -921,7 +923,7 @@ void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, 
       if ((t & (blockN | blockZ)) || (z & blockN) || (t && !(regs & t) && popc(regs) >= kSmallRegBits)) {
         blockN |= t;
         blockZ |= z;
-        if (((blockN | blockZ) & all) == all) break;
+        if ((blockN & all) == all) break;
         continue;
       }
       regs |= t;
@@ -938,14 +940,13 @@ void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, 
       for (int k = 0; k < kSmallRegBits; ++k) r |= static_cast<uint8_t>(((m >> ph.reg[k]) & 1) << k);
       return r;
     };
-    if (out.empty() || out.back().ops.size() + mine.size() > static_cast<size_t>(kSmallGates)) out.emplace_back();
-    small_program& prog = out.back();
-    ph.begin = static_cast<uint16_t>(prog.ops.size());
+    ops.clear();
     for (size_t i : mine) {
       const hgate& g = gates[i];
       small_op o{};
       o.kind = g.kind;
       o.diag_one = g.diag_one;
+      o.slot = -1;
       std::memcpy(o.m, g.m, sizeof(o.m));
       const uint64_t c = map_mask(g.cmask, perm);
       o.creg = reg_mask(c);
@@ -958,11 +959,25 @@ void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, 
         o.dreg = reg_mask(bit(perm[g.target]));
         o.dbase = static_cast<uint16_t>(bit(perm[g.target]) & ~regs);
       }
-      prog.ops.push_back(o);
+      ops.push_back(o);
     }
-    ph.end = static_cast<uint16_t>(prog.ops.size());
-    prog.phases.push_back(ph);
+    emit(ops, mine, ph);
   }
+}
+
+void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv,
+                std::vector<small_program>& out)
+{
+  plan_small_phases(n, gates, perm, inv, static_cast<size_t>(kSmallGates),
+                    [&](const std::vector<small_op>& ops, const std::vector<size_t>&, const small_phase& phase) {
+                      if (out.empty() || out.back().ops.size() + ops.size() > static_cast<size_t>(kSmallGates)) out.emplace_back();
+                      small_program& prog = out.back();
+                      small_phase ph = phase;
+                      ph.begin = static_cast<uint16_t>(prog.ops.size());
+                      prog.ops.insert(prog.ops.end(), ops.begin(), ops.end());
+                      ph.end = static_cast<uint16_t>(prog.ops.size());
+                      prog.phases.push_back(ph);
+                    });
 }
 
 void plan_passes(const plan_params& p, const std::vector<hgate>& gates, std::vector<int>& perm,

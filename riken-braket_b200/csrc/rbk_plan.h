@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include "rbk_internal.h"
@@ -59,10 +60,15 @@ struct small_program {
   std::vector<small_phase> phases;
 };
 
-// The queue as launches of the small-state kernel (n <= kSmallBits), gates in
-// physical bits; SWAPs only update the layout map.  A phase takes, in order,
-// every gate that commutes with those it leaves behind and whose target is, or
-// can still join, its register bits.
+// The queue in register phases of a small state: emit(ops, indices, phase) for
+// each, with the ops in physical bits, the gates they come from, and the phase's
+// register bits.  A phase takes, in order, every gate that commutes with those
+// it leaves behind and whose target is, or can still join, its register bits, at
+// most max_ops of them; SWAPs only update the layout map.
+void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv, size_t max_ops,
+                       const std::function<void(const std::vector<small_op>&, const std::vector<size_t>&, const small_phase&)>& emit);
+
+// The queue as launches of the small-state kernel (n <= kSmallBits).
 void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv,
                 std::vector<small_program>& out);
 

@@ -1,0 +1,719 @@
+// rbk_small_adjoint.cu -- see rbk_small_adjoint.h.
+//
+// One instance is one CTA (n <= 12) or one cluster of 2^(n - 12) CTAs.  Both
+// states stay in shared memory; the CTAs of a cluster hold consecutive ranges
+// and reach each other's over distributed shared memory.  A register phase
+// (small_phase) moves 8 amplitudes of a state per thread into registers and
+// applies its gates there, so that a layer of one-qubit rotations costs n / 3
+// exchanges and barriers; a parameter's overlap is taken from the same
+// registers before its gate is un-applied.  Arithmetic in registers is
+// complex<double> for both precisions, storage is the batch's precision.
+//   Bound by FP64 work on the instance's SMs and by the latency of a phase
+// (two moves, a barrier, the reductions).  The one-gate sweeps of one CTA per
+// instance before took about 1 us a sweep (12 qubits, 16 layers: 2.2 ms) and
+// 13 to 15 qubits took 1.05 to 1.15 ms for 10 layers in engine launches.
+#include "rbk_small_adjoint.h"
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <complex>
+#include <cstring>
+#include <string>
+
+#include "rbk_device.cuh"
+#include "rbk_kernels.h"
+#include "rbk_plan.h"
+
+namespace rbk {
+namespace {
+
+constexpr int kSaThreads = 512;
+constexpr int kSaPhaseOps = 48;  // ops of one phase, staged in shared memory twice
+constexpr int kSaRegs = 1 << kSmallRegBits;
+constexpr int kSaLocalBits = 12;  // amplitudes a CTA holds of each state
+constexpr int kSaClassBits = 10;  // instances of fewer qubits share the launch of this size
+
+struct sa_args {
+  const sa_inst* inst;
+  const sa_phase* phases;
+  const sa_rot* rots;
+  const sa_term* terms;
+  small_op* ops;
+  const double* theta;
+  double* partial;
+  double* energy;
+  double* overlaps;
+};
+
+__device__ __forceinline__ double sa_warp_sum(double v)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank)
+{
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
+// An amplitude of a state in shared memory (of this CTA, or of the cluster at a mapped address).
+template <typename Real, int CS> struct sa_mem;
+template <int CS> struct sa_mem<double, CS> {
+  static __device__ __forceinline__ double2 get(uint32_t a)
+  {
+    double2 v;
+    if constexpr (CS > 1) asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    else asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void put(uint32_t a, double2 v)
+  {
+    if constexpr (CS > 1) asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" :: "r"(a), "d"(v.x), "d"(v.y) : "memory");
+    else asm volatile("st.shared.v2.f64 [%0], {%1, %2};" :: "r"(a), "d"(v.x), "d"(v.y) : "memory");
+  }
+};
+template <int CS> struct sa_mem<float, CS> {
+  static __device__ __forceinline__ double2 get(uint32_t a)
+  {
+    float2 v;
+    if constexpr (CS > 1) asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    else asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    return double2{double(v.x), double(v.y)};
+  }
+  static __device__ __forceinline__ void put(uint32_t a, double2 d)
+  {
+    const float x = float(d.x), y = float(d.y);
+    if constexpr (CS > 1) asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" :: "r"(a), "f"(x), "f"(y) : "memory");
+    else asm volatile("st.shared.v2.f32 [%0], {%1, %2};" :: "r"(a), "f"(x), "f"(y) : "memory");
+  }
+};
+
+template <int CS>
+__device__ __forceinline__ void sa_sync()
+{
+  if constexpr (CS > 1) {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+}
+
+// A 2x2 gate of target register bit B on 8 amplitudes; INV: its conjugate transpose.
+template <int B, bool INV>
+__device__ __forceinline__ void sa_target(double2 (&a)[kSaRegs], const small_op& o)
+{
+  const uint32_t creg = o.creg;
+#pragma unroll
+  for (int i = 0; i < kSaRegs; ++i) {
+    if (i & (1 << B)) continue;
+    if ((uint32_t(i) & creg) != creg) continue;
+    double2 &x = a[i], &y = a[i | (1 << B)];
+    const double2 a0 = x, a1 = y;
+    if (o.kind == OPK_X) {
+      x = a1;
+      y = a0;
+    } else if (o.kind == OPK_Y) {
+      x = double2{a1.y, -a1.x};
+      y = double2{-a0.y, a0.x};
+    } else if (o.real) {
+      x = rmac2(a0, a1, o.m[0], o.m[INV ? 4 : 2]);
+      y = rmac2(a0, a1, o.m[INV ? 2 : 4], o.m[6]);
+    } else if (INV) {
+      x = cmac2(a0, a1, o.m[0], -o.m[1], o.m[4], -o.m[5]);
+      y = cmac2(a0, a1, o.m[2], -o.m[3], o.m[6], -o.m[7]);
+    } else {
+      x = cmac2(a0, a1, o.m[0], o.m[1], o.m[2], o.m[3]);
+      y = cmac2(a0, a1, o.m[4], o.m[5], o.m[6], o.m[7]);
+    }
+  }
+}
+
+template <bool INV>
+__device__ __forceinline__ void sa_gate(double2 (&a)[kSaRegs], const small_op& o, uint32_t base)
+{
+  if ((base & o.cbase) != o.cbase) return;
+  if (o.kind == OPK_DIAG || o.kind == OPK_NEG) {
+    const uint32_t creg = o.creg, dreg = o.dreg;
+    const bool hi = (base & o.dbase) != 0, neg = o.kind == OPK_NEG, one = o.diag_one;
+#pragma unroll
+    for (int i = 0; i < kSaRegs; ++i) {
+      if ((uint32_t(i) & creg) != creg) continue;
+      if (neg) a[i] = double2{-a[i].x, -a[i].y};
+      else if (hi || (uint32_t(i) & dreg)) a[i] = cmul(a[i], double2{o.m[2], INV ? -o.m[3] : o.m[3]});
+      else if (!one) a[i] = cmul(a[i], double2{o.m[0], INV ? -o.m[1] : o.m[1]});
+    }
+  } else if (o.treg == 0) {
+    sa_target<0, INV>(a, o);
+  } else if (o.treg == 1) {
+    sa_target<1, INV>(a, o);
+  } else {
+    sa_target<2, INV>(a, o);
+  }
+}
+
+// Im <lambda| P |psi> over this thread's amplitudes, P = X or Y on register bit B.
+template <int B>
+__device__ __forceinline__ double sa_overlap(const double2 (&p)[kSaRegs], const double2 (&l)[kSaRegs], bool y)
+{
+  double s = 0.0;
+#pragma unroll
+  for (int i = 0; i < kSaRegs; ++i) {
+    if (i & (1 << B)) continue;
+    const double2 l0 = l[i], l1 = l[i | (1 << B)], p0 = p[i], p1 = p[i | (1 << B)];
+    if (y) s += (l1.x * p0.x + l1.y * p0.y) - (l0.x * p1.x + l0.y * p1.y);
+    else s += (l0.x * p1.y - l0.y * p1.x) + (l1.x * p0.y - l1.y * p0.x);
+  }
+  return s;
+}
+
+// The shared-memory address of each register slot of a phase.
+template <typename Real, int CS>
+__device__ __forceinline__ void sa_addresses(uint32_t smem, uint32_t base, const uint8_t (&reg)[kSmallRegBits], int local_bits,
+                                             uint32_t (&addr)[kSaRegs])
+{
+  constexpr uint32_t S = uint32_t(sizeof(typename ctype<Real>::c));
+#pragma unroll
+  for (int i = 0; i < kSaRegs; ++i) {
+    uint32_t x = base;
+#pragma unroll
+    for (int k = 0; k < kSmallRegBits; ++k)
+      if ((i >> k) & 1) x |= 1u << reg[k];
+    const uint32_t local = CS > 1 ? x & ((1u << local_bits) - 1) : x;
+    addr[i] = smem + smem_slot<0>(local) * S;
+    if constexpr (CS > 1) addr[i] = map_rank(addr[i], x >> local_bits);
+  }
+}
+
+template <typename Real, int CS>
+__global__ void __launch_bounds__(kSaThreads, 1) small_adjoint_kernel(const sa_args A, int first)
+{
+  constexpr int kClusterLog = CS == 8 ? 3 : CS == 4 ? 2 : CS == 2 ? 1 : 0;
+  constexpr uint32_t S = uint32_t(sizeof(typename ctype<Real>::c));
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(16) small_op ops[2][kSaPhaseOps];
+  const sa_inst I = A.inst[first + blockIdx.x / CS];
+  const uint32_t rank = blockIdx.x % CS;  // cluster dimensions (CS, 1, 1): the CTA's rank in its cluster
+  const int local_bits = max(I.n, kSmallRegBits) - kClusterLog;
+  const uint32_t local = 1u << local_bits, groups = local / kSaRegs;
+  const uint32_t psi = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw)), lam = psi + local * S;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  const uint32_t warps = blockDim.x >> 5, all_warps = warps * CS, gwarp = rank * warps + (tid >> 5);
+  double* partial = A.partial + I.partial_begin;
+  small_op* gops = A.ops + I.op_begin;
+  const sa_phase* phases = A.phases + I.phase_begin;
+  const double* theta = A.theta + I.theta_begin;
+
+  // Matrices of the parametrised rotations.
+  for (int k = int(rank * blockDim.x + tid); k < I.num_rots; k += int(blockDim.x * CS)) {
+    const sa_rot r = A.rots[I.rot_begin + k];
+    const double phi = (r.param >= 0 ? r.scale * theta[r.param] : 0.0) + r.offset;
+    double sn, cs;
+    sincos(phi, &sn, &cs);
+    small_op& o = gops[r.op];
+    if (o.rot == 1) {         // cos I + i sin X
+      o.m[0] = cs; o.m[1] = 0; o.m[2] = 0; o.m[3] = sn; o.m[4] = 0; o.m[5] = sn; o.m[6] = cs; o.m[7] = 0;
+    } else if (o.rot == 2) {  // cos I + i sin Y
+      o.m[0] = cs; o.m[1] = 0; o.m[2] = sn; o.m[3] = 0; o.m[4] = -sn; o.m[5] = 0; o.m[6] = cs; o.m[7] = 0;
+    } else {                  // diag(e^{i phi}, e^{-i phi})
+      o.m[0] = cs; o.m[1] = sn; o.m[2] = cs; o.m[3] = -sn;
+    }
+  }
+  for (uint32_t i = tid; i < local; i += blockDim.x) {
+    const uint32_t a = psi + smem_slot<0>(i) * S;
+    sa_mem<Real, 1>::put(a, double2{rank == 0 && i == 0 ? 1.0 : 0.0, 0.0});
+  }
+  __threadfence();
+  sa_sync<CS>();
+
+  // Ops of a phase into staging buffer b, through L2 (the matrices above were written by other CTAs too).
+  auto stage = [&](const sa_phase& ph, int b) {
+    const char* src = reinterpret_cast<const char*>(gops + ph.begin);
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(&ops[b][0]));
+    const uint32_t words = uint32_t(ph.end - ph.begin) * uint32_t(sizeof(small_op) / 16);
+    for (uint32_t i = tid; i < words; i += blockDim.x)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(dst + 16 * i), "l"(src + 16 * i) : "memory");
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  auto staged = [&]() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); };
+  auto group_base = [&](uint32_t g, const sa_phase& ph) {
+    uint32_t base = rank * groups + g;
+#pragma unroll
+    for (int k = 0; k < kSmallRegBits; ++k) base = uint32_t(insert_zero(base, ph.reg[k]));
+    return base;
+  };
+
+  // Forward.
+  if (I.num_phases > 0) {
+    stage(phases[0], 0);
+    staged();
+    __syncthreads();
+  }
+  sa_phase next = I.num_phases > 0 ? phases[0] : sa_phase{};
+  for (int p = 0; p < I.num_phases; ++p) {
+    const sa_phase ph = next;
+    const int b = p & 1, count = ph.end - ph.begin;
+    if (p + 1 < I.num_phases) {
+      next = phases[p + 1];
+      stage(next, b ^ 1);
+    }
+    for (uint32_t g = tid; g < groups; g += blockDim.x) {
+      const uint32_t base = group_base(g, ph);
+      uint32_t addr[kSaRegs];
+      sa_addresses<Real, CS>(psi, base, ph.reg, local_bits, addr);
+      double2 a[kSaRegs];
+#pragma unroll
+      for (int i = 0; i < kSaRegs; ++i) a[i] = sa_mem<Real, CS>::get(addr[i]);
+      for (int k = 0; k < count; ++k) sa_gate<false>(a, ops[b][k], base);
+#pragma unroll
+      for (int i = 0; i < kSaRegs; ++i) sa_mem<Real, CS>::put(addr[i], a[i]);
+    }
+    staged();
+    sa_sync<CS>();
+  }
+
+  // lambda = H psi, E = <psi|lambda>.
+  {
+    const sa_term* terms = A.terms + I.term_begin;
+    const uint32_t size = 1u << I.n;
+    double er = 0.0;
+    for (uint32_t j = tid; j < local; j += blockDim.x) {
+      const uint32_t i = rank * local + j;
+      double lr = 0.0, li = 0.0;
+      double2 v{0.0, 0.0};
+      uint32_t have = ~0u;
+      for (int t = 0; t < I.num_terms && i < size; ++t) {
+        const sa_term T = terms[t];
+        if (T.flip != have) {
+          have = T.flip;
+          const uint32_t x = i ^ T.flip;
+          uint32_t a = psi + smem_slot<0>(x & (local - 1)) * S;
+          if constexpr (CS > 1) a = map_rank(a, x >> local_bits);
+          v = sa_mem<Real, CS>::get(a);
+        }
+        const bool neg = __popc(i & T.sign) & 1;
+        const double wr = neg ? -T.wr : T.wr, wi = neg ? -T.wi : T.wi;
+        lr += wr * v.x - wi * v.y;
+        li += wr * v.y + wi * v.x;
+      }
+      const uint32_t off = smem_slot<0>(j) * S;
+      sa_mem<Real, 1>::put(lam + off, double2{lr, li});
+      const double2 pv = sa_mem<Real, 1>::get(psi + off);
+      er += pv.x * lr + pv.y * li;
+    }
+    er = sa_warp_sum(er);
+    if (lane == 0) partial[size_t(I.num_slots) * all_warps + gwarp] = er;
+  }
+  if (I.num_phases > 0) {
+    next = phases[I.num_phases - 1];
+    stage(next, (I.num_phases - 1) & 1);
+    staged();
+  }
+  sa_sync<CS>();
+
+  // Reverse: every op un-applied from both states, a rotation's overlap taken before it.
+  const uint32_t rounds = (groups + blockDim.x - 1) / blockDim.x;
+  for (int p = I.num_phases - 1; p >= 0; --p) {
+    const sa_phase ph = next;
+    const int b = p & 1, count = ph.end - ph.begin;
+    if (p > 0) {
+      next = phases[p - 1];
+      stage(next, b ^ 1);
+    }
+    for (uint32_t r = 0; r < rounds; ++r) {  // whole warps together: the overlaps are warp sums
+      const uint32_t g = r * blockDim.x + tid;
+      const bool active = g < groups;
+      const uint32_t base = group_base(active ? g : 0u, ph);
+      uint32_t addr[kSaRegs];
+      sa_addresses<Real, CS>(psi, base, ph.reg, local_bits, addr);
+      const uint32_t to_lam = lam - psi;
+      double2 a[kSaRegs], l[kSaRegs];
+#pragma unroll
+      for (int i = 0; i < kSaRegs; ++i) {
+        a[i] = l[i] = double2{0.0, 0.0};
+        if (active) {
+          a[i] = sa_mem<Real, CS>::get(addr[i]);
+          l[i] = sa_mem<Real, CS>::get(addr[i] + to_lam);
+        }
+      }
+      for (int k = count - 1; k >= 0; --k) {
+        const small_op& o = ops[b][k];
+        if (o.slot >= 0) {
+          double s = 0.0;
+          if (o.rot == 3) {
+            const bool hi = (base & o.dbase) != 0;
+            const uint32_t dreg = o.dreg;
+#pragma unroll
+            for (int i = 0; i < kSaRegs; ++i) {
+              const double c = l[i].x * a[i].y - l[i].y * a[i].x;
+              s += (hi || (uint32_t(i) & dreg)) ? -c : c;
+            }
+          } else if (o.treg == 0) {
+            s = sa_overlap<0>(a, l, o.rot == 2);
+          } else if (o.treg == 1) {
+            s = sa_overlap<1>(a, l, o.rot == 2);
+          } else {
+            s = sa_overlap<2>(a, l, o.rot == 2);
+          }
+          s = sa_warp_sum(s);
+          if (lane == 0) {
+            double* out = partial + size_t(o.slot) * all_warps + gwarp;
+            *out = r > 0 ? *out + s : s;
+          }
+        }
+        sa_gate<true>(a, o, base);
+        sa_gate<true>(l, o, base);
+      }
+      if (active) {
+#pragma unroll
+        for (int i = 0; i < kSaRegs; ++i) {
+          sa_mem<Real, CS>::put(addr[i], a[i]);
+          sa_mem<Real, CS>::put(addr[i] + to_lam, l[i]);
+        }
+      }
+    }
+    staged();
+    sa_sync<CS>();
+  }
+  __threadfence();
+  sa_sync<CS>();  // the partial sums of every CTA are visible
+  for (int s = int(rank * blockDim.x + tid); s <= I.num_slots; s += int(blockDim.x * CS)) {
+    double acc = 0.0;
+    for (uint32_t w = 0; w < all_warps; ++w) acc += __ldcg(partial + size_t(s) * all_warps + w);
+    if (s == I.num_slots) A.energy[I.out] = acc;
+    else A.overlaps[I.slot_begin + s] = acc;
+  }
+}
+
+// ---- host side ------------------------------------------------------------
+
+using cplx = std::complex<double>;
+constexpr double kOneDivRootTwo = 0.707106781186547524400844362104849039284835937688474036588;
+constexpr double kTwoPi = 6.28318530717958647692528676655900576839433879875021164195;
+
+void put(double* m, int k, cplx v) { m[2 * k] = v.real(); m[2 * k + 1] = v.imag(); }
+
+// The engine's records of the fixed gates (rbk_hadamard, rbk_phase_shift2/3, ...); a
+// rotation gets kind and qubits here and its matrix on the device.
+bool lower_gate(int n, const rbk_circuit_gate& g, hgate& h)
+{
+  h = hgate{};
+  h.target2 = -1;
+  const bool two = g.kind == RBK_GATE_CNOT || g.kind == RBK_GATE_CZ || g.kind == RBK_GATE_U || g.kind == RBK_GATE_SWAP;
+  if (g.qubits[0] < 0 || g.qubits[0] >= n) return false;
+  if (two && (g.qubits[1] < 0 || g.qubits[1] >= n || g.qubits[1] == g.qubits[0])) return false;
+  const uint64_t b0 = 1ull << g.qubits[0], b1 = two ? 1ull << g.qubits[1] : 0;
+  h.target = static_cast<int8_t>(g.qubits[0]);
+  auto phase = [&](cplx c) {
+    h.kind = OPK_DIAG;
+    h.diag_one = 1;
+    put(h.m, 0, {1.0, 0.0});
+    put(h.m, 1, c);
+  };
+  switch (g.kind) {
+    case RBK_GATE_H:
+      h.kind = OPK_MAT;
+      put(h.m, 0, {kOneDivRootTwo, 0}); put(h.m, 1, {kOneDivRootTwo, 0});
+      put(h.m, 2, {kOneDivRootTwo, 0}); put(h.m, 3, {-kOneDivRootTwo, 0});
+      return true;
+    case RBK_GATE_X: h.kind = OPK_X; return true;
+    case RBK_GATE_Y: h.kind = OPK_Y; return true;
+    case RBK_GATE_Z: h.kind = OPK_NEG; h.target = -1; h.cmask = b0; return true;
+    case RBK_GATE_U1: phase(std::exp(cplx{0, g.angles[0]})); return true;
+    case RBK_GATE_U2: {
+      const cplx c1 = std::exp(cplx{0, g.angles[0]}), c2 = std::exp(cplx{0, g.angles[1]});
+      const cplx mc1 = kOneDivRootTwo * c1;
+      h.kind = OPK_MAT;
+      put(h.m, 0, {kOneDivRootTwo, 0}); put(h.m, 1, -(kOneDivRootTwo * c2));
+      put(h.m, 2, mc1); put(h.m, 3, mc1 * c2);
+      return true;
+    }
+    case RBK_GATE_U3: {
+      const double sine = std::sin(0.5 * g.angles[0]), cosine = std::cos(0.5 * g.angles[0]);
+      const cplx c2 = std::exp(cplx{0, g.angles[1]}), c3 = std::exp(cplx{0, g.angles[2]});
+      h.kind = OPK_MAT;
+      put(h.m, 0, {cosine, 0}); put(h.m, 1, -(sine * c3));
+      put(h.m, 2, sine * c2); put(h.m, 3, (cosine * c3) * c2);
+      return true;
+    }
+    case RBK_GATE_CNOT:  // qubits[0] = control, qubits[1] = target
+      h.kind = OPK_X;
+      h.target = static_cast<int8_t>(g.qubits[1]);
+      h.cmask = b0;
+      return true;
+    case RBK_GATE_CZ: h.kind = OPK_NEG; h.target = -1; h.cmask = b0 | b1; return true;
+    case RBK_GATE_U: {
+      const int k = static_cast<int>(g.angles[0]), ak = k < 0 ? -k : k;
+      cplx c = std::exp(cplx{0, std::ldexp(kTwoPi, -ak)});
+      if (k < 0) c = std::conj(c);
+      phase(c);
+      h.target = static_cast<int8_t>(g.qubits[1]);
+      h.cmask = b0;
+      return true;
+    }
+    case RBK_GATE_EX: case RBK_GATE_EY: h.kind = OPK_MAT; return true;
+    case RBK_GATE_EZ: h.kind = OPK_DIAG; return true;
+    case RBK_GATE_SWAP:
+      h.kind = HK_SWAP;
+      h.target2 = static_cast<int8_t>(g.qubits[1]);
+      return true;
+    default: return false;
+  }
+}
+
+int rot_type(int kind) { return kind == RBK_GATE_EX ? 1 : kind == RBK_GATE_EY ? 2 : kind == RBK_GATE_EZ ? 3 : 0; }
+
+int sa_fail(int code, const std::string& m) { return set_last_error(code, m.c_str()); }
+
+size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
+
+int cluster_of(int n) { return n > kSaLocalBits ? 1 << (n - kSaLocalBits) : 1; }
+int threads_of(int n, int most)
+{
+  const int need = std::max(32, (1 << std::max(0, std::min(n, kSaLocalBits) - kSmallRegBits)));
+  return std::min(need, std::min(most, kSaThreads));
+}
+
+template <typename Real, int CS>
+cudaError_t launch_class(const sa_args& args, int first, int count, int n, int threads, cudaStream_t stream)
+{
+  const int local_bits = std::max(kSmallRegBits, std::min(n, kSaLocalBits));
+  const size_t smem = 2 * (sizeof(typename ctype<Real>::c) << local_bits);
+  static std::atomic<bool> configured[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(small_adjoint_kernel<Real, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(2 * (sizeof(typename ctype<Real>::c) << kSaLocalBits)));
+    if (e != cudaSuccess) return e;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(count) * CS);
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = CS;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = CS > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, small_adjoint_kernel<Real, CS>, args, first);
+}
+
+template <typename Real>
+cudaError_t launch_class(const sa_args& args, int first, int count, int n, int threads, cudaStream_t stream)
+{
+  switch (cluster_of(n)) {
+    case 1: return launch_class<Real, 1>(args, first, count, n, threads, stream);
+    case 2: return launch_class<Real, 2>(args, first, count, n, threads, stream);
+    case 4: return launch_class<Real, 4>(args, first, count, n, threads, stream);
+    case 8: return launch_class<Real, 8>(args, first, count, n, threads, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace
+
+bool sa_plan(int n, const rbk_circuit_gate* gates, int num_gates, int num_terms, const char* strings, const double* coeffs,
+             sa_program& out)
+{
+  if (n < 1 || n > kSmallAdjointBits) return false;
+  out = sa_program{};
+  out.n = n;
+  std::vector<hgate> queue(static_cast<size_t>(num_gates));
+  for (int i = 0; i < num_gates; ++i)
+    if (!lower_gate(n, gates[i], queue[static_cast<size_t>(i)])) return false;
+  std::vector<int> perm(static_cast<size_t>(n)), inv(static_cast<size_t>(n));
+  for (int q = 0; q < n; ++q) perm[static_cast<size_t>(q)] = inv[static_cast<size_t>(q)] = q;
+  plan_small_phases(n, queue, perm, inv, static_cast<size_t>(kSaPhaseOps),
+                    [&](const std::vector<small_op>& ops, const std::vector<size_t>& from, const small_phase& phase) {
+                      sa_phase ph{};
+                      std::memcpy(ph.reg, phase.reg, sizeof(ph.reg));
+                      ph.begin = static_cast<int32_t>(out.ops.size());
+                      for (size_t k = 0; k < ops.size(); ++k) {
+                        const rbk_circuit_gate& g = gates[from[k]];
+                        small_op o = ops[k];
+                        o.rot = static_cast<uint16_t>(rot_type(g.kind));
+                        if (o.rot) {
+                          o.real = o.rot == 2 ? 1 : 0;
+                          out.rots.push_back({static_cast<int32_t>(out.ops.size()), g.param, g.scale, g.angles[0]});
+                          if (g.param >= 0) {
+                            o.slot = static_cast<int32_t>(out.slot_param.size());
+                            out.slot_param.push_back(g.param);
+                            out.slot_scale.push_back(g.scale);
+                          }
+                        }
+                        out.ops.push_back(o);
+                      }
+                      ph.end = static_cast<int32_t>(out.ops.size());
+                      out.phases.push_back(ph);
+                    });
+  static const cplx pow_mi[4] = {{1, 0}, {0, -1}, {-1, 0}, {0, 1}};
+  for (int t = 0; t < num_terms; ++t) {
+    uint32_t x = 0, y = 0, z = 0;
+    for (int q = 0; q < n; ++q) {
+      const char c = strings[static_cast<size_t>(t) * static_cast<size_t>(n) + static_cast<size_t>(q)];
+      const uint32_t b = 1u << perm[static_cast<size_t>(q)];
+      if (c == 'X') x |= b;
+      else if (c == 'Y') y |= b;
+      else if (c == 'Z') z |= b;
+      else if (c != 'I') return false;
+    }
+    const cplx w = cplx{coeffs[2 * t], coeffs[2 * t + 1]} * pow_mi[__builtin_popcount(y) & 3];
+    out.terms.push_back({x | y, y | z, w.real(), w.imag()});
+  }
+  std::stable_sort(out.terms.begin(), out.terms.end(), [](const sa_term& a, const sa_term& b) { return a.flip < b.flip; });
+  return true;
+}
+
+int sa_set::fetch(cudaStream_t stream)
+{
+  if (cudaMemcpyAsync(h_out_, d_out_, sizeof(double) * (insts_.size() + size_t(slots_)), cudaMemcpyDeviceToHost, stream) != cudaSuccess)
+    return sa_fail(RBK_ERR_CUDA, "small adjoint: results");
+  return RBK_OK;
+}
+
+sa_set::~sa_set()
+{
+  if (h_out_) cudaFreeHost(h_out_);
+  if (d_image_) cudaFree(d_image_);
+  if (h_image_) cudaFreeHost(h_image_);
+  if (d_partial_) cudaFree(d_partial_);
+  if (d_out_) cudaFree(d_out_);
+}
+
+int sa_set::assign(int precision, const std::vector<const sa_program*>& programs, const double* theta, int num_theta,
+                   cudaStream_t stream)
+{
+  precision_ = precision;
+  std::vector<int> order(programs.size());
+  for (size_t i = 0; i < order.size(); ++i) order[i] = static_cast<int>(i);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return programs[size_t(a)]->n > programs[size_t(b)]->n; });
+  insts_.clear();
+  slot_begin_.assign(programs.size(), 0);
+  size_t ops = 0, phases = 0, rots = 0, terms = 0, partial = 0;
+  slots_ = 0;
+  for (int i : order) {
+    const sa_program& P = *programs[size_t(i)];
+    sa_inst I{};
+    I.n = P.n;
+    I.num_phases = int32_t(P.phases.size());
+    I.num_rots = int32_t(P.rots.size());
+    I.num_slots = int32_t(P.slot_param.size());
+    I.num_terms = int32_t(P.terms.size());
+    I.op_begin = int32_t(ops);
+    I.phase_begin = int32_t(phases);
+    I.rot_begin = int32_t(rots);
+    I.slot_begin = slots_;
+    I.term_begin = int32_t(terms);
+    I.theta_begin = P.theta_begin;
+    I.out = i;
+    I.partial_begin = int64_t(partial);
+    slot_begin_[size_t(i)] = slots_;
+    ops += P.ops.size();
+    phases += P.phases.size();
+    rots += P.rots.size();
+    terms += P.terms.size();
+    slots_ += I.num_slots;
+    partial += size_t(I.num_slots + 1) * size_t(cluster_of(P.n)) * size_t(threads_of(std::max(kSaClassBits, P.n), kSaThreads) / 32);
+    insts_.push_back(I);
+  }
+  if (ops > size_t(INT32_MAX) || terms > size_t(INT32_MAX)) return sa_fail(RBK_ERR_UNSUPPORTED, "batch: too many gates");
+  off_phase_ = align16(sizeof(sa_inst) * insts_.size());
+  off_rot_ = align16(off_phase_ + sizeof(sa_phase) * phases);
+  off_term_ = align16(off_rot_ + sizeof(sa_rot) * rots);
+  off_op_ = align16(off_term_ + sizeof(sa_term) * terms);
+  off_theta_ = align16(off_op_ + sizeof(small_op) * ops);
+  const size_t bytes = off_theta_ + sizeof(double) * size_t(theta ? num_theta : 0);
+  auto grow = [&](size_t want, size_t& cap, auto&& alloc) {
+    if (want <= cap) return true;
+    cap = 0;
+    if (!alloc(want + want / 4 + 256)) return false;
+    cap = want + want / 4 + 256;
+    return true;
+  };
+  const bool ok =
+    grow(bytes, image_cap_, [&](size_t n) {
+      if (d_image_) cudaFree(d_image_);
+      if (h_image_) cudaFreeHost(h_image_);
+      d_image_ = h_image_ = nullptr;
+      return cudaMalloc(reinterpret_cast<void**>(&d_image_), n) == cudaSuccess &&
+             cudaMallocHost(reinterpret_cast<void**>(&h_image_), n) == cudaSuccess;
+    }) &&
+    grow(partial, partial_cap_, [&](size_t n) {
+      if (d_partial_) cudaFree(d_partial_);
+      d_partial_ = nullptr;
+      return cudaMalloc(reinterpret_cast<void**>(&d_partial_), sizeof(double) * n) == cudaSuccess;
+    }) &&
+    grow(programs.size() + size_t(slots_), out_cap_, [&](size_t n) {
+      if (d_out_) cudaFree(d_out_);
+      if (h_out_) cudaFreeHost(h_out_);
+      d_out_ = h_out_ = nullptr;
+      return cudaMalloc(reinterpret_cast<void**>(&d_out_), sizeof(double) * n) == cudaSuccess &&
+             cudaMallocHost(reinterpret_cast<void**>(&h_out_), sizeof(double) * n) == cudaSuccess;
+    });
+  if (!ok) {
+    cudaGetLastError();
+    return sa_fail(RBK_ERR_OOM, "small adjoint: memory exhausted");
+  }
+  std::memcpy(h_image_, insts_.data(), sizeof(sa_inst) * insts_.size());
+  for (const sa_inst& I : insts_) {
+    const sa_program& P = *programs[size_t(I.out)];
+    std::memcpy(h_image_ + off_phase_ + sizeof(sa_phase) * size_t(I.phase_begin), P.phases.data(), sizeof(sa_phase) * P.phases.size());
+    std::memcpy(h_image_ + off_rot_ + sizeof(sa_rot) * size_t(I.rot_begin), P.rots.data(), sizeof(sa_rot) * P.rots.size());
+    std::memcpy(h_image_ + off_term_ + sizeof(sa_term) * size_t(I.term_begin), P.terms.data(), sizeof(sa_term) * P.terms.size());
+    std::memcpy(h_image_ + off_op_ + sizeof(small_op) * size_t(I.op_begin), P.ops.data(), sizeof(small_op) * P.ops.size());
+  }
+  if (theta && num_theta > 0) std::memcpy(h_image_ + off_theta_, theta, sizeof(double) * size_t(num_theta));
+  if (cudaMemcpyAsync(d_image_, h_image_, bytes, cudaMemcpyHostToDevice, stream) != cudaSuccess)
+    return sa_fail(RBK_ERR_CUDA, "small adjoint: upload");
+  return RBK_OK;
+}
+
+int sa_set::launch(const double* d_theta, int max_threads, cudaStream_t stream, const std::vector<cudaStream_t>& side,
+                   const std::vector<cudaEvent_t>& events)
+{
+  sa_args A{};
+  A.inst = reinterpret_cast<const sa_inst*>(d_image_);
+  A.phases = reinterpret_cast<const sa_phase*>(d_image_ + off_phase_);
+  A.rots = reinterpret_cast<const sa_rot*>(d_image_ + off_rot_);
+  A.terms = reinterpret_cast<const sa_term*>(d_image_ + off_term_);
+  A.ops = reinterpret_cast<small_op*>(d_image_ + off_op_);
+  A.theta = d_theta ? d_theta : reinterpret_cast<const double*>(d_image_ + off_theta_);
+  A.partial = d_partial_;
+  A.energy = d_out_;
+  A.overlaps = d_out_ + insts_.size();
+  // Classes of one launch shape: 15, 14, 13, 12, 11 and at most 10 qubits.
+  size_t used = 0;
+  for (size_t i = 0; i < insts_.size();) {
+    const int cls = std::max(kSaClassBits, insts_[i].n), n = insts_[i].n;  // the first is the largest of its class
+    size_t j = i;
+    while (j < insts_.size() && std::max(kSaClassBits, insts_[j].n) == cls) ++j;
+    cudaStream_t on = stream;
+    if (i > 0 && used < side.size()) {
+      on = side[used];
+      if (used == 0 && cudaEventRecord(events[0], stream) != cudaSuccess) return sa_fail(RBK_ERR_CUDA, "small adjoint: fork");
+      if (cudaStreamWaitEvent(on, events[0], 0) != cudaSuccess) return sa_fail(RBK_ERR_CUDA, "small adjoint: fork");
+      ++used;
+    }
+    const int threads = threads_of(n, max_threads);
+    const cudaError_t e = precision_ == RBK_C128 ? launch_class<double>(A, int(i), int(j - i), n, threads, on)
+                                                 : launch_class<float>(A, int(i), int(j - i), n, threads, on);
+    if (e != cudaSuccess) return sa_fail(RBK_ERR_CUDA, std::string("small adjoint: ") + cudaGetErrorString(e));
+    i = j;
+  }
+  for (size_t k = 0; k < used; ++k)
+    if (cudaEventRecord(events[1 + k], side[k]) != cudaSuccess || cudaStreamWaitEvent(stream, events[1 + k], 0) != cudaSuccess)
+      return sa_fail(RBK_ERR_CUDA, "small adjoint: join");
+  return RBK_OK;
+}
+
+}  // namespace rbk
