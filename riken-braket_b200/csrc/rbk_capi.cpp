@@ -186,7 +186,7 @@ int flush(rbk_state* s)
   try {
     if (s->n > rbk::kSmallBits) {
       std::vector<rbk::dev_pass> passes;
-      rbk::plan_passes(params_of(s), s->queue, s->perm, s->inv, passes);
+      rbk::plan_passes(params_of(s), rbk::simplify_queue(s->n, s->queue), s->perm, s->inv, passes);
       rc = run_passes(s, passes);
       if (rc) { s->queue.clear(); return rc; }
       s->stats.passes += passes.size();

@@ -39,6 +39,15 @@ struct plan_params {
   int factored_min = 3;    // layers of at least this many gates take the factored form (0: never)
 };
 
+// The same circuit with fewer and cheaper gates for the fused passes.  An
+// uncontrolled diagonal, X or Y gate is multiplied into the matrix before it on
+// its qubit where the gates between commute with it.  A matrix gives its right
+// factor to the matrix before it where the gates between commute with that
+// factor: a diagonal through controls and phases, an X rotation through CNOT
+// targets.  What is left of it is (diagonal) x (real rotation), which a factored
+// layer runs without pre factors (3/4 of its FP64 work).
+std::vector<hgate> simplify_queue(int n, const std::vector<hgate>& gates);
+
 // Plans `gates` (in order) into passes, updating the layout map
 // perm (logical -> physical) and inv (physical -> logical).
 void plan_passes(const plan_params& p, const std::vector<hgate>& gates, std::vector<int>& perm,
