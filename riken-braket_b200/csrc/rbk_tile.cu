@@ -143,17 +143,43 @@ __device__ __forceinline__ void cmul_acc(double& xr, double& xi, double dr, doub
   xr = t;
 }
 
+// Multiplies the amplitudes of the register slots with index bits i below bit B
+// fixed by f times the product of l over the slot's bits from B up, depth
+// first: 2^R - 1 products in all.  Bits of `common` are one in every slot that
+// takes a factor (their l is part of f).
+template <typename Real, int R, int B, int I>
+__device__ __forceinline__ void apply_products(typename ctype<Real>::c* a, uint32_t common, double fr, double fi,
+                                               const double* lr, const double* li)
+{
+  if constexpr (B == R) {
+    const double xr = double(a[I].x), xi = double(a[I].y);
+    a[I].x = static_cast<Real>(xr * fr - xi * fi);
+    a[I].y = static_cast<Real>(xr * fi + xi * fr);
+  } else if ((common >> B) & 1u) {
+    apply_products<Real, R, B + 1, I | (1 << B)>(a, common, fr, fi, lr, li);
+  } else {
+    apply_products<Real, R, B + 1, I>(a, common, fr, fi, lr, li);
+    cmul_acc(fr, fi, lr[B], li[B]);
+    apply_products<Real, R, B + 1, I | (1 << B)>(a, common, fr, fi, lr, li);
+  }
+}
+
 // A run of phase gates (PHASES header; rbk_plan.cpp group_phase_runs): gate k
 // multiplies the amplitudes whose bits creg / cthr / cout are all one by its
-// factor (m[2], m[3]).  The members come sorted by accumulator, with the class
-// sizes in the header's dout: gates on no register bit multiply the thread's
-// accumulator, gates on one register bit b that of b, and every amplitude takes
-// the product of its accumulators once at the end; gates on two or more
-// register bits (the rest of the run) multiply their amplitudes directly.
+// factor (m[2], m[3]).  Register bits that every gate of the run has (the
+// header's creg) select the amplitudes once; by its further register bits a gate
+// multiplies the thread's accumulator (none), that of one register bit, or its
+// amplitudes directly (two or more: the rest of the run).  Every amplitude takes
+// the product of its accumulators once at the end.  The members come sorted that
+// way, with the class sizes in the header's m[0], one byte each.
 // Accumulation in double for both precisions.
+//   The products of the accumulators, 2^R - 1 complex multiplies of a tree over
+// the register bits, replace R / 2 per amplitude; the common bits halve the
+// amplitudes of a run such as the QFT's phases behind one Hadamard, which were
+// also multiplied one gate after the other where both qubits were register bits.
 template <typename Real, int R>
 __device__ __forceinline__ void apply_phase_run(typename ctype<Real>::c* a, const dev_op* run, int count,
-                                                uint64_t classes, uint32_t tid, uint64_t base)
+                                                uint64_t classes, uint32_t common, uint32_t tid, uint64_t base)
 {
   constexpr int NR = 1 << R;
   double fr = 1.0, fi = 0.0;
@@ -186,16 +212,7 @@ __device__ __forceinline__ void apply_phase_run(typename ctype<Real>::c* a, cons
       a[i].y = static_cast<Real>(xi);
     }
   }
-#pragma unroll
-  for (int i = 0; i < NR; ++i) {
-    double pr = fr, pi = fi;
-#pragma unroll
-    for (int b = 0; b < R; ++b)
-      if ((i >> b) & 1) cmul_acc(pr, pi, lr[b], li[b]);
-    const double xr = double(a[i].x), xi = double(a[i].y);
-    a[i].x = static_cast<Real>(xr * pr - xi * pi);
-    a[i].y = static_cast<Real>(xr * pi + xi * pr);
-  }
+  apply_products<Real, R, 0, 0>(a, common, fr, fi, lr, li);
 }
 
 // One gate of a LAYER on register bit B, in the layer's matrix form.
@@ -355,7 +372,8 @@ __device__ __forceinline__ int apply_op(typename ctype<Real>::c* a, const dev_op
       break;
     }
     case op_code(OPK_PHASES, 0, true, 0):
-      apply_phase_run<Real, R>(a, &op + 1, static_cast<int>(op.run), op.dout, tid, base);
+      apply_phase_run<Real, R>(a, &op + 1, static_cast<int>(op.run), static_cast<uint64_t>(__double_as_longlong(op.m[0])), creg,
+                               tid, base);
       return static_cast<int>(op.run);
 #define RBK_LAYER_CASE(FORM, FULL) \
     case op_code(OPK_LAYER, FORM, FULL, 0): \
