@@ -26,6 +26,9 @@ class CircuitGate(ctypes.Structure):
 def gate_array(spec):
     """spec: list of (mnemonic, qubits, param_index or None, scale, angles)."""
     arr = (CircuitGate * max(1, len(spec)))()
+    if rbk.marshal():
+        rbk.marshal().fill_gates(ctypes.addressof(arr), spec, GATE)
+        return arr, len(spec)
     for i, (mnem, qubits, param, scale, angles) in enumerate(spec):
         g = arr[i]
         g.kind = GATE[mnem]

@@ -144,15 +144,13 @@ int mark_launch_start(rbk_state* s)
   return RBK_OK;
 }
 
-int run_passes(rbk_state* s, const std::vector<rbk::dev_pass>& passes)
+int run_pass(rbk_state* s, const rbk::dev_pass& pass)
 {
-  for (const auto& pass : passes) {
-    const cudaError_t e = s->precision == RBK_C128
-      ? rbk::launch_tile_pass<double>(s->amps, s->n, pass, s->shape, s->stream)
-      : rbk::launch_tile_pass<float>(s->amps, s->n, pass, s->shape, s->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "tile pass launch");
-    ++s->stats.kernel_launches;
-  }
+  const cudaError_t e = s->precision == RBK_C128
+    ? rbk::launch_tile_pass<double>(s->amps, s->n, pass, s->shape, s->stream)
+    : rbk::launch_tile_pass<float>(s->amps, s->n, pass, s->shape, s->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "tile pass launch");
+  ++s->stats.kernel_launches;
   return RBK_OK;
 }
 
@@ -185,11 +183,15 @@ int flush(rbk_state* s)
   if (rc) return rc;
   try {
     if (s->n > rbk::kSmallBits) {
-      std::vector<rbk::dev_pass> passes;
-      rbk::plan_passes(params_of(s), rbk::simplify_queue(s->n, s->queue), s->perm, s->inv, passes);
-      rc = run_passes(s, passes);
+      // Each pass is launched as soon as it is planned: the device works on the
+      // first while the host plans the rest (20-qubit brick, 17 passes: 0.37 ms of
+      // planning before the first launch otherwise).
+      rbk::plan_passes(params_of(s), rbk::simplify_queue(s->n, s->queue), s->perm, s->inv, [&](const rbk::dev_pass& pass) {
+        rc = run_pass(s, pass);
+        if (!rc) ++s->stats.passes;
+        return rc == RBK_OK;
+      });
       if (rc) { s->queue.clear(); return rc; }
-      s->stats.passes += passes.size();
     } else if ((rc = run_small(s, s->queue, &s->stats.passes))) {
       s->queue.clear();
       return rc;
@@ -253,8 +255,8 @@ int move_layout(rbk_state* s, const std::vector<int>& target)
   }
   rc = mark_launch_start(s);
   if (rc) return rc;
-  rc = run_passes(s, passes);
-  if (rc) return rc;
+  for (const auto& pass : passes)
+    if ((rc = run_pass(s, pass))) return rc;
   s->stats.relabel_passes += passes.size();
   RBK_CUDA(cudaEventRecord(s->ev_last, s->stream));
   return RBK_OK;

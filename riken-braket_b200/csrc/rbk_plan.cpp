@@ -1143,6 +1143,16 @@ std::vector<hgate> simplify_queue(int n, const std::vector<hgate>& gates)
 void plan_passes(const plan_params& p, const std::vector<hgate>& gates, std::vector<int>& perm,
                  std::vector<int>& inv, std::vector<dev_pass>& out)
 {
+  plan_passes(p, gates, perm, inv, [&](const dev_pass& pass) {
+    out.push_back(pass);
+    return true;
+  });
+}
+
+bool plan_passes(const plan_params& p, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv,
+                 const std::function<bool(const dev_pass&)>& emit)
+{
+  dev_pass pass;
   const uint64_t all = p.n >= 64 ? ~0ull : bit(p.n) - 1;
   const uint64_t low_mask = bit(p.LOW) - 1;
   std::vector<char> taken(gates.size(), 0);
@@ -1278,9 +1288,10 @@ void plan_passes(const plan_params& p, const std::vector<hgate>& gates, std::vec
     }
     int relabel_to[16];
     apply_relabel(p, tile_phys, new_phys, perm, inv, relabel_to);
-    out.emplace_back();
-    build_pass(p, tile, ops, relabel_to, tile_phys, out.back());
+    build_pass(p, tile, ops, relabel_to, tile_phys, pass);
+    if (!emit(pass)) return false;
   }
+  return true;
 }
 
 void plan_layout(const plan_params& p, std::vector<int>& perm, std::vector<int>& inv, const std::vector<int>& target,

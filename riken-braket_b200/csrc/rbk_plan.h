@@ -52,6 +52,10 @@ std::vector<hgate> simplify_queue(int n, const std::vector<hgate>& gates);
 // perm (logical -> physical) and inv (physical -> logical).
 void plan_passes(const plan_params& p, const std::vector<hgate>& gates, std::vector<int>& perm,
                  std::vector<int>& inv, std::vector<dev_pass>& out);
+// The same, each pass handed to emit as soon as it is planned (perm and inv are
+// those after it); emit returning false ends the planning, as does the result.
+bool plan_passes(const plan_params& p, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv,
+                 const std::function<bool(const dev_pass&)>& emit);
 
 // Passes that only move data so that perm becomes `target` (a permutation of
 // 0..n-1: logical qubit q on physical bit target[q]); the multi-qubit form of
