@@ -107,6 +107,17 @@ bool get_real(PyObject* seq, Py_ssize_t i, double* out)
   return !PyErr_Occurred();
 }
 
+// As float(x) takes it: strings of digits too.
+bool get_float(PyObject* seq, Py_ssize_t i, double* out)
+{
+  PyObject* o = item(seq, i);
+  PyObject* v = o ? PyNumber_Float(o) : nullptr;
+  if (!v) return false;
+  *out = PyFloat_AS_DOUBLE(v);
+  Py_DECREF(v);
+  return true;
+}
+
 // int(value) of element i.
 bool get_int(PyObject* seq, Py_ssize_t i, int* out)
 {
@@ -239,8 +250,8 @@ PyObject* py_fill_gates(PyObject*, PyObject* args)
       if ((ok = get_int(q, j, &v))) r.qubits[j] = v;
     r.param = -1;
     if (ok && item(g, 2) != Py_None && (ok = get_int(g, 2, &v))) r.param = v;
-    ok = ok && get_real(g, 3, &r.scale);
-    for (Py_ssize_t j = 0; ok && j < 3 && j < PySequence_Fast_GET_SIZE(angles); ++j) ok = get_real(angles, j, &r.angles[j]);
+    ok = ok && get_float(g, 3, &r.scale);
+    for (Py_ssize_t j = 0; ok && j < 3 && j < PySequence_Fast_GET_SIZE(angles); ++j) ok = get_float(angles, j, &r.angles[j]);
     if (!ok) break;
     out[k] = r;
   }
