@@ -1411,6 +1411,13 @@ struct rbk::adjoint_workspace {
   double* mpart = nullptr;
   double* tpart = nullptr;  // tiled overlaps (n >= tile bits)
   double* ppart = nullptr;  // Z sums and pair sums (n >= 8 + kPairRegBits)
+  // Pair-rotate launches whose overlaps are not formed yet: their partial sums
+  // (kRotateLaunches launches' worth) and what these mean, also in device memory.
+  double* rpart = nullptr;
+  size_t rused = 0;
+  std::vector<pair_rotate_result> rresults;
+  pair_rotate_result* d_rresults = nullptr;
+  pair_rotate_result* h_rresults = nullptr;  // pinned
   std::unique_ptr<sa_set> small;  // n <= kSmallAdjointBits
   ~adjoint_workspace()
   {
@@ -1420,6 +1427,9 @@ struct rbk::adjoint_workspace {
     if (mpart) cudaFree(mpart);
     if (tpart) cudaFree(tpart);
     if (ppart) cudaFree(ppart);
+    if (rpart) cudaFree(rpart);
+    if (d_rresults) cudaFree(d_rresults);
+    if (h_rresults) cudaFreeHost(h_rresults);
     if (lam) rbk_state_destroy(lam);
     if (psi) rbk_state_destroy(psi);
   }
@@ -1577,16 +1587,47 @@ bool owed_from_queue(const rbk_state* s, rbk::pre_diag& o)
   return true;
 }
 
+// Partial sums kept before the overlaps are formed: 64 launches' worth, 8 MB.
+constexpr int kRotateLaunches = 64;
+constexpr size_t kRotateResults = size_t(kRotateLaunches) * (rbk::kMaxRotFlips + rbk::kMaxQubits);
+
+// Forms the overlaps of the pair-rotate launches made so far.  `last`: the sweep
+// ends, and the pinned entries are next written after the caller's wait; before
+// that, a wait keeps them until they are copied.
+int finish_rotations(rbk::adjoint_workspace& w, rbk_state* psi, double* ov, bool last)
+{
+  if (w.rresults.empty()) return RBK_OK;
+  const size_t count = w.rresults.size();
+  std::copy(w.rresults.begin(), w.rresults.end(), w.h_rresults);
+  RBK_CUDA(cudaMemcpyAsync(w.d_rresults, w.h_rresults, sizeof(rbk::pair_rotate_result) * count, cudaMemcpyHostToDevice, psi->stream));
+  RBK_CUDA(rbk::launch_finish_pair_rotate(w.rpart, w.d_rresults, static_cast<int>(count), ov, psi->stream));
+  w.rresults.clear();
+  w.rused = 0;
+  return last ? RBK_OK : bounded_sync(psi);
+}
+
 // Pair-rotate launches over `items` (rbk::plan_rotations), the owed diagonal,
 // if any, in the first.
-int launch_rotations(const rbk::adjoint_workspace& w, rbk_state* lam, rbk_state* psi,
+int launch_rotations(rbk::adjoint_workspace& w, rbk_state* lam, rbk_state* psi,
                      const std::vector<rbk::rotate_item>& items, double* ov, const rbk::pre_diag* owed)
 {
   const bool c128 = w.precision == RBK_C128;
+  const size_t room = kRotateLaunches * rbk::pair_rotate_partials_doubles();
+  if (!w.rpart) {
+    RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&w.rpart), sizeof(double) * room));
+    RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&w.d_rresults), sizeof(rbk::pair_rotate_result) * kRotateResults));
+    RBK_CUDA(cudaMallocHost(reinterpret_cast<void**>(&w.h_rresults), sizeof(rbk::pair_rotate_result) * kRotateResults));
+  }
   for (const rbk::pair_rotate_set& set : rbk::plan_rotations(w.n, items, owed)) {
-    const cudaError_t e = c128 ? rbk::launch_pair_rotate<double>(lam->amps, psi->amps, w.n, set, w.ppart, ov, psi->stream)
-                               : rbk::launch_pair_rotate<float>(lam->amps, psi->amps, w.n, set, w.ppart, ov, psi->stream);
+    if (w.rused + rbk::pair_rotate_partials_doubles() > room ||
+        w.rresults.size() + rbk::kMaxRotFlips + rbk::kMaxQubits > kRotateResults)
+      if (int rc = finish_rotations(w, psi, ov, false)) return rc;
+    size_t used = 0;
+    const cudaError_t e = c128
+      ? rbk::launch_pair_rotate<double>(lam->amps, psi->amps, w.n, set, w.rpart, w.rused, w.rresults, &used, psi->stream)
+      : rbk::launch_pair_rotate<float>(lam->amps, psi->amps, w.n, set, w.rpart, w.rused, w.rresults, &used, psi->stream);
     if (e != cudaSuccess) return cuda_fail(e, "pair rotations");
+    w.rused += used;
   }
   return RBK_OK;
 }
@@ -1835,7 +1876,12 @@ int rbk::adjoint_run(adjoint_workspace* w, const rbk_circuit_gate* gates, int nu
       return RBK_OK;
     }
     if (int rc = rbk_state_reset(psi.s, 0)) return rc;
-    if (int rc = rbk_state_reset(lam.s, 0)) return rc;
+    // lambda's amplitudes are written whole by H psi: only its queue and layout map start anew.
+    lam.s->queue.clear();
+    lam.s->in_fusion = false;
+    for (int q = 0; q < num_qubits; ++q) lam.s->perm[q] = lam.s->inv[q] = q;
+    w->rresults.clear();  // of a sweep that ended in an error
+    w->rused = 0;
 
     int num_pg = 0;
     for (int i = 0; i < num_gates; ++i) num_pg += gates[i].param >= 0 ? 1 : 0;
@@ -2057,6 +2103,7 @@ int rbk::adjoint_run(adjoint_workspace* w, const rbk_circuit_gate* gates, int nu
       i = j;
     }
     if (int rc = settle_z()) return rc;
+    if (int rc = finish_rotations(*w, psi.s, ov.p, true)) return rc;
     std::vector<double> host(2 * (num_pg + 1));
     RBK_CUDA(cudaMemcpyAsync(host.data(), ov.p, sizeof(double) * host.size(), cudaMemcpyDeviceToHost, psi.s->stream));
     if (int rc = bounded_sync(psi.s)) return rc;

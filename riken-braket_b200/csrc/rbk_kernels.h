@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include "rbk_internal.h"
 
@@ -208,8 +209,20 @@ struct pair_rotate_set {
   pre_diag pre;
 };
 size_t pair_rotate_partials_doubles();  // per block: nflips overlap sums, then 1 + n Z sums when pre.nz > 0
-template <typename Real> cudaError_t launch_pair_rotate(void* lam, void* psi, int n, const pair_rotate_set& set,
-                                                        double* partials, double* out, cudaStream_t stream);
+// A launch leaves its partial sums at partials[begin ..] (*used doubles of them)
+// and adds what they mean to `results`; launch_finish_pair_rotate forms the
+// overlaps of many launches at once (a finish after each took 5 us and a launch,
+// 48 times in a 20-qubit gradient of 16 layers).
+struct pair_rotate_result {
+  uint64_t begin;
+  int32_t blocks, width, column, second, slot, pad;
+  double w;
+};
+template <typename Real> cudaError_t launch_pair_rotate(void* lam, void* psi, int n, const pair_rotate_set& set, double* partials,
+                                                        size_t begin, std::vector<pair_rotate_result>& results, size_t* used,
+                                                        cudaStream_t stream);
+cudaError_t launch_finish_pair_rotate(const double* partials, const pair_rotate_result* entries, int count, double* out,
+                                      cudaStream_t stream);
 template <typename Real> cudaError_t launch_zsum2(const void* lam, const void* psi, int n, const zsum2_set& set,
                                                   double* partials, double* out, cudaStream_t stream);
 template <typename Real> cudaError_t launch_pair_overlaps(const void* lam, const void* psi, int n, const pair_overlap_set& set,
