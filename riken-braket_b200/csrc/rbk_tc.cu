@@ -16,7 +16,7 @@
 // tensor cores.  This is the bra-fused 2^k x 2^k unitary of a fusion block
 // (bra/src/nompi_state.cpp:1285-1357 replays the gates instead).
 //
-// One CTA per SM (persistent), 288 threads in three roles that meet at
+// One CTA per SM (persistent), 672 threads in three roles that meet at
 // mbarriers (see the kernel): producer warps stream K quarters of 128-row
 // tiles from HBM, kTcDepth quarters ahead in registers, and split them into
 // A_hi / A_lo operand slots; one thread issues the tcgen05.mma of each quarter;
@@ -36,8 +36,15 @@
 namespace rbk {
 namespace {
 
-constexpr int kTcThreads = 288;  // 4 producer, 4 epilogue and 1 MMA warp
-constexpr int kTcDepth = 3;       // K quarters whose loads are in flight
+// Bound by the loads in flight, then by shared memory (87 % of its bandwidth at
+// targets 0-5, half of it bank conflicts of the operand stores and the epilogue's
+// turn-around): a producer thread holds PER_THREAD float4 per quarter in flight.
+// 27 qubits, 2^31 B read and written: 4 warps 3 quarters deep 2540 / 2842 / 2329
+// GB/s (targets 0-5 / spread / k = 5), 8 warps 5 deep 3069 / 3336 / 2715, 16 warps
+// 6 deep 3197 / 3458 / 2740.
+constexpr int kTcProducers = 16;  // producer warps
+constexpr int kTcThreads = (kTcProducers + 5) * 32;  // and 4 epilogue warps and 1 MMA warp
+constexpr int kTcDepth = 6;       // K quarters whose loads are in flight
 constexpr int kTcM = 128;
 constexpr uint32_t kWaitLimit = 1u << 22;
 
@@ -147,15 +154,15 @@ unitary_tf32x3_kernel(float2* __restrict__ state, uint64_t rows, const float4* _
                       const __grid_constant__ tc_layout L)
 {
   // Warp roles, all running at once and meeting at mbarriers:
-  //   warps 0-3 (producers): load a K quarter ("stage") of the CTA's next
+  //   warps 0 .. kTcProducers - 1 (producers): load a K quarter ("stage") of the CTA's next
   //     128-row tile from HBM into registers, kTcDepth stages ahead, split it
   //     into TF32 hi / lo and store both into A slot (stage % 2), then arrive
   //     on full[slot];
-  //   warp 8 (MMA issuer, one thread): for each stage wait full[slot], issue
+  //   the last warp (MMA issuer, one thread): for each stage wait full[slot], issue
   //     the 3 x K/32 tcgen05.mma into accumulator (tile % 2) and commit to
   //     empty[slot]; after a tile's fourth stage also commit to acc_full[acc];
-  //   warps 4-7 (epilogue): wait acc_full[acc], read the accumulator rows
-  //     (warp 4 + q owns TMEM lanes 32q..32q+31), write them back to HBM and
+  //   the four warps between (epilogue): wait acc_full[acc], read the accumulator rows
+  //     (the q-th owns TMEM lanes 32q..32q+31), write them back to HBM and
   //     arrive on acc_empty[acc] for the MMA issuer.
   // The producers stream the next tile while the tensor cores multiply and
   // the epilogue stores the previous one.
@@ -164,10 +171,10 @@ unitary_tf32x3_kernel(float2* __restrict__ state, uint64_t rows, const float4* _
   constexpr uint32_t SBO_A = (KQ / 4) * 128u, SBO_B = (K / 4) * 128u;
   constexpr uint32_t NCOLS = 2 * N;  // two FP32 accumulators of 128 lanes x N columns
   constexpr uint32_t CG = KQ / 16;   // groups of 4 float4 per row quarter
-  constexpr uint32_t PROD_WARPS = 4, PROD_THREADS = PROD_WARPS * 32, EPI_THREADS = 128, MMA_WARP = 8;
+  constexpr uint32_t PROD_WARPS = kTcProducers, PROD_THREADS = PROD_WARPS * 32, EPI_THREADS = 128, MMA_WARP = PROD_WARPS + 4;
   constexpr uint32_t PER_THREAD = (kTcM / 8) * CG / PROD_WARPS;  // float4 per producer thread per stage
   static_assert(PER_THREAD * PROD_WARPS == (kTcM / 8) * CG, "stage split over the producer warps");
-  static_assert(kTcThreads == 9 * 32, "4 producer warps, 4 epilogue warps, 1 MMA warp");
+  static_assert(PROD_WARPS % 4 == 0, "an epilogue warp reads the TMEM lanes of its index modulo 4");
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* b_hi = smem;
   unsigned char* b_lo = smem + B_BYTES;
@@ -326,7 +333,7 @@ unitary_tf32x3_kernel(float2* __restrict__ state, uint64_t rows, const float4* _
       if (!mbar_wait_bounded(smem_addr(&done), 0u)) atomicExch(error_flag, 1);
     }
   } else {
-    // Epilogue: warp 4 + q reads TMEM lanes 32q .. 32q + 31 (its rows), 32 columns at a time, and
+    // Epilogue: its warp q reads TMEM lanes 32q .. 32q + 31 (its rows), 32 columns at a time, and
     // turns them around in its 4 KB of shared memory so that 8 lanes write one row's 128 bytes
     // (lane = row would put the 32 lanes of a store 512 bytes apart).  The float4 slots of a
     // staged row are XOR-swizzled by the row, which keeps both sides free of bank conflicts.
