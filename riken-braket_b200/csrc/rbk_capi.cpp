@@ -1856,8 +1856,8 @@ int rbk::adjoint_run(adjoint_workspace* w, const rbk_circuit_gate* gates, int nu
     device_guard dg(w->device);
     // Small circuits run in one launch (RBK_ADJOINT_PAIR_ROTATE, which selects among
     // the engine's sweeps, keeps to those).  The line lies where the sweep's launches
-    // over several SMs catch up with one SM (10 layers, one gradient): 4.2 ms in
-    // launches against 0.85 ms at 10 qubits, 0.97 against 1.11 ms at 12.
+    // over several SMs catch up with one SM (10 layers, one gradient): 0.90 ms in
+    // launches against 0.32 ms at 10 qubits, 0.39 each at 11, 0.52 against 0.57 ms at 12.
     constexpr int kOneLaunchBits = 10;
     bool one_launch = num_qubits <= kOneLaunchBits && !std::getenv("RBK_ADJOINT_PAIR_ROTATE");
     for (int i = 0; i < num_gates && one_launch; ++i)

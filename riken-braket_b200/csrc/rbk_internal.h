@@ -200,18 +200,29 @@ struct dev_pass {
 constexpr int kSmallBits = 12;    // 2^12 complex<double> = 64 KB
 constexpr int kSmallRegBits = 3;  // states of fewer qubits are padded to this
 constexpr int kSmallGates = 368;  // gates of one launch (32 KB of kernel parameters is the most)
-struct alignas(8) small_op {
+// The record's first 16 bytes are one shared-memory load; `code` is the kernels'
+// dispatch (target register bit included), `act` has a bit for every register
+// slot whose register-bit controls are one, `hi` for every slot whose target bit is.
+enum small_code : uint8_t {
+  SMALL_MAT = 0,    // + target register bit: any 2x2 matrix
+  SMALL_REAL = 3,   // + target: a real one
+  SMALL_X = 6,      // + target
+  SMALL_Y = 9,      // + target
+  SMALL_DIAG = 12,  // diag(d0, d1)
+  SMALL_DIAG1 = 13, // diag(1, d1)
+  SMALL_NEG = 14    // -1 where the controls are one
+};
+struct alignas(16) small_op {
+  uint8_t code, act, hi;
+  uint8_t rot;       // adjoint sweeps: 1, 2, 3 = a rotation of X, Y, Z type, 0 = none
+  uint16_t cbase, dbase;
+  int32_t slot;      // adjoint sweeps: the number of the overlap taken at this gate, or -1
   uint8_t kind;      // op_kind
   uint8_t treg;      // MAT/X/Y: target register bit
-  uint8_t real;      // MAT: every entry is real
-  uint8_t diag_one;  // DIAG: d0 == 1 exactly
   uint8_t creg, dreg;
-  uint16_t cbase, dbase;
-  uint16_t rot;      // adjoint sweeps: 1, 2, 3 = a rotation of X, Y, Z type whose overlap is taken, 0 = none
-  int32_t slot;      // ... and the overlap's number
   double m[8];
 };
-struct small_phase {
+struct alignas(8) small_phase {
   uint8_t reg[kSmallRegBits];
   uint8_t pad;
   uint16_t begin, end;

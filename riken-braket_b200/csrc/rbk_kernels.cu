@@ -17,6 +17,7 @@
 #include "rbk_device.cuh"
 #include "rbk_internal.h"
 #include "rbk_kernels.h"
+#include "rbk_small_core.cuh"
 
 namespace rbk {
 
@@ -39,35 +40,9 @@ namespace rbk {
 template <int CAP>
 struct small_params {
   uint32_t num_ops, num_phases;
-  small_phase phases[CAP];
+  alignas(8) small_phase phases[CAP];
   small_op ops[CAP];
 };
-
-template <int B>
-__device__ __forceinline__ void small_target(double2 (&a)[1 << kSmallRegBits], const small_op& o)
-{
-  const uint32_t creg = o.creg;
-#pragma unroll
-  for (int i = 0; i < (1 << kSmallRegBits); ++i) {
-    if (i & (1 << B)) continue;
-    if ((uint32_t(i) & creg) != creg) continue;
-    double2 &x = a[i], &y = a[i | (1 << B)];
-    const double2 a0 = x, a1 = y;
-    if (o.kind == OPK_X) {
-      x = a1;
-      y = a0;
-    } else if (o.kind == OPK_Y) {
-      x = double2{a1.y, -a1.x};
-      y = double2{-a0.y, a0.x};
-    } else if (o.real) {
-      x = rmac2(a0, a1, o.m[0], o.m[2]);
-      y = rmac2(a0, a1, o.m[4], o.m[6]);
-    } else {
-      x = cmac2(a0, a1, o.m[0], o.m[1], o.m[2], o.m[3]);
-      y = cmac2(a0, a1, o.m[4], o.m[5], o.m[6], o.m[7]);
-    }
-  }
-}
 
 constexpr int kSmallCircuitThreads = 512;  // 1024 (64 registers) spilled
 template <typename Real, int CAP>
@@ -80,6 +55,7 @@ small_circuit_kernel(typename ctype<Real>::c* __restrict__ state, int n, const _
   double2* s = reinterpret_cast<double2*>(smem_raw);
   const uint32_t size = 1u << n, padded = max(size, uint32_t(NR));
   small_op* ops = reinterpret_cast<small_op*>(s + padded);
+  __shared__ small_phase phases[CAP];  // indexed by the phase: a constant-cache miss per line otherwise
   {
     // Through a generic pointer: the threads read the parameter block side by side,
     // where indexing it by the thread would go word by word through the constant cache.
@@ -87,6 +63,9 @@ small_circuit_kernel(typename ctype<Real>::c* __restrict__ state, int n, const _
     asm volatile("" : "+l"(src));
     uint64_t* dst = reinterpret_cast<uint64_t*>(ops);
     for (uint32_t i = threadIdx.x; i < P.num_ops * uint32_t(sizeof(small_op) / 8); i += blockDim.x) dst[i] = src[i];
+    const uint64_t* psrc = reinterpret_cast<const uint64_t*>(P.phases);
+    asm volatile("" : "+l"(psrc));
+    for (uint32_t i = threadIdx.x; i < P.num_phases; i += blockDim.x) reinterpret_cast<uint64_t*>(phases)[i] = psrc[i];
   }
   // Slots are swizzled (smem_slot) so that the lanes of a phase reach distinct banks whichever bits it holds.
   for (uint32_t i = threadIdx.x; i < padded; i += blockDim.x) {
@@ -99,7 +78,7 @@ small_circuit_kernel(typename ctype<Real>::c* __restrict__ state, int n, const _
   }
   __syncthreads();
   for (uint32_t p = 0; p < P.num_phases; ++p) {
-    const small_phase ph = P.phases[p];
+    const small_phase ph = phases[p];
     uint32_t rs[kSmallRegBits];
 #pragma unroll
     for (int k = 0; k < kSmallRegBits; ++k) rs[k] = smem_slot<0>(1u << ph.reg[k]);
@@ -117,27 +96,14 @@ small_circuit_kernel(typename ctype<Real>::c* __restrict__ state, int n, const _
           if ((i >> k) & 1) x ^= rs[k];
         a[i] = s[x];
       }
+      uint32_t signs = 0;
+      small_header h = small_load_header(ops + ph.begin);
       for (uint32_t g = ph.begin; g < ph.end; ++g) {
-        const small_op& o = ops[g];
-        if ((base & o.cbase) != o.cbase) continue;
-        if (o.kind == OPK_DIAG || o.kind == OPK_NEG) {
-          const uint32_t creg = o.creg, dreg = o.dreg;
-          const bool hi = (base & o.dbase) != 0, neg = o.kind == OPK_NEG, one = o.diag_one;
-#pragma unroll
-          for (int i = 0; i < NR; ++i) {
-            if ((uint32_t(i) & creg) != creg) continue;
-            if (neg) a[i] = double2{-a[i].x, -a[i].y};
-            else if (hi || (uint32_t(i) & dreg)) a[i] = cmul(a[i], double2{o.m[2], o.m[3]});
-            else if (!one) a[i] = cmul(a[i], double2{o.m[0], o.m[1]});
-          }
-        } else if (o.treg == 0) {
-          small_target<0>(a, o);
-        } else if (o.treg == 1) {
-          small_target<1>(a, o);
-        } else {
-          small_target<2>(a, o);
-        }
+        const small_header next = small_load_header(ops + min(g + 1, P.num_ops - 1));
+        small_gate<false, false>(a, a, h, ops + g, base, signs);
+        h = next;
       }
+      if (signs) small_signs(a, signs);
 #pragma unroll
       for (int i = 0; i < NR; ++i) {
         uint32_t x = sb;

@@ -910,6 +910,7 @@ void apply_relabel(const plan_params& p, const int* tile_phys, const int* new_ph
 }  // namespace
 
 void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv, size_t max_ops,
+                       const std::vector<char>& marked, int max_marked,
                        const std::function<void(const std::vector<small_op>&, const std::vector<size_t>&, const small_phase&)>& emit)
 {
   std::vector<char> taken(gates.size(), 0);
@@ -921,6 +922,7 @@ void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>&
     while (first < gates.size() && taken[first]) ++first;
     if (first >= gates.size()) break;
     uint64_t blockN = 0, blockZ = 0, regs = 0;
+    int marks = 0;
     mine.clear();
     for (size_t i = first; i < gates.size() && mine.size() < max_ops; ++i) {
       if (taken[i]) continue;
@@ -937,13 +939,15 @@ void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>&
       }
       const uint64_t t = is_target_kind(g.kind) ? bit(perm[g.target]) : 0;
       const uint64_t z = map_mask(g.cmask, perm) | (g.kind == OPK_DIAG ? bit(perm[g.target]) : 0);
-      if ((t & (blockN | blockZ)) || (z & blockN) || (t && !(regs & t) && popc(regs) >= kSmallRegBits)) {
+      if ((t & (blockN | blockZ)) || (z & blockN) || (t && !(regs & t) && popc(regs) >= kSmallRegBits) ||
+          (!marked.empty() && marked[i] && marks >= max_marked)) {
         blockN |= t;
         blockZ |= z;
         if ((blockN & all) == all) break;
         continue;
       }
       regs |= t;
+      if (!marked.empty() && marked[i]) ++marks;
       mine.push_back(i);
       taken[i] = 1;
     }
@@ -962,19 +966,25 @@ void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>&
       const hgate& g = gates[i];
       small_op o{};
       o.kind = g.kind;
-      o.diag_one = g.diag_one;
       o.slot = -1;
       std::memcpy(o.m, g.m, sizeof(o.m));
       const uint64_t c = map_mask(g.cmask, perm);
       o.creg = reg_mask(c);
       o.cbase = static_cast<uint16_t>(c & ~regs);
       if (is_target_kind(g.kind)) {
-        const uint8_t tm = reg_mask(bit(perm[g.target]));
-        o.treg = static_cast<uint8_t>(__builtin_ctz(tm));
-        o.real = g.m[1] == 0.0 && g.m[3] == 0.0 && g.m[5] == 0.0 && g.m[7] == 0.0;
+        o.treg = static_cast<uint8_t>(__builtin_ctz(reg_mask(bit(perm[g.target]))));
+        const bool real = g.m[1] == 0.0 && g.m[3] == 0.0 && g.m[5] == 0.0 && g.m[7] == 0.0;
+        o.code = static_cast<uint8_t>((g.kind == OPK_X ? SMALL_X : g.kind == OPK_Y ? SMALL_Y : real ? SMALL_REAL : SMALL_MAT) + o.treg);
       } else if (g.kind == OPK_DIAG) {
         o.dreg = reg_mask(bit(perm[g.target]));
         o.dbase = static_cast<uint16_t>(bit(perm[g.target]) & ~regs);
+        o.code = static_cast<uint8_t>(g.diag_one ? SMALL_DIAG1 : SMALL_DIAG);
+      } else {
+        o.code = SMALL_NEG;
+      }
+      for (int i2 = 0; i2 < (1 << kSmallRegBits); ++i2) {
+        if ((i2 & o.creg) == o.creg) o.act |= static_cast<uint8_t>(1u << i2);
+        if (i2 & o.dreg) o.hi |= static_cast<uint8_t>(1u << i2);
       }
       ops.push_back(o);
     }
@@ -985,7 +995,7 @@ void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>&
 void plan_small(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv,
                 std::vector<small_program>& out)
 {
-  plan_small_phases(n, gates, perm, inv, static_cast<size_t>(kSmallGates),
+  plan_small_phases(n, gates, perm, inv, static_cast<size_t>(kSmallGates), {}, 0,
                     [&](const std::vector<small_op>& ops, const std::vector<size_t>&, const small_phase& phase) {
                       if (out.empty() || out.back().ops.size() + ops.size() > static_cast<size_t>(kSmallGates)) out.emplace_back();
                       small_program& prog = out.back();

@@ -77,8 +77,10 @@ struct small_program {
 // each, with the ops in physical bits, the gates they come from, and the phase's
 // register bits.  A phase takes, in order, every gate that commutes with those
 // it leaves behind and whose target is, or can still join, its register bits, at
-// most max_ops of them; SWAPs only update the layout map.
+// most max_ops of them and max_marked of the marked ones (marked: one entry per
+// gate, or empty); SWAPs only update the layout map.
 void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv, size_t max_ops,
+                       const std::vector<char>& marked, int max_marked,
                        const std::function<void(const std::vector<small_op>&, const std::vector<size_t>&, const small_phase&)>& emit);
 
 // The queue as launches of the small-state kernel (n <= kSmallBits).

@@ -24,13 +24,15 @@
 #include "rbk_device.cuh"
 #include "rbk_kernels.h"
 #include "rbk_plan.h"
+#include "rbk_small_core.cuh"
 
 namespace rbk {
 namespace {
 
 constexpr int kSaThreads = 512;
 constexpr int kSaPhaseOps = 48;  // ops of one phase, staged in shared memory twice
-constexpr int kSaRegs = 1 << kSmallRegBits;
+constexpr int kSaPhaseSlots = 8;  // overlaps of one phase: a column of partial sums per thread each, staged twice
+constexpr int kSaRegs = kSmallSlots;
 constexpr int kSaLocalBits = 12;  // amplitudes a CTA holds of each state
 constexpr int kSaClassBits = 10;  // instances of fewer qubits share the launch of this size
 
@@ -103,59 +105,6 @@ __device__ __forceinline__ void sa_sync()
   }
 }
 
-// A 2x2 gate of target register bit B on 8 amplitudes; INV: its conjugate transpose.
-template <int B, bool INV>
-__device__ __forceinline__ void sa_target(double2 (&a)[kSaRegs], const small_op& o)
-{
-  const uint32_t creg = o.creg;
-#pragma unroll
-  for (int i = 0; i < kSaRegs; ++i) {
-    if (i & (1 << B)) continue;
-    if ((uint32_t(i) & creg) != creg) continue;
-    double2 &x = a[i], &y = a[i | (1 << B)];
-    const double2 a0 = x, a1 = y;
-    if (o.kind == OPK_X) {
-      x = a1;
-      y = a0;
-    } else if (o.kind == OPK_Y) {
-      x = double2{a1.y, -a1.x};
-      y = double2{-a0.y, a0.x};
-    } else if (o.real) {
-      x = rmac2(a0, a1, o.m[0], o.m[INV ? 4 : 2]);
-      y = rmac2(a0, a1, o.m[INV ? 2 : 4], o.m[6]);
-    } else if (INV) {
-      x = cmac2(a0, a1, o.m[0], -o.m[1], o.m[4], -o.m[5]);
-      y = cmac2(a0, a1, o.m[2], -o.m[3], o.m[6], -o.m[7]);
-    } else {
-      x = cmac2(a0, a1, o.m[0], o.m[1], o.m[2], o.m[3]);
-      y = cmac2(a0, a1, o.m[4], o.m[5], o.m[6], o.m[7]);
-    }
-  }
-}
-
-template <bool INV>
-__device__ __forceinline__ void sa_gate(double2 (&a)[kSaRegs], const small_op& o, uint32_t base)
-{
-  if ((base & o.cbase) != o.cbase) return;
-  if (o.kind == OPK_DIAG || o.kind == OPK_NEG) {
-    const uint32_t creg = o.creg, dreg = o.dreg;
-    const bool hi = (base & o.dbase) != 0, neg = o.kind == OPK_NEG, one = o.diag_one;
-#pragma unroll
-    for (int i = 0; i < kSaRegs; ++i) {
-      if ((uint32_t(i) & creg) != creg) continue;
-      if (neg) a[i] = double2{-a[i].x, -a[i].y};
-      else if (hi || (uint32_t(i) & dreg)) a[i] = cmul(a[i], double2{o.m[2], INV ? -o.m[3] : o.m[3]});
-      else if (!one) a[i] = cmul(a[i], double2{o.m[0], INV ? -o.m[1] : o.m[1]});
-    }
-  } else if (o.treg == 0) {
-    sa_target<0, INV>(a, o);
-  } else if (o.treg == 1) {
-    sa_target<1, INV>(a, o);
-  } else {
-    sa_target<2, INV>(a, o);
-  }
-}
-
 // Im <lambda| P |psi> over this thread's amplitudes, P = X or Y on register bit B.
 template <int B>
 __device__ __forceinline__ double sa_overlap(const double2 (&p)[kSaRegs], const double2 (&l)[kSaRegs], bool y)
@@ -201,6 +150,8 @@ __global__ void __launch_bounds__(kSaThreads, 1) small_adjoint_kernel(const sa_a
   const int local_bits = max(I.n, kSmallRegBits) - kClusterLog;
   const uint32_t local = 1u << local_bits, groups = local / kSaRegs;
   const uint32_t psi = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw)), lam = psi + local * S;
+  // Per-thread overlap sums: columns[buffer][overlap of the phase][thread].
+  double* const columns = reinterpret_cast<double*>(smem_raw + 2 * size_t(local) * S);
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
   const uint32_t warps = blockDim.x >> 5, all_warps = warps * CS, gwarp = rank * warps + (tid >> 5);
   double* partial = A.partial + I.partial_begin;
@@ -268,7 +219,14 @@ __global__ void __launch_bounds__(kSaThreads, 1) small_adjoint_kernel(const sa_a
       double2 a[kSaRegs];
 #pragma unroll
       for (int i = 0; i < kSaRegs; ++i) a[i] = sa_mem<Real, CS>::get(addr[i]);
-      for (int k = 0; k < count; ++k) sa_gate<false>(a, ops[b][k], base);
+      uint32_t signs = 0;
+      small_header h = small_load_header(&ops[b][0]);
+      for (int k = 0; k < count; ++k) {
+        const small_header next_h = small_load_header(&ops[b][min(k + 1, count - 1)]);
+        small_gate<false, false>(a, a, h, &ops[b][k], base, signs);
+        h = next_h;
+      }
+      if (signs) small_signs(a, signs);
 #pragma unroll
       for (int i = 0; i < kSaRegs; ++i) sa_mem<Real, CS>::put(addr[i], a[i]);
     }
@@ -306,7 +264,7 @@ __global__ void __launch_bounds__(kSaThreads, 1) small_adjoint_kernel(const sa_a
       er += pv.x * lr + pv.y * li;
     }
     er = sa_warp_sum(er);
-    if (lane == 0) partial[size_t(I.num_slots) * all_warps + gwarp] = er;
+    if (lane == 0) partial[size_t(I.num_slots) * CS + gwarp] = er;
   }
   if (I.num_phases > 0) {
     next = phases[I.num_phases - 1];
@@ -340,35 +298,41 @@ __global__ void __launch_bounds__(kSaThreads, 1) small_adjoint_kernel(const sa_a
           l[i] = sa_mem<Real, CS>::get(addr[i] + to_lam);
         }
       }
+      uint32_t signs = 0;
+      small_header h = small_load_header(&ops[b][count - 1]);
       for (int k = count - 1; k >= 0; --k) {
-        const small_op& o = ops[b][k];
-        if (o.slot >= 0) {
+        const small_header next_h = small_load_header(&ops[b][max(k - 1, 0)]);
+        if (h.slot() >= 0) {
           double s = 0.0;
-          if (o.rot == 3) {
-            const bool hi = (base & o.dbase) != 0;
-            const uint32_t dreg = o.dreg;
+          if (h.rot() == 3) {  // sign flips not applied yet are on both states: no matter
+            const uint32_t m1 = (base & h.dbase()) ? kAllSlots : h.hi();
 #pragma unroll
-            for (int i = 0; i < kSaRegs; ++i) {
-              const double c = l[i].x * a[i].y - l[i].y * a[i].x;
-              s += (hi || (uint32_t(i) & dreg)) ? -c : c;
-            }
-          } else if (o.treg == 0) {
-            s = sa_overlap<0>(a, l, o.rot == 2);
-          } else if (o.treg == 1) {
-            s = sa_overlap<1>(a, l, o.rot == 2);
+            for (int i = 0; i < kSaRegs; ++i)
+              s += small_flip(l[i].x * a[i].y - l[i].y * a[i].x, (m1 << (31 - i)) & 0x80000000u);
           } else {
-            s = sa_overlap<2>(a, l, o.rot == 2);
+            if (signs) {
+              small_signs(a, signs);
+              small_signs(l, signs);
+              signs = 0;
+            }
+            const uint32_t t = h.code() % 3u;  // target register bit
+            s = t == 0 ? sa_overlap<0>(a, l, h.rot() == 2) : t == 1 ? sa_overlap<1>(a, l, h.rot() == 2) : sa_overlap<2>(a, l, h.rot() == 2);
           }
-          s = sa_warp_sum(s);
-          if (lane == 0) {
-            double* out = partial + size_t(o.slot) * all_warps + gwarp;
-            *out = r > 0 ? *out + s : s;
-          }
+          double* c = columns + (size_t(b) * kSaPhaseSlots + size_t(h.slot() - ph.slot_begin)) * blockDim.x + tid;
+          *c = r > 0 ? *c + s : s;
         }
-        sa_gate<true>(a, o, base);
-        sa_gate<true>(l, o, base);
+        small_gate<true, true>(a, l, h, &ops[b][k], base, signs);
+        h = next_h;
+      }
+      if (signs) {
+        small_signs(a, signs);
+        small_signs(l, signs);
       }
       if (active) {
+        // Addresses formed again from an opaque copy of the base: kept through the gates they would hold 8 registers.
+        uint32_t again = base;
+        asm volatile("" : "+r"(again));
+        sa_addresses<Real, CS>(psi, again, ph.reg, local_bits, addr);
 #pragma unroll
         for (int i = 0; i < kSaRegs; ++i) {
           sa_mem<Real, CS>::put(addr[i], a[i]);
@@ -378,12 +342,20 @@ __global__ void __launch_bounds__(kSaThreads, 1) small_adjoint_kernel(const sa_a
     }
     staged();
     sa_sync<CS>();
+    // The phase's overlaps over the CTA, one warp each, while other warps are in the next phase.
+    for (int q = int(tid >> 5); q < ph.slots; q += int(warps)) {
+      const double* c = columns + (size_t(b) * kSaPhaseSlots + size_t(q)) * blockDim.x;
+      double s = 0.0;
+      for (uint32_t i = lane; i < blockDim.x; i += 32) s += c[i];
+      s = sa_warp_sum(s);
+      if (lane == 0) partial[size_t(ph.slot_begin + q) * CS + rank] = s;
+    }
   }
   __threadfence();
   sa_sync<CS>();  // the partial sums of every CTA are visible
   for (int s = int(rank * blockDim.x + tid); s <= I.num_slots; s += int(blockDim.x * CS)) {
     double acc = 0.0;
-    for (uint32_t w = 0; w < all_warps; ++w) acc += __ldcg(partial + size_t(s) * all_warps + w);
+    for (uint32_t w = 0; w < (s == I.num_slots ? all_warps : uint32_t(CS)); ++w) acc += __ldcg(partial + size_t(s) * CS + w);
     if (s == I.num_slots) A.energy[I.out] = acc;
     else A.overlaps[I.slot_begin + s] = acc;
   }
@@ -482,7 +454,8 @@ template <typename Real, int CS>
 cudaError_t launch_class(const sa_args& args, int first, int count, int n, int threads, cudaStream_t stream)
 {
   const int local_bits = std::max(kSmallRegBits, std::min(n, kSaLocalBits));
-  const size_t smem = 2 * (sizeof(typename ctype<Real>::c) << local_bits);
+  constexpr size_t column = 2 * kSaPhaseSlots * sizeof(double);  // of each thread
+  const size_t smem = 2 * (sizeof(typename ctype<Real>::c) << local_bits) + column * size_t(threads);
   static std::atomic<bool> configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -490,7 +463,7 @@ cudaError_t launch_class(const sa_args& args, int first, int count, int n, int t
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (!configured[dev].load(std::memory_order_acquire)) {
     e = cudaFuncSetAttribute(small_adjoint_kernel<Real, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(2 * (sizeof(typename ctype<Real>::c) << kSaLocalBits)));
+                             int(2 * (sizeof(typename ctype<Real>::c) << kSaLocalBits) + column * kSaThreads));
     if (e != cudaSuccess) return e;
     configured[dev].store(true, std::memory_order_release);
   }
@@ -533,17 +506,21 @@ bool sa_plan(int n, const rbk_circuit_gate* gates, int num_gates, int num_terms,
     if (!lower_gate(n, gates[i], queue[static_cast<size_t>(i)])) return false;
   std::vector<int> perm(static_cast<size_t>(n)), inv(static_cast<size_t>(n));
   for (int q = 0; q < n; ++q) perm[static_cast<size_t>(q)] = inv[static_cast<size_t>(q)] = q;
-  plan_small_phases(n, queue, perm, inv, static_cast<size_t>(kSaPhaseOps),
+  std::vector<char> marked(queue.size(), 0);
+  for (size_t i = 0; i < queue.size(); ++i) marked[i] = gates[i].param >= 0 && rot_type(gates[i].kind) ? 1 : 0;
+  plan_small_phases(n, queue, perm, inv, static_cast<size_t>(kSaPhaseOps), marked, kSaPhaseSlots,
                     [&](const std::vector<small_op>& ops, const std::vector<size_t>& from, const small_phase& phase) {
                       sa_phase ph{};
                       std::memcpy(ph.reg, phase.reg, sizeof(ph.reg));
                       ph.begin = static_cast<int32_t>(out.ops.size());
+                      ph.slot_begin = static_cast<int32_t>(out.slot_param.size());
                       for (size_t k = 0; k < ops.size(); ++k) {
                         const rbk_circuit_gate& g = gates[from[k]];
                         small_op o = ops[k];
-                        o.rot = static_cast<uint16_t>(rot_type(g.kind));
-                        if (o.rot) {
-                          o.real = o.rot == 2 ? 1 : 0;
+                        o.rot = static_cast<uint8_t>(rot_type(g.kind));
+                        if (o.rot) {  // the matrix comes on the device
+                          if (o.rot < 3) o.code = static_cast<uint8_t>((o.rot == 2 ? SMALL_REAL : SMALL_MAT) + o.treg);
+                          else o.code = SMALL_DIAG;
                           out.rots.push_back({static_cast<int32_t>(out.ops.size()), g.param, g.scale, g.angles[0]});
                           if (g.param >= 0) {
                             o.slot = static_cast<int32_t>(out.slot_param.size());
@@ -554,6 +531,7 @@ bool sa_plan(int n, const rbk_circuit_gate* gates, int num_gates, int num_terms,
                         out.ops.push_back(o);
                       }
                       ph.end = static_cast<int32_t>(out.ops.size());
+                      ph.slots = static_cast<int32_t>(out.slot_param.size()) - ph.slot_begin;
                       out.phases.push_back(ph);
                     });
   static const cplx pow_mi[4] = {{1, 0}, {0, -1}, {-1, 0}, {0, 1}};
@@ -623,7 +601,8 @@ int sa_set::assign(int precision, const std::vector<const sa_program*>& programs
     rots += P.rots.size();
     terms += P.terms.size();
     slots_ += I.num_slots;
-    partial += size_t(I.num_slots + 1) * size_t(cluster_of(P.n)) * size_t(threads_of(std::max(kSaClassBits, P.n), kSaThreads) / 32);
+    // an overlap per CTA, the energy per warp
+    partial += size_t(cluster_of(P.n)) * (size_t(I.num_slots) + size_t(threads_of(std::max(kSaClassBits, P.n), kSaThreads) / 32));
     insts_.push_back(I);
   }
   if (ops > size_t(INT32_MAX) || terms > size_t(INT32_MAX)) return sa_fail(RBK_ERR_UNSUPPORTED, "batch: too many gates");

@@ -20,7 +20,8 @@ constexpr int kSmallAdjointBits = 15;
 
 struct sa_term { uint32_t flip, sign; double wr, wi; };  // (P psi)_i = w (-1)^popcount(i & sign) psi_{i ^ flip}
 struct sa_rot { int32_t op, param; double scale, offset; };  // ops[op].m from phi = scale * theta[param] + offset
-struct sa_phase { uint8_t reg[kSmallRegBits], pad; int32_t begin, end; };
+// Ops [begin, end) and their overlaps [slot_begin, slot_begin + slots), numbered in op order.
+struct sa_phase { uint8_t reg[kSmallRegBits], pad; int32_t begin, end, slot_begin, slots; };
 
 // One planned circuit, in physical bits.
 struct sa_program {

@@ -65,13 +65,21 @@ static void run_program(std::vector<cd>& phys, int n, const rbk::small_program& 
       }
       for (uint32_t g = ph.begin; g < ph.end; ++g) {
         const auto& o = p.ops[g];
+        const int family = o.kind == rbk::OPK_X ? rbk::SMALL_X : o.kind == rbk::OPK_Y ? rbk::SMALL_Y
+                           : o.code >= rbk::SMALL_REAL ? rbk::SMALL_REAL : rbk::SMALL_MAT;
+        const bool diag = o.kind == rbk::OPK_DIAG || o.kind == rbk::OPK_NEG;
+        if (diag ? (o.kind == rbk::OPK_NEG ? o.code != rbk::SMALL_NEG : o.code != rbk::SMALL_DIAG && o.code != rbk::SMALL_DIAG1)
+                 : o.code != family + o.treg)
+          fail("dispatch code");
+        for (int i = 0; i < NR; ++i)
+          if (((o.act >> i) & 1) != ((i & o.creg) == o.creg) || ((o.hi >> i) & 1) != ((i & o.dreg) != 0)) fail("slot masks");
         if ((base & o.cbase) != o.cbase) continue;
         for (int i = 0; i < NR; ++i) {
-          if ((i & o.creg) != o.creg) continue;
+          if (!((o.act >> i) & 1)) continue;
           if (o.kind == rbk::OPK_NEG) a[i] = -a[i];
           else if (o.kind == rbk::OPK_DIAG) {
-            if ((base & o.dbase) || (i & o.dreg)) a[i] *= at(o.m, 1);
-            else if (!o.diag_one) a[i] *= at(o.m, 0);
+            if ((base & o.dbase) || ((o.hi >> i) & 1)) a[i] *= at(o.m, 1);
+            else if (o.code == rbk::SMALL_DIAG) a[i] *= at(o.m, 0);
           } else {
             if (o.treg >= R) fail("target register");
             if ((i >> o.treg) & 1) continue;
@@ -79,7 +87,7 @@ static void run_program(std::vector<cd>& phys, int n, const rbk::small_program& 
             const cd u = x, v = y;
             if (o.kind == rbk::OPK_X) { x = v; y = u; }
             else if (o.kind == rbk::OPK_Y) { x = cd{v.imag(), -v.real()}; y = cd{-u.imag(), u.real()}; }
-            else if (o.real) { x = o.m[0] * u + o.m[2] * v; y = o.m[4] * u + o.m[6] * v; }
+            else if (family == rbk::SMALL_REAL) { x = o.m[0] * u + o.m[2] * v; y = o.m[4] * u + o.m[6] * v; }
             else { x = at(o.m, 0) * u + at(o.m, 1) * v; y = at(o.m, 2) * u + at(o.m, 3) * v; }
           }
         }
