@@ -175,6 +175,8 @@ struct dev_hbm_layout {
   uint64_t tphys_lo[16], tphys_hi[32];
 };
 
+constexpr int kMaxStraight = 6;  // phases of a straight pass
+constexpr uint32_t kStraightPre = 0x100;
 struct dev_pass {
   uint8_t tile_phys[16];      // physical bit of tile bit b
   uint8_t num_runs;           // the block index is deposited into the non-tile bits run by run:
@@ -190,6 +192,19 @@ struct dev_pass {
   dev_phase phases[kMaxPhases];
   dev_op ops[kMaxPassOps];
   alignas(16) double tabs[kMaxLayerTabs * kTabDoubles];  // factored layers' diagonal factors (complex<double> or complex<float>)
+  // Straight passes: every phase is at most one layer of uncontrolled 2x2 gates
+  // in the factored form (its CNOT / X gates are all folded).  straight: the
+  // number of phases, 0 for any other pass.  The kernel for them is unrolled over
+  // the phases, so that all of this sits at compile-time addresses.
+  struct straight_layer {
+    double t[8];              // t0, t1 of each register bit, in the state's precision
+    double pre[kTabDoubles];  // a factor per register slot
+    double post[kTabDoubles];
+    uint32_t bits;            // register bits with a gate; kStraightPre: pre factors other than 1
+    uint32_t pad[3];
+  };
+  alignas(16) straight_layer straight_layers[kMaxStraight];
+  uint32_t straight, pad2[3];
 };
 
 // Program of a state that fits one CTA's shared memory (n <= kSmallBits): the

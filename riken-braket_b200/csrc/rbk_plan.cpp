@@ -225,6 +225,60 @@ std::vector<phase_build> phases_by_dag(const std::vector<pop>& ops, const int* t
   return phases;
 }
 
+// Register phases of a straight pass: each takes ready 2x2 gates on up to R
+// different bits, then the ready CNOT / X gates that can fold into its write
+// layout (fold_trailing_x).  Empty if some gate is of another kind or the phases
+// do not fit kMaxStraight.
+std::vector<phase_build> phases_straight(const std::vector<pop>& ops, const int* tile_of_phys, uint64_t tile_mask, int R)
+{
+  const int m = static_cast<int>(ops.size());
+  for (const pop& o : ops)
+    if (o.kind != OPK_X ? o.kind != OPK_MAT || o.cmask : popc(o.cmask & tile_mask) > 1) return {};
+  std::vector<std::vector<int>> preds(m);
+  for (int j = 0; j < m; ++j)
+    for (int i = 0; i < j; ++i)
+      if (conflict(ops[i], ops[j])) preds[j].push_back(i);
+  std::vector<char> done(m, 0);
+  auto ready = [&](int j) {
+    return !done[j] && std::all_of(preds[j].begin(), preds[j].end(), [&](int i) { return done[i]; });
+  };
+  std::vector<phase_build> phases;
+  for (int remaining = m; remaining > 0;) {
+    if (static_cast<int>(phases.size()) == kMaxStraight) return {};
+    phase_build pb;
+    uint64_t reg = 0, gates = 0, moved = 0;  // physical bits: in registers, with a 2x2 gate, targets of folds
+    auto take = [&](int j) {
+      const int t = ops[j].target;
+      if (!(reg & bit(t))) {
+        reg |= bit(t);
+        pb.reg.push_back(tile_of_phys[t]);
+      }
+      done[j] = 1;
+      --remaining;
+      pb.ops.push_back(j);
+    };
+    auto fits = [&](int t) { return (reg & bit(t)) || static_cast<int>(pb.reg.size()) < R; };
+    for (int j = 0; j < m; ++j)
+      if (ops[j].kind == OPK_MAT && !(gates & bit(ops[j].target)) && fits(ops[j].target) && ready(j)) {
+        gates |= bit(ops[j].target);
+        take(j);
+      }
+    int conditional = 0;
+    for (int j = 0; j < m; ++j) {
+      const pop& o = ops[j];
+      if (o.kind != OPK_X || !fits(o.target) || (o.cmask & moved) || !ready(j)) continue;
+      const bool outside = (o.cmask & ~tile_mask) != 0;
+      if (outside && conditional == kMaxFolds) continue;
+      conditional += outside ? 1 : 0;
+      moved |= bit(o.target);
+      take(j);
+    }
+    if (pb.ops.empty()) return {};
+    phases.push_back(pb);
+  }
+  return phases;
+}
+
 // CNOT / X gates at the end of a phase permute the tile's indices GF(2)-affinely:
 // instead of running them, the write-back layout absorbs them.  A gate X_t
 // controlled by one bit c (a register bit, a warp-uniform thread bit, or none)
@@ -600,8 +654,53 @@ void group_layers(const plan_params& p, dev_pass& out, dev_phase& dp, int& op_en
   op_end = begin + static_cast<int>(grouped.size());
 }
 
-void build_pass(const plan_params& p, uint64_t tile_mask, const std::vector<pop>& ops,
-                const int* relabel_to, const int* tile_phys, dev_pass& out)
+// The ops of a phase as a straight layer (dev_pass::straight_layers): uncontrolled
+// 2x2 gates on distinct register bits, each in the factored form.
+bool straight_layer_of(const plan_params& p, const dev_op* ops, int count, dev_pass::straight_layer& out)
+{
+  using cd = std::complex<double>;
+  std::vector<cd> q(static_cast<size_t>(p.R), 1.0), p0(static_cast<size_t>(p.R), 1.0), p1(static_cast<size_t>(p.R), 1.0);
+  std::vector<double> t(2 * static_cast<size_t>(p.R), 0.0);
+  uint32_t used = 0;
+  bool pre = false;
+  for (int k = 0; k < count; ++k) {
+    const dev_op& d = ops[k];
+    gate_factors f;
+    if (d.kind != OPK_MAT || d.creg || d.cthr || d.cout || ((used >> d.treg) & 1u) || !factor_gate(d.m, f)) return false;
+    used |= 1u << d.treg;
+    q[d.treg] = f.q;
+    p0[d.treg] = f.p0;
+    p1[d.treg] = f.p1;
+    t[2 * size_t(d.treg)] = f.t0;
+    t[2 * size_t(d.treg) + 1] = f.t1;
+    pre = pre || f.q != cd{1.0, 0.0};
+  }
+  auto put = [&](double* to, size_t i, double v) {
+    if (p.vbits == 0) to[i] = v;
+    else reinterpret_cast<float*>(to)[i] = static_cast<float>(v);
+  };
+  for (size_t i = 0; i < t.size(); ++i) put(out.t, i, t[i]);
+  for (int i = 0; i < (1 << p.R); ++i) {
+    cd a = 1.0, b = 1.0;
+    for (int r = 0; r < p.R; ++r) {
+      const size_t s = static_cast<size_t>(r);
+      if ((i >> r) & 1) { a *= q[s]; b *= p1[s]; }
+      else b *= p0[s];
+    }
+    put(out.pre, 2 * size_t(i), a.real());
+    put(out.pre, 2 * size_t(i) + 1, a.imag());
+    put(out.post, 2 * size_t(i), b.real());
+    put(out.post, 2 * size_t(i) + 1, b.imag());
+  }
+  out.bits = used | (pre ? kStraightPre : 0);
+  return true;
+}
+
+// straight: build a straight pass or return false, with `out` unfinished.
+// direct_store: the last phase may store straight to HBM.
+bool build_pass(const plan_params& p, uint64_t tile_mask, const std::vector<pop>& ops,
+                const int* relabel_to, const int* tile_phys, std::vector<phase_build> phases, const bool straight,
+                const bool direct_store, dev_pass& out)
 {
   std::memset(&out, 0, sizeof(out));
   const int K = p.K, R = p.R, T = K - R;
@@ -627,14 +726,6 @@ void build_pass(const plan_params& p, uint64_t tile_mask, const std::vector<pop>
     }
     out.num_runs = static_cast<uint8_t>(runs);
   }
-
-  std::vector<phase_build> phases = phases_by_dag(ops, tile_of_phys, R, false);
-  if (p.defer_x) {  // taking CNOT / X gates last lets them fold; keep it unless it costs register phases
-    std::vector<phase_build> deferred = phases_by_dag(ops, tile_of_phys, R, true);
-    if (deferred.size() <= phases.size()) phases.swap(deferred);
-  }
-  if (static_cast<int>(phases.size()) > kMaxPhases) phases = phases_in_order(ops, tile_of_phys, R);
-  if (static_cast<int>(phases.size()) > kMaxPhases) throw std::logic_error("planner: too many phases");
 
   // Tile bits lane0 .. lane0+4 are contiguous in HBM (512-byte runs); for c64
   // tile bit 0 is the amplitude pair inside one 16-byte vector.
@@ -675,7 +766,7 @@ void build_pass(const plan_params& p, uint64_t tile_mask, const std::vector<pop>
       return 0;
     };
     const int lmode = first ? mode_for(identity) : 0;
-    const int smode = last ? mode_for(relabel_from) : 0;
+    const int smode = last && direct_store ? mode_for(relabel_from) : 0;
     // Bits the fill should keep out of (or bring into) the registers for those modes.
     std::vector<int> keep_out, bring_in;
     if (lmode) {
@@ -820,11 +911,42 @@ void build_pass(const plan_params& p, uint64_t tile_mask, const std::vector<pop>
              : op_code(d.kind, 0, true, 0);
     }
     if (p.fold_x) fold_trailing_x(p, out, dp, op_index, last && ds ? smode : 0);
+    if (straight) {
+      if (!straight_layer_of(p, out.ops + dp.op_begin, op_index - dp.op_begin, out.straight_layers[ph])) return false;
+      dp.op_end = static_cast<uint16_t>(op_index);
+      continue;
+    }
     if (p.phase_runs) group_phase_runs(p, out, dp, op_index, headers_left);
     if (p.layers) group_layers(p, out, dp, op_index, headers_left, tabs_used);
     dp.op_end = static_cast<uint16_t>(op_index);
   }
   out.num_phases = static_cast<uint8_t>(phases.size());
+  out.straight = straight ? static_cast<uint32_t>(phases.size()) : 0;
+  return out.straight != 0;
+}
+
+// A pass's kernel parameters: as a straight pass where its gates allow that --
+// without the direct store if only that stood against folding the last phase's
+// CNOT gates --, otherwise in the general form.
+void build_pass(const plan_params& p, uint64_t tile_mask, const std::vector<pop>& ops,
+                const int* relabel_to, const int* tile_phys, dev_pass& out)
+{
+  int tile_of_phys[64];
+  for (int b = 0; b < p.K; ++b) tile_of_phys[tile_phys[b]] = b;
+  if (p.straight) {
+    const std::vector<phase_build> phases = phases_straight(ops, tile_of_phys, tile_mask, p.R);
+    if (!phases.empty())
+      for (const bool direct : {true, false})
+        if (build_pass(p, tile_mask, ops, relabel_to, tile_phys, phases, true, direct, out)) return;
+  }
+  std::vector<phase_build> phases = phases_by_dag(ops, tile_of_phys, p.R, false);
+  if (p.defer_x) {  // taking CNOT / X gates last lets them fold; keep it unless it costs register phases
+    std::vector<phase_build> deferred = phases_by_dag(ops, tile_of_phys, p.R, true);
+    if (deferred.size() <= phases.size()) phases.swap(deferred);
+  }
+  if (static_cast<int>(phases.size()) > kMaxPhases) phases = phases_in_order(ops, tile_of_phys, p.R);
+  if (static_cast<int>(phases.size()) > kMaxPhases) throw std::logic_error("planner: too many phases");
+  build_pass(p, tile_mask, ops, relabel_to, tile_phys, phases, false, true, out);
 }
 
 // Single-qubit gates without controls as 2x2 matrices (row-major, re/im pairs).

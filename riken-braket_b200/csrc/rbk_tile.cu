@@ -492,6 +492,78 @@ __device__ __forceinline__ void apply_folds(const dev_phase& ph, uint64_t base, 
   }
 }
 
+// Registers of phase 0 straight from HBM.  mode 1: 16-byte vectors, 2: 8-byte
+// complex<float> amplitudes.
+template <typename Real, int R>
+__device__ __forceinline__ void load_direct(typename ctype<Real>::c* a, const typename ctype<Real>::c* __restrict__ state,
+                                            const dev_pass& P, uint64_t base, uint32_t tid, int mode)
+{
+  using C = typename ctype<Real>::c;
+  using V = typename ctype<Real>::v16;
+  using PT = precision_traits<Real>;
+  constexpr int NR = 1 << R, VEC = PT::VEC, VB = PT::VB;
+  const V* gsrc = reinterpret_cast<const V*>(state);
+  const uint64_t tphys = base | P.load.tphys_lo[tid & 15] | P.load.tphys_hi[tid >> 4];
+  uint64_t rphys[R];
+#pragma unroll
+  for (int b = 0; b < R; ++b) rphys[b] = P.load.rphys[b];
+  if (sizeof(Real) == 4 && mode == 2) {
+    const C* src = state;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      uint64_t phys = tphys;
+#pragma unroll
+      for (int b = 0; b < R; ++b) if (i & (1 << b)) phys |= rphys[b];
+      a[i] = __ldcs(src + phys);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NR; i += VEC) {
+      uint64_t phys = tphys;
+#pragma unroll
+      for (int b = VB; b < R; ++b) if (i & (1 << b)) phys |= rphys[b];
+      vec_io<Real>::unpack(__ldcs(gsrc + (phys >> VB)), &a[i]);
+    }
+  }
+}
+
+// The last phase's registers straight to HBM (the pass's direct_store, modes as above).
+template <typename Real, int R>
+__device__ __forceinline__ void store_direct(const typename ctype<Real>::c* a, typename ctype<Real>::c* __restrict__ state,
+                                             const dev_pass& P, const dev_phase& ph, uint64_t base, uint32_t tid)
+{
+  using C = typename ctype<Real>::c;
+  using V = typename ctype<Real>::v16;
+  using PT = precision_traits<Real>;
+  constexpr int NR = 1 << R, VEC = PT::VEC, VB = PT::VB;
+  V* gdst = reinterpret_cast<V*>(state);
+  // base holds only bits outside the tile, the tables only tile bits;
+  // folded CNOTs make table contributions overlap, hence XOR.
+  uint64_t tphys = base ^ P.store.tphys_lo[tid & 15] ^ P.store.tphys_hi[tid >> 4];
+  uint64_t rphys[R];
+#pragma unroll
+  for (int b = 0; b < R; ++b) rphys[b] = P.store.rphys[b];
+  apply_folds<R>(ph, base, tid, tphys, rphys);
+  if (sizeof(Real) == 4 && P.direct_store == 2) {
+    C* dst = state;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      uint64_t phys = tphys;
+#pragma unroll
+      for (int b = 0; b < R; ++b) if (i & (1 << b)) phys ^= rphys[b];
+      __stcs(dst + phys, a[i]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NR; i += VEC) {
+      uint64_t phys = tphys;
+#pragma unroll
+      for (int b = VB; b < R; ++b) if (i & (1 << b)) phys ^= rphys[b];
+      __stcs(gdst + (phys >> VB), vec_io<Real>::pack(&a[i]));
+    }
+  }
+}
+
 // One tile through the pass's phases, ending with the tile stored to HBM.
 // load_mode: phase 0 loads its registers straight from HBM (the pass's direct
 // load: 1 in 16-byte vectors, 2 in 8-byte complex<float> amplitudes); 0: the
@@ -504,39 +576,14 @@ __device__ __forceinline__ void tile_phases(typename ctype<Real>::c* __restrict_
 {
   const bool from_hbm = load_mode != 0;
   using C = typename ctype<Real>::c;
-  using V = typename ctype<Real>::v16;
-  using PT = precision_traits<Real>;
-  constexpr int NR = 1 << R, T = K - R, VEC = PT::VEC, VB = PT::VB;
-  const V* gsrc = reinterpret_cast<const V*>(state);
-  V* gdst = reinterpret_cast<V*>(state);
+  constexpr int NR = 1 << R, T = K - R;
 
   C a[NR];
   const int nph = P.num_phases;
   for (int p = 0; p < nph; ++p) {
     const dev_phase& ph = P.phases[p];
     if (p == 0 && from_hbm) {
-      const uint64_t tphys = base | P.load.tphys_lo[tid & 15] | P.load.tphys_hi[tid >> 4];
-      uint64_t rphys[R];
-#pragma unroll
-      for (int b = 0; b < R; ++b) rphys[b] = P.load.rphys[b];
-      if (sizeof(Real) == 4 && load_mode == 2) {
-        const C* src = state;
-#pragma unroll
-        for (int i = 0; i < NR; ++i) {
-          uint64_t phys = tphys;
-#pragma unroll
-          for (int b = 0; b < R; ++b) if (i & (1 << b)) phys |= rphys[b];
-          a[i] = __ldcs(src + phys);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < NR; i += VEC) {
-          uint64_t phys = tphys;
-#pragma unroll
-          for (int b = VB; b < R; ++b) if (i & (1 << b)) phys |= rphys[b];
-          vec_io<Real>::unpack(__ldcs(gsrc + (phys >> VB)), &a[i]);
-        }
-      }
+      load_direct<Real, R>(a, state, P, base, tid, load_mode);
     } else {
       const uint32_t ts = ph.tslot_lo[tid & 15] ^ ph.tslot_hi[tid >> 4];
       uint32_t rs[R];
@@ -558,31 +605,7 @@ __device__ __forceinline__ void tile_phases(typename ctype<Real>::c* __restrict_
       // CTA must have read its amplitudes before any warp overwrites the tile
       // in its relabelled order.
       if (p == 0 && from_hbm) __syncthreads();
-      // base holds only bits outside the tile, the tables only tile bits;
-      // folded CNOTs make table contributions overlap, hence XOR.
-      uint64_t tphys = base ^ P.store.tphys_lo[tid & 15] ^ P.store.tphys_hi[tid >> 4];
-      uint64_t rphys[R];
-#pragma unroll
-      for (int b = 0; b < R; ++b) rphys[b] = P.store.rphys[b];
-      apply_folds<R>(ph, base, tid, tphys, rphys);
-      if (sizeof(Real) == 4 && P.direct_store == 2) {
-        C* dst = state;
-#pragma unroll
-        for (int i = 0; i < NR; ++i) {
-          uint64_t phys = tphys;
-#pragma unroll
-          for (int b = 0; b < R; ++b) if (i & (1 << b)) phys ^= rphys[b];
-          __stcs(dst + phys, a[i]);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < NR; i += VEC) {
-          uint64_t phys = tphys;
-#pragma unroll
-          for (int b = VB; b < R; ++b) if (i & (1 << b)) phys ^= rphys[b];
-          __stcs(gdst + (phys >> VB), vec_io<Real>::pack(&a[i]));
-        }
-      }
+      store_direct<Real, R>(a, state, P, ph, base, tid);
     } else {
       // Every thread has read this phase's layout from `tile` (a phase that
       // loaded straight from HBM has not used it).
@@ -604,6 +627,129 @@ __device__ __forceinline__ void tile_phases(typename ctype<Real>::c* __restrict_
   }
 
   if (!P.direct_store) tile_copy<Real, K, T, 1>(state, P, tile, base, tid);
+}
+
+// Phase PH of a straight pass (dev_pass::straight): the layer's constants are at
+// compile-time addresses of the parameter block, operands of the arithmetic
+// instructions themselves.  The general kernel indexes its op records and tables
+// at run time, and their loads kept a layer of 320 FP64 instructions at three times
+// its issue time.  The full layer has code of its own: with a branch per register
+// bit for every layer the 30-qubit brick took 319 ms instead of 306.
+template <typename Real, int R, int PH>
+__device__ __forceinline__ void apply_straight_layer(typename ctype<Real>::c* a, const dev_pass& P)
+{
+  using C = typename ctype<Real>::c;
+  constexpr int NR = 1 << R;
+  const auto& L = P.straight_layers[PH];
+  if (L.bits == 0) return;
+  if (L.bits & kStraightPre) {
+    const C* pre = reinterpret_cast<const C*>(L.pre);
+#pragma unroll
+    for (int i = 1; i < NR; ++i) a[i] = cmul(a[i], pre[i]);
+  }
+  const Real* t = reinterpret_cast<const Real*>(L.t);
+  if ((L.bits & ((1u << R) - 1)) == (1u << R) - 1) {
+    apply_factor<Real, 0, NR>(a, t[0], t[1]);
+    apply_factor<Real, 1, NR>(a, t[2], t[3]);
+    apply_factor<Real, 2, NR>(a, t[4], t[5]);
+    apply_factor<Real, 3, NR>(a, t[6], t[7]);
+    if constexpr (R > 4) apply_factor<Real, (R > 4 ? 4 : 0), NR>(a, t[8], t[9]);
+  } else {
+    if (L.bits & 1) apply_factor<Real, 0, NR>(a, t[0], t[1]);
+    if (L.bits & 2) apply_factor<Real, 1, NR>(a, t[2], t[3]);
+    if (L.bits & 4) apply_factor<Real, 2, NR>(a, t[4], t[5]);
+    if (L.bits & 8) apply_factor<Real, 3, NR>(a, t[6], t[7]);
+    if constexpr (R > 4) if (L.bits & 16) apply_factor<Real, (R > 4 ? 4 : 0), NR>(a, t[8], t[9]);
+  }
+  const C* post = reinterpret_cast<const C*>(L.post);
+#pragma unroll
+  for (int i = 0; i < NR; ++i) a[i] = cmul(a[i], post[i]);
+}
+
+// Registers <-> the tile in shared memory in a phase's layout.
+template <typename Real, int R>
+__device__ __forceinline__ void exchange_in(typename ctype<Real>::c* a, const dev_phase& ph, const typename ctype<Real>::c* tile, uint32_t tid)
+{
+  const uint32_t ts = ph.tslot_lo[tid & 15] ^ ph.tslot_hi[tid >> 4];
+#pragma unroll
+  for (int i = 0; i < (1 << R); ++i) {
+    uint32_t sidx = ts;
+#pragma unroll
+    for (int b = 0; b < R; ++b) if (i & (1 << b)) sidx ^= ph.rslot[b];
+    a[i] = tile[sidx];
+  }
+}
+
+template <typename Real, int R>
+__device__ __forceinline__ void exchange_out(const typename ctype<Real>::c* a, const dev_phase& ph, typename ctype<Real>::c* tile,
+                                             uint64_t base, uint32_t tid)
+{
+  uint32_t ts = ph.wtslot_lo[tid & 15] ^ ph.wtslot_hi[tid >> 4];
+  uint32_t rs[R];
+#pragma unroll
+  for (int b = 0; b < R; ++b) rs[b] = ph.wslot[b];
+  apply_folds<R>(ph, base, tid, ts, rs);
+#pragma unroll
+  for (int i = 0; i < (1 << R); ++i) {
+    uint32_t sidx = ts;
+#pragma unroll
+    for (int b = 0; b < R; ++b) if (i & (1 << b)) sidx ^= rs[b];
+    tile[sidx] = a[i];
+  }
+}
+
+// Phases PH .. N - 1 of a straight pass; the registers hold phase PH's layout on entry.
+template <typename Real, int R, int N, int PH>
+__device__ __forceinline__ void straight_phases(typename ctype<Real>::c* a, const dev_pass& P, typename ctype<Real>::c* tile,
+                                                uint64_t base, uint32_t tid, bool tile_read)
+{
+  apply_straight_layer<Real, R, PH>(a, P);
+  if constexpr (PH + 1 < N) {
+    if (tile_read) __syncthreads();  // every thread has read this phase's layout
+    exchange_out<Real, R>(a, P.phases[PH], tile, base, tid);
+    __syncthreads();
+    exchange_in<Real, R>(a, P.phases[PH + 1], tile, tid);
+    straight_phases<Real, R, N, PH + 1>(a, P, tile, base, tid, true);
+  }
+}
+
+// One tile per CTA, as tile_pass_kernel, for a straight pass of N phases, unrolled.
+// Bound in complex<double> by HBM while the phases are three full layers (5.6 TB/s,
+// 0.85 of the copy rate; FP64 pipe 39 %), by the shared-memory exchanges with six;
+// in complex<float> by exchanges and instruction issue (2.9 TB/s at four phases).
+// Brick of 30 qubits, 20 layers, device time: complex<double> 369 -> 306 ms,
+// complex<float> 249 -> 163 ms.
+template <typename Real, int N>
+__global__ void __launch_bounds__(1 << (tile_shape<Real, 2>::K - tile_shape<Real, 2>::R), tile_shape<Real, 2>::CTAS)
+straight_pass_kernel(typename ctype<Real>::c* __restrict__ state, const __grid_constant__ dev_pass P)
+{
+  using C = typename ctype<Real>::c;
+  using SH = tile_shape<Real, 2>;
+  constexpr int K = SH::K, R = SH::R, T = K - R, NR = 1 << R;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* tile = reinterpret_cast<C*>(smem_raw);
+  const uint32_t tid = threadIdx.x;
+  const uint64_t base = tile_base(P, blockIdx.x);
+  C a[NR];
+  if (P.direct_load) {
+    load_direct<Real, R>(a, state, P, base, tid, P.direct_load);
+  } else {
+    tile_copy<Real, K, T, 0>(state, P, tile, base, tid);
+    __syncthreads();
+    exchange_in<Real, R>(a, P.phases[0], tile, tid);
+  }
+  straight_phases<Real, R, N, 0>(a, P, tile, base, tid, !P.direct_load);
+  if (P.direct_store) {
+    // A one-phase pass that loaded straight from HBM: every warp must have read its
+    // amplitudes before any overwrites the tile in its relabelled order.
+    if (N == 1 && P.direct_load) __syncthreads();
+    store_direct<Real, R>(a, state, P, P.phases[N - 1], base, tid);
+  } else {
+    if (N > 1 || !P.direct_load) __syncthreads();
+    exchange_out<Real, R>(a, P.phases[N - 1], tile, base, tid);
+    __syncthreads();
+    tile_copy<Real, K, T, 1>(state, P, tile, base, tid);
+  }
 }
 
 // One CTA per tile (PIPE false): the tile is loaded (straight into registers
@@ -692,9 +838,49 @@ cudaError_t launch_shape(void* state, int n, const dev_pass& pass, cudaStream_t 
 
 }  // namespace
 
+namespace {
+
+template <typename Real, int N>
+cudaError_t launch_straight(void* state, int n, const dev_pass& pass, cudaStream_t stream)
+{
+  using SH = tile_shape<Real, 2>;
+  constexpr size_t smem = sizeof(typename ctype<Real>::c) << SH::K;
+  static std::atomic<bool> configured[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(straight_pass_kernel<Real, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  if (n < SH::K) return cudaErrorInvalidValue;
+  straight_pass_kernel<Real, N><<<(unsigned)(1ull << (n - SH::K)), 1 << (SH::K - SH::R), smem, stream>>>(
+    static_cast<typename ctype<Real>::c*>(state), pass);
+  return cudaGetLastError();
+}
+
+template <typename Real>
+cudaError_t launch_straight(void* state, int n, const dev_pass& pass, cudaStream_t stream)
+{
+  switch (pass.straight) {
+    case 1: return launch_straight<Real, 1>(state, n, pass, stream);
+    case 2: return launch_straight<Real, 2>(state, n, pass, stream);
+    case 3: return launch_straight<Real, 3>(state, n, pass, stream);
+    case 4: return launch_straight<Real, 4>(state, n, pass, stream);
+    case 5: return launch_straight<Real, 5>(state, n, pass, stream);
+    case 6: return launch_straight<Real, 6>(state, n, pass, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace
+
 template <typename Real>
 cudaError_t launch_tile_pass(void* state, int n, const dev_pass& pass, int shape, cudaStream_t stream)
 {
+  if (pass.straight > 0 && shape == 2) return launch_straight<Real>(state, n, pass, stream);
   switch (shape) {
     case 0: return launch_shape<Real, 0>(state, n, pass, stream);
     // Shape 1 (2^12-amplitude tile, 8 per thread, 512 threads) is not built:
