@@ -1,8 +1,7 @@
 // rbk_kernels.cu -- sm_100a kernels of the state-vector engine.
 //
 //   (the fused tile pass lives in rbk_tile.cu)
-//   gate_kernel        one unfused gate straight on HBM (states smaller than a
-//                      tile, and the unfused execution mode).
+//   small_circuit_kernel  a whole queue of gates on a state of up to 12 qubits.
 //   reductions         norm, probabilities, Z / pair sums for spins and Pauli
 //                      strings, inner product: warp-shuffle + block reduction
 //                      with FP64 accumulation, per-block partials reduced in a
@@ -320,9 +319,9 @@ pauli_kernel(const typename ctype<Real>::c* __restrict__ a, int n, uint64_t flip
       for (int t = 0; t < T.count; ++t) {
         const double si = (__popcll(i & T.sign[t]) & 1) ? -1.0 : 1.0;
         const double sj = (__popcll(j & T.sign[t]) & 1) ? -1.0 : 1.0;
-        // si * c * w + sj * conj(c) * w   (one-sided: si * c * w)
-        const double xr = T.one_sided ? si * cr : si * cr + sj * cr;
-        const double xi = T.one_sided ? si * ci : si * ci - sj * ci;
+        // si * c * w + sj * conj(c) * w
+        const double xr = si * cr + sj * cr;
+        const double xi = si * ci - sj * ci;
         re += xr * T.w[t][0] - xi * T.w[t][1];
         im += xr * T.w[t][1] + xi * T.w[t][0];
       }
@@ -816,28 +815,6 @@ __global__ void pauli_apply_kernel(const typename ctype<Real>::c* __restrict__ s
   }
 }
 
-// sum_i conj(lam_i) w (-1)^popcount(i & sign) psi_{i ^ flip}: <lam| P |psi> for
-// one Pauli string P given as (flip, sign, w) -- the overlap of the adjoint sweep.
-template <typename Real>
-__global__ void __launch_bounds__(kRedThreads)
-overlap_kernel(const typename ctype<Real>::c* __restrict__ lam, const typename ctype<Real>::c* __restrict__ psi,
-               uint64_t size, uint64_t flip, uint64_t sign, double wr, double wi, double* partials)
-{
-  double re = 0, im = 0;
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < size; i += stride) {
-    const auto l = lam[i], p = psi[i ^ flip];
-    const double s = (__popcll(i & sign) & 1) ? -1.0 : 1.0;
-    // conj(l) * p
-    const double cr = double(l.x) * double(p.x) + double(l.y) * double(p.y);
-    const double ci = double(l.x) * double(p.y) - double(l.y) * double(p.x);
-    re += s * (cr * wr - ci * wi);
-    im += s * (cr * wi + ci * wr);
-  }
-  double vals[2] = {re, im};
-  block_sum_store<2>(vals, 2, partials + size_t(blockIdx.x) * 2);
-}
-
 template <typename Real>
 cudaError_t launch_pauli_apply(const void* src, void* dst, int n, const pauli_sum& P, cudaStream_t stream)
 {
@@ -1115,18 +1092,6 @@ cudaError_t launch_pauli_apply_tiled(const void* src, void* dst, int n, const pa
 }
 template cudaError_t launch_pauli_apply_tiled<double>(const void*, void*, int, const pauli_sum&, cudaStream_t);
 template cudaError_t launch_pauli_apply_tiled<float>(const void*, void*, int, const pauli_sum&, cudaStream_t);
-
-template <typename Real>
-cudaError_t launch_overlap(const void* lam, const void* psi, int n, uint64_t flip, uint64_t sign, double wr, double wi,
-                           double* partials, double* out, cudaStream_t stream)
-{
-  const int blocks = reduction_blocks();
-  overlap_kernel<Real><<<blocks, kRedThreads, 0, stream>>>(static_cast<const typename ctype<Real>::c*>(lam),
-                                                           static_cast<const typename ctype<Real>::c*>(psi), 1ull << n,
-                                                           flip, sign, wr, wi, partials);
-  finish_partials_kernel<<<2, kFinishThreads, 0, stream>>>(partials, blocks, 2, out);
-  return cudaGetLastError();
-}
 
 // Several overlaps in one launch: blockIdx.y selects the Pauli of overlap y;
 // partials of overlap y sit at partials[(y * gridDim.x + x) * 2].
@@ -1978,8 +1943,6 @@ template cudaError_t launch_overlaps<float>(const void*, const void*, int, const
 
 template cudaError_t launch_pauli_apply<double>(const void*, void*, int, const pauli_sum&, cudaStream_t);
 template cudaError_t launch_pauli_apply<float>(const void*, void*, int, const pauli_sum&, cudaStream_t);
-template cudaError_t launch_overlap<double>(const void*, const void*, int, uint64_t, uint64_t, double, double, double*, double*, cudaStream_t);
-template cudaError_t launch_overlap<float>(const void*, const void*, int, uint64_t, uint64_t, double, double, double*, double*, cudaStream_t);
 
 }  // namespace rbk
 

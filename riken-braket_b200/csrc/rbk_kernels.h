@@ -16,7 +16,6 @@ constexpr int kMaxPauliTerms = 64;
 //   W(i) = sum_t w_t * (-1)^popcount(i & sign_t)     (physical bits)
 struct pauli_terms {
   int count;
-  int one_sided;  // 1: only the conj(a_i) a_{i^F} side with bit lowbit(F) of i clear (spin sums)
   uint64_t sign[kMaxPauliTerms];
   double w[kMaxPauliTerms][2];
 };
@@ -73,9 +72,6 @@ template <typename Real> cudaError_t launch_pauli_apply(const void* src, void* d
 // flip does not fit one layout.
 template <typename Real> cudaError_t launch_pauli_apply_tiled(const void* src, void* dst, int n, const pauli_sum& P,
                                                               cudaStream_t stream);
-// out (device, 2 doubles) = <lam| P |psi> with P = w (-1)^popcount(i & sign) X^flip
-template <typename Real> cudaError_t launch_overlap(const void* lam, const void* psi, int n, uint64_t flip, uint64_t sign,
-                                                    double wr, double wi, double* partials, double* out, cudaStream_t stream);
 // Up to kMaxOverlaps overlaps <lam| P_y |psi> in one launch; out[2y], out[2y+1] = (re, im) of overlap y.
 constexpr int kMaxOverlaps = 64;
 struct overlap_spec { uint64_t flip, sign; double wr, wi; };
