@@ -55,7 +55,7 @@ typedef struct rbk_state rbk_state;
 typedef struct rbk_stats {
   uint64_t gates_issued;     /* gate calls accepted */
   uint64_t passes;           /* fused read+write passes over the whole state */
-  uint64_t gate_launches;    /* unfused single-gate kernel launches */
+  uint64_t gate_launches;    /* single-gate kernel launches: 0, gates run in passes at every size */
   uint64_t reduction_passes; /* read-only passes (observables) */
   uint64_t relabel_passes;   /* passes that only moved qubits (layout changes) */
   uint64_t kernel_launches;  /* all kernels launched */
@@ -213,10 +213,10 @@ int rbk_shor_box(rbk_state* s, uint32_t num_exponent_qubits, uint64_t divisor, u
 
 /* ---- dense unitaries --------------------------------------------------------
  * u is 2^k x 2^k complex (re, im), row-major: u[r][c] = <r|U|c>, where bit i of
- * the basis index is qubits[i].  The qubits are first moved onto the low
- * physical bits by relabelling passes.  complex<float> states with k = 5 or 6
+ * the basis index is qubits[i].  complex<float> states with k = 5 or 6
  * (and n >= k + 7) run on the tensor cores as 3xTF32 split-precision GEMMs with
- * FP32 accumulation (tcgen05, accumulator in TMEM); other cases on CUDA cores.
+ * FP32 accumulation (tcgen05, accumulator in TMEM); other cases on CUDA cores,
+ * with the qubits where they lie.
  * No counterpart in ket beyond the fused blocks below; k <= 10. */
 int rbk_apply_unitary(rbk_state* s, const double* u, const uint32_t* qubits, int k);
 /* 0 (default): BEGIN/END FUSION blocks run gate by gate inside the fused passes.
@@ -321,10 +321,11 @@ int rbk_adjoint_gradient(int num_qubits, int precision, int device, const rbk_ci
 /* ---- batches of parametrised circuits (no counterpart in the reference) -----
  * Energies and adjoint gradients of many independent circuits of uneven size,
  * each with its own parameters and observable (same conventions as
- * rbk_adjoint_gradient).  Instances with n <= 12 (c128) / n <= 13 (c64) run in
- * one persistent kernel launch, replayed from a CUDA graph, one CTA per
- * instance with both state vectors in shared memory; the CTA size is chosen by
- * timing the candidates at rbk_batch_create.  Larger instances run through
+ * rbk_adjoint_gradient).  Instances of up to 15 qubits run in
+ * one launch per size class, replayed from a CUDA graph, one CTA (n <= 12 in
+ * c128, n <= 13 in c64) or one cluster of CTAs per instance with both state
+ * vectors in shared memory; the CTA size is chosen by timing the candidates at
+ * rbk_batch_create.  Larger instances run through
  * rbk_adjoint_gradient.  Parameters and gradients are concatenated in instance
  * order. */
 typedef struct rbk_batch rbk_batch;
