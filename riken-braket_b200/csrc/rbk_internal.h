@@ -193,18 +193,20 @@ struct dev_pass {
   dev_op ops[kMaxPassOps];
   alignas(16) double tabs[kMaxLayerTabs * kTabDoubles];  // factored layers' diagonal factors (complex<double> or complex<float>)
   // Straight passes: every phase is at most one layer of uncontrolled 2x2 gates
-  // in the factored form (its CNOT / X gates are all folded).  straight: the
-  // number of phases, 0 for any other pass.  The kernel for them is unrolled over
+  // in the factored form, then at most one run of phase gates (its CNOT / X gates
+  // are all folded).  straight: the number of phases, 0 for any other pass;
+  // straight_runs: some phase has a run.  The kernel for them is unrolled over
   // the phases, so that all of this sits at compile-time addresses.
   struct straight_layer {
     double t[8];              // t0, t1 of each register bit, in the state's precision
     double pre[kTabDoubles];  // a factor per register slot
     double post[kTabDoubles];
     uint32_t bits;            // register bits with a gate; kStraightPre: pre factors other than 1
-    uint32_t pad[3];
+    int32_t run;              // record of the PHASES header that follows the layer, or -1
+    uint32_t pad[2];
   };
   alignas(16) straight_layer straight_layers[kMaxStraight];
-  uint32_t straight, pad2[3];
+  uint32_t straight, straight_runs, pad2[2];
 };
 
 // Program of a state that fits one CTA's shared memory (n <= kSmallBits): the

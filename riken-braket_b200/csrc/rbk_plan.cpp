@@ -226,14 +226,14 @@ std::vector<phase_build> phases_by_dag(const std::vector<pop>& ops, const int* t
 }
 
 // Register phases of a straight pass: each takes ready 2x2 gates on up to R
-// different bits, then the ready CNOT / X gates that can fold into its write
-// layout (fold_trailing_x).  Empty if some gate is of another kind or the phases
-// do not fit kMaxStraight.
+// different bits, then the ready diagonal gates, then the ready CNOT / X gates
+// that can fold into its write layout (fold_trailing_x).  Empty if some gate is
+// of another kind or the phases do not fit kMaxStraight.
 std::vector<phase_build> phases_straight(const std::vector<pop>& ops, const int* tile_of_phys, uint64_t tile_mask, int R)
 {
   const int m = static_cast<int>(ops.size());
   for (const pop& o : ops)
-    if (o.kind != OPK_X ? o.kind != OPK_MAT || o.cmask : popc(o.cmask & tile_mask) > 1) return {};
+    if (o.kind == OPK_X ? popc(o.cmask & tile_mask) > 1 : o.kind == OPK_MAT ? o.cmask != 0 : o.kind != OPK_DIAG && o.kind != OPK_NEG) return {};
   std::vector<std::vector<int>> preds(m);
   for (int j = 0; j < m; ++j)
     for (int i = 0; i < j; ++i)
@@ -262,6 +262,12 @@ std::vector<phase_build> phases_straight(const std::vector<pop>& ops, const int*
       if (ops[j].kind == OPK_MAT && !(gates & bit(ops[j].target)) && fits(ops[j].target) && ready(j)) {
         gates |= bit(ops[j].target);
         take(j);
+      }
+    for (int j = 0; j < m; ++j)
+      if ((ops[j].kind == OPK_DIAG || ops[j].kind == OPK_NEG) && ready(j)) {
+        done[j] = 1;
+        --remaining;
+        pb.ops.push_back(j);
       }
     int conditional = 0;
     for (int j = 0; j < m; ++j) {
@@ -440,7 +446,8 @@ std::vector<dev_op> phase_members(const std::vector<dev_op>& list, size_t i, siz
 
 // headers_left: headers the pass may still add (kMaxPassOps - kMaxPassGates in
 // all), so that the gates of later phases still fit in the op records.
-void group_phase_runs(const plan_params& p, dev_pass& out, dev_phase& dp, int& op_end, int& headers_left)
+void group_phase_runs(const plan_params& p, dev_pass& out, dev_phase& dp, int& op_end, int& headers_left,
+                      size_t shortest = 2)
 {
   const int begin = dp.op_begin;
   std::vector<dev_op> list(out.ops + begin, out.ops + op_end);
@@ -451,15 +458,15 @@ void group_phase_runs(const plan_params& p, dev_pass& out, dev_phase& dp, int& o
     size_t j = i;
     while (j < list.size() && is_phase_op(list[j], true)) ++j;
     std::vector<dev_op> members;
-    if (j - i >= 2 && headers_left > 0) {
+    if (j - i >= shortest && headers_left > 0) {
       members = phase_members(list, i, j);
       if (static_cast<int>(members.size()) - static_cast<int>(j - i) > headers_left - 1 || members.empty()) {
         j = i;
         while (j < list.size() && is_phase_op(list[j], false)) ++j;
-        members = j - i >= 2 ? phase_members(list, i, j) : std::vector<dev_op>{};
+        members = j - i >= shortest ? phase_members(list, i, j) : std::vector<dev_op>{};
       }
     }
-    if (j - i >= 2 && headers_left > 0 && !members.empty()) {
+    if (j - i >= shortest && headers_left > 0 && !members.empty()) {
       auto cls = [&](const dev_op& g) {
         const int c = __builtin_popcount(g.creg);
         return c == 0 ? 0 : c == 1 ? 1 + __builtin_ctz(g.creg) : 1 + p.R;
@@ -912,7 +919,20 @@ bool build_pass(const plan_params& p, uint64_t tile_mask, const std::vector<pop>
     }
     if (p.fold_x) fold_trailing_x(p, out, dp, op_index, last && ds ? smode : 0);
     if (straight) {
-      if (!straight_layer_of(p, out.ops + dp.op_begin, op_index - dp.op_begin, out.straight_layers[ph])) return false;
+      const int begin = dp.op_begin;
+      int mats = begin;
+      while (mats < op_index && out.ops[mats].kind == OPK_MAT) ++mats;
+      dev_pass::straight_layer& layer = out.straight_layers[ph];
+      if (!straight_layer_of(p, out.ops + begin, mats - begin, layer)) return false;
+      layer.run = -1;
+      if (mats < op_index) {
+        dp.op_begin = static_cast<uint16_t>(mats);
+        group_phase_runs(p, out, dp, op_index, headers_left, 1);
+        dp.op_begin = static_cast<uint16_t>(begin);
+        if (out.ops[mats].kind != OPK_PHASES || mats + 1 + static_cast<int>(out.ops[mats].run) != op_index) return false;
+        layer.run = mats;
+        out.straight_runs = 1;
+      }
       dp.op_end = static_cast<uint16_t>(op_index);
       continue;
     }
@@ -935,7 +955,10 @@ void build_pass(const plan_params& p, uint64_t tile_mask, const std::vector<pop>
   for (int b = 0; b < p.K; ++b) tile_of_phys[tile_phys[b]] = b;
   if (p.straight) {
     const std::vector<phase_build> phases = phases_straight(ops, tile_of_phys, tile_mask, p.R);
-    if (!phases.empty())
+    // With diagonal gates (a QFT's: one Hadamard a layer) the general form may need fewer
+    // phases; one more than it is worth the straight kernel.
+    const bool diagonal = std::any_of(ops.begin(), ops.end(), [](const pop& o) { return o.kind == OPK_DIAG || o.kind == OPK_NEG; });
+    if (!phases.empty() && (!diagonal || phases.size() <= phases_by_dag(ops, tile_of_phys, p.R, false).size() + 1))
       for (const bool direct : {true, false})
         if (build_pass(p, tile_mask, ops, relabel_to, tile_phys, phases, true, direct, out)) return;
   }

@@ -34,8 +34,13 @@ static double layer_error(const plan_params& p, const dev_pass& P, std::mt19937_
     for (auto& x : a) x = cplx{nd(rng), nd(rng)};
     want = a;
     run_layer(p, P.straight_layers[ph], a);
+    if (P.straight_layers[ph].run >= 0 && (!P.straight_runs || P.ops[P.straight_layers[ph].run].kind != OPK_PHASES)) return 1.0;
     for (int o = P.phases[ph].op_begin; o < P.phases[ph].op_end; ++o) {
       const dev_op& g = P.ops[o];
+      if (g.kind == OPK_PHASES) {  // one run, the last records of the phase (run_pass checks its members)
+        if (P.straight_layers[ph].run != o || o + 1 + int(g.run) != P.phases[ph].op_end) return 1.0;
+        break;
+      }
       if (g.kind != OPK_MAT || g.creg || g.cthr || g.cout) return 1.0;  // nothing else may be left in a straight pass
       hgate h{};
       h.kind = OPK_MAT;
@@ -76,7 +81,7 @@ static std::vector<hgate> cnot_gates(std::mt19937_64& rng, int n, int count, boo
 
 int main()
 {
-  int failures = 0, most_phases = 0, most_folds = 0;
+  int failures = 0, most_phases = 0, most_folds = 0, with_runs = 0;
   for (int prec = 0; prec < 2; ++prec)
   for (int seed = 0; seed < 24; ++seed) {
     std::mt19937_64 rng(7000 * prec + seed);
@@ -88,7 +93,7 @@ int main()
     p.dense_budget = seed % 8 == 7 ? 30 : 1 + static_cast<int>(rng() % 20);
     p.straight = true;
     const bool others = seed % 4 == 3;
-    const auto gates = seed % 2 ? cnot_gates(rng, p.n, 200, others) : brick_gates(rng, p.n, 6);
+    const auto gates = seed % 8 == 1 ? ansatz_gates(rng, p.n, 6) : seed % 2 ? cnot_gates(rng, p.n, 200, others) : brick_gates(rng, p.n, 6);
     std::vector<cplx> st(1ull << p.n), want;
     std::normal_distribution<double> nd;
     for (auto& x : st) x = cplx{nd(rng), nd(rng)};
@@ -105,6 +110,7 @@ int main()
       run_pass(st, p, P);
       if (!P.straight) continue;
       ++straight;
+      with_runs += P.straight_runs != 0;
       if (P.straight != P.num_phases || P.straight > unsigned(kMaxStraight)) ++failures;
       layers = std::max(layers, layer_error(p, P, rng));
       most_phases = std::max<int>(most_phases, P.num_phases);
@@ -121,8 +127,8 @@ int main()
     if (!(err < (prec == 0 ? 1e-12 : 1e-5)) || !(layers < (prec == 0 ? 1e-13 : 3e-6))) ++failures;
     if (seed % 2 == 0 && straight == 0) ++failures;  // brick circuits
   }
-  std::printf("phases up to %d, conditional folds up to %d\n", most_phases, most_folds);
-  if (most_phases != kMaxStraight || most_folds == 0) ++failures;
+  std::printf("phases up to %d, conditional folds up to %d, passes with phase runs %d\n", most_phases, most_folds, with_runs);
+  if (most_phases != kMaxStraight || most_folds == 0 || with_runs == 0) ++failures;
   std::printf(failures ? "FAILED %d\n" : "ALL OK\n", failures);
   return failures ? 1 : 0;
 }

@@ -1,5 +1,5 @@
-"""Straight passes (layers of uncontrolled 2x2 gates whose CNOT / X gates all fold
-into the exchanges): the planner's programs on the host against the gates one by
+"""Straight passes (layers of uncontrolled 2x2 gates, runs of phase gates, and
+CNOT / X gates that all fold into the exchanges): the planner's programs on the host against the gates one by
 one, and the kernel against the oracle and against the general tile pass (tile
 shape 0 has no straight form) at the smallest state of the kind, at odd sizes and
 at every number of phases.  Tolerances: rounding 1e-16 (6e-8 in complex<float>) at
@@ -28,12 +28,15 @@ def test_straight_programs_are_exact(tmp_path):
     assert "ALL OK" in r.stdout
 
 
+ANGLES = {"U3": 3, "U1": 1, "EZ": 1}
+
+
 def cnot_circuit(n, rng, count, rare):
     ops = []
     for _ in range(count):
         a, b = (int(x) for x in rng.permutation(n)[:2])
         kind = str(rng.choice(["U3", "U3", "H", "X", "CNOT", "CNOT"] + rare))
-        ops.append((kind, (a, b) if kind in ("CNOT", "CZ") else (a,), tuple(rng.uniform(-3, 3, 3)) if kind == "U3" else ()))
+        ops.append((kind, (a, b) if kind in ("CNOT", "CZ") else (a,), tuple(rng.uniform(-3, 3, ANGLES.get(kind, 0)))))
     return ops
 
 
@@ -42,7 +45,8 @@ def cnot_circuit(n, rng, count, rare):
 @pytest.mark.parametrize("n", [13, 14, 16, 17])
 def test_straight_passes_vs_oracle(pkg, precision, n):
     rng = np.random.default_rng(n)
-    circuits = [pkg.circuits.brick(n, 5, seed=n), cnot_circuit(n, rng, 300, []), cnot_circuit(n, rng, 300, ["CZ"])]
+    circuits = [pkg.circuits.brick(n, 5, seed=n), cnot_circuit(n, rng, 300, []), cnot_circuit(n, rng, 300, ["CZ", "U1", "Z", "EZ"]),
+                pkg.circuits.ansatz(n, 4, seed=n)[0]]
     for ops in circuits:
         ref = oracle.COracle(n)
         ref.apply(ops)
