@@ -1,5 +1,6 @@
 // rbk::simplify_queue on random queues of every gate form: the state it gives
-// equals the original's, gates that are not plain unitaries included.
+// equals the original's, gates that are not plain unitaries included; and the
+// matrices it makes of rotations close to pi are as exact as those it is given.
 #include <cmath>
 #include <complex>
 #include <cstdint>
@@ -11,10 +12,10 @@
 
 using cd = std::complex<double>;
 
-static cd at(const double* m, int k) { return {m[2 * k], m[2 * k + 1]}; }
-
-static void apply(std::vector<cd>& a, const rbk::hgate& g)
+template <typename C>
+static void apply(std::vector<C>& a, const rbk::hgate& g)
 {
+  auto at = [](const double* m, int k) { return C(m[2 * k], m[2 * k + 1]); };
   for (uint32_t i = 0; i < a.size(); ++i) {
     if (g.kind == rbk::HK_SWAP) {
       const uint32_t x = 1u << g.target, y = 1u << g.target2;
@@ -30,11 +31,66 @@ static void apply(std::vector<cd>& a, const rbk::hgate& g)
       continue;
     }
     if (i & t) continue;
-    const cd x = a[i], y = a[i | t];
+    const C x = a[i], y = a[i | t];
     if (g.kind == rbk::OPK_X) { a[i] = y; a[i | t] = x; }
-    else if (g.kind == rbk::OPK_Y) { a[i] = cd{y.imag(), -y.real()}; a[i | t] = cd{-x.imag(), x.real()}; }
+    else if (g.kind == rbk::OPK_Y) { a[i] = C{y.imag(), -y.real()}; a[i | t] = C{-x.imag(), x.real()}; }
     else { a[i] = at(g.m, 0) * x + at(g.m, 1) * y; a[i | t] = at(g.m, 2) * x + at(g.m, 3) * y; }
   }
+}
+
+// Chains of U3, CZ, U3, CNOT on 2 qubits with |cos(theta / 2)| from 1e-3 to 1, whose
+// matrices take phases and X rotations from one another.  Every simplified matrix is a
+// product of at most 4 of some 4 roundings each: 16 * 1.1e-16 in each entry, twice
+// that in its unitarity.  The states are evaluated in long double, so that their
+// distance is the matrices' rounding alone, which adds up over 24 gates like a random
+// walk: 5 * 16 * 1.1e-16.
+static bool precise_near_pi()
+{
+  using cl = std::complex<long double>;
+  std::mt19937_64 rng(5);
+  std::uniform_real_distribution<double> u(-3.2, 3.2), e(-3.0, 0.0);
+  double defect = 0;
+  long double distance = 0;
+  for (int run = 0; run < 20000; ++run) {
+    std::vector<rbk::hgate> q;
+    for (int k = 0; k < 12; ++k) {
+      for (int b = 0; b < 2; ++b) {
+        rbk::hgate g{};
+        g.kind = rbk::OPK_MAT;
+        g.target = int8_t(b);
+        g.target2 = -1;
+        const double c = std::pow(10.0, e(rng)), s = std::sqrt((1.0 - c) * (1.0 + c)), p = u(rng), l = u(rng);
+        const cd v[4] = {c, -s * std::polar(1.0, l), s * std::polar(1.0, p), c * std::polar(1.0, p + l)};
+        for (int i = 0; i < 4; ++i) { g.m[2 * i] = v[i].real(); g.m[2 * i + 1] = v[i].imag(); }
+        q.push_back(g);
+      }
+      rbk::hgate g{};
+      g.target2 = -1;
+      const bool cz = rng() % 2;
+      g.kind = cz ? rbk::OPK_NEG : rbk::OPK_X;
+      g.target = cz ? int8_t(-1) : int8_t(rng() % 2);
+      g.cmask = cz ? 3ull : 1ull << (1 - g.target);
+      q.push_back(g);
+    }
+    const auto s = rbk::simplify_queue(2, q);
+    for (const auto& g : s) {
+      if (g.kind != rbk::OPK_MAT) continue;
+      const cl a(g.m[0], g.m[1]), b(g.m[2], g.m[3]), c(g.m[4], g.m[5]), d(g.m[6], g.m[7]);
+      defect = std::max({defect, double(std::abs(std::norm(a) + std::norm(b) - 1)), double(std::abs(std::norm(c) + std::norm(d) - 1)),
+                         double(std::abs(a * std::conj(c) + b * std::conj(d)))});
+    }
+    std::vector<cl> x(4), y;
+    for (auto& v : x) v = cl{u(rng), u(rng)};
+    y = x;
+    long double norm = 0, err = 0;
+    for (const auto& v : x) norm += std::norm(v);
+    for (const auto& g : q) apply(x, g);
+    for (const auto& g : s) apply(y, g);
+    for (size_t i = 0; i < x.size(); ++i) err += std::norm(x[i] - y[i]);
+    distance = std::max(distance, std::sqrt(err / norm));
+  }
+  std::printf("rotations close to pi: unitarity defect %.3g, distance %.3Lg\n", defect, distance);
+  return defect <= 32 * 1.1e-16 && distance <= 80 * 1.1e-16L;
 }
 
 int main()
@@ -101,6 +157,7 @@ int main()
   std::printf("gates %zu -> %zu, worst relative error %.3g\n", before, after, worst);
   // 60 gates of some 1e-16 each; a non-unitary gate may shrink the state against its rounding by 1e2
   if (!(worst < 1e-12) || after >= before) { std::printf("FAILED\n"); return 1; }
+  if (!precise_near_pi()) { std::printf("FAILED\n"); return 1; }
   std::printf("ALL OK\n");
   return 0;
 }
