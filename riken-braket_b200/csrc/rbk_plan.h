@@ -77,9 +77,10 @@ struct small_program {
 // The queue in register phases of a small state: emit(ops, indices, phase) for
 // each, with the ops in physical bits, the gates they come from, and the phase's
 // register bits.  A phase takes, in order, every gate that commutes with those
-// it leaves behind and whose target is, or can still join, its register bits, at
-// most max_ops of them and max_marked of the marked ones (marked: one entry per
-// gate, or empty); SWAPs only update the layout map.
+// it leaves behind (it looks past a few hundred of them) and whose target is, or
+// can still join, its register bits, at most max_ops of them and max_marked of
+// the marked ones (marked: one entry per gate, or empty); SWAPs only update the
+// layout map.  The time is linear in the number of gates.
 void plan_small_phases(int n, const std::vector<hgate>& gates, std::vector<int>& perm, std::vector<int>& inv, size_t max_ops,
                        const std::vector<char>& marked, int max_marked,
                        const std::function<void(const std::vector<small_op>&, const std::vector<size_t>&, const small_phase&)>& emit);

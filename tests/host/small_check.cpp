@@ -1,10 +1,12 @@
 // CPU model of small_circuit_kernel over the programs of rbk::plan_small: every
 // phase through the kernel's index arithmetic (swizzled slots, register and base
-// masks), against the gates applied one by one to a logical state.
+// masks), against the gates applied one by one to a logical state.  Then the time
+// that planning a long queue takes where a qubit is never a target.
 #include <complex>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
+#include <ctime>
 #include <random>
 #include <set>
 #include <vector>
@@ -177,6 +179,36 @@ int main()
     }
   std::printf("worst relative error %.3g\n", worst);
   if (!(worst < 1e-12)) fail("error");
+  // 200,000 gates on 11 of 12 qubits, the twelfth idle or only a control: 0.1 s here
+  // where a phase looks ahead a bounded way, 60 s where it scans the whole queue.
+  for (const bool control : {false, true}) {
+    constexpr int n = 12, count = 200000;
+    std::vector<rbk::hgate> q;
+    for (int k = 0; k < count; ++k) {
+      rbk::hgate g{};
+      g.target2 = -1;
+      g.target = int8_t(rng() % (n - 1));
+      if (rng() % 2) {
+        g.kind = rbk::OPK_X;
+        g.cmask = 1ull << (control && rng() % 3 == 0 ? n - 1 : (g.target + 1 + rng() % (n - 2)) % (n - 1));
+      } else {
+        g.kind = rbk::OPK_MAT;
+        g.m[0] = g.m[6] = 0.6; g.m[2] = 0.8; g.m[4] = -0.8;
+      }
+      q.push_back(g);
+    }
+    std::vector<int> perm(n), inv(n);
+    for (int b = 0; b < n; ++b) perm[b] = inv[b] = b;
+    std::vector<rbk::small_program> progs;
+    const std::clock_t t0 = std::clock();
+    rbk::plan_small(n, q, perm, inv, progs);
+    const double seconds = double(std::clock() - t0) / CLOCKS_PER_SEC;
+    size_t ops = 0;
+    for (const auto& p : progs) ops += p.ops.size();
+    std::printf("%d gates planned in %.3f s\n", count, seconds);
+    if (ops != count) fail("gates lost");
+    if (seconds > 5.0) fail("planning time");
+  }
   std::printf("ALL OK\n");
   return 0;
 }

@@ -2,7 +2,8 @@
 rbk::plan_small, executed by a C++ model of small_circuit_kernel
 (tests/host/small_check.cpp), equal the gates applied one by one, for every
 size from 1 to 12 qubits, programs longer than one launch, SWAPs and layout maps
-that are not the identity.  The model is built with AddressSanitizer."""
+that are not the identity; and planning takes time linear in the queue where a
+qubit is never a target.  The model is built with AddressSanitizer."""
 import os
 import shutil
 import subprocess
