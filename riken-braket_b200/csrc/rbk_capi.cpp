@@ -1617,11 +1617,12 @@ int launch_rotations(rbk::adjoint_workspace& w, rbk_state* lam, rbk_state* psi,
 {
   const bool c128 = w.precision == RBK_C128;
   const size_t room = kRotateLaunches * rbk::pair_rotate_partials_doubles();
-  if (!w.rpart) {
-    RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&w.rpart), sizeof(double) * room));
+  // Each on its own: a sweep in which one could not be had leaves the others to the next.
+  if (!w.rpart) RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&w.rpart), sizeof(double) * room));
+  if (!w.d_rresults)
     RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&w.d_rresults), sizeof(rbk::pair_rotate_result) * kRotateResults));
+  if (!w.h_rresults)
     RBK_CUDA(cudaMallocHost(reinterpret_cast<void**>(&w.h_rresults), sizeof(rbk::pair_rotate_result) * kRotateResults));
-  }
   for (const rbk::pair_rotate_set& set : rbk::plan_rotations(w.n, items, owed)) {
     if (w.rused + rbk::pair_rotate_partials_doubles() > room ||
         w.rresults.size() + rbk::kMaxRotFlips + rbk::kMaxQubits > kRotateResults)

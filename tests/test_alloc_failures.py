@@ -1,0 +1,27 @@
+"""Host logic (CPU, no GPU): an allocation that fails inside a call is reported
+by that call and leaves the object usable -- tests/host/alloc_check.cpp runs
+rbk_capi.cpp over a fake CUDA runtime that fails one allocation after the other.
+Built with AddressSanitizer."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+
+def test_calls_recover_from_failed_allocations(tmp_path):
+    if not shutil.which("g++"):
+        pytest.skip("no host C++ compiler")
+    exe = tmp_path / "alloc_check"
+    csrc = os.path.join(ROOT, "riken-braket_b200", "csrc")
+    cuda_inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    # rbk_capi.cpp names launches that these calls never reach; only those they reach have a fake.
+    subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-fsanitize=address", "-fno-omit-frame-pointer", "-no-pie",
+                    "-Wl,--unresolved-symbols=ignore-in-object-files", "-I", csrc, "-I", os.path.join(ROOT, "include"),
+                    "-I", cuda_inc, "-o", str(exe), os.path.join(ROOT, "tests", "host", "alloc_check.cpp"),
+                    *(os.path.join(csrc, f) for f in ("rbk_capi.cpp", "rbk_plan.cpp", "rbk_rotate_plan.cpp"))], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
+    assert "ALL OK" in r.stdout
