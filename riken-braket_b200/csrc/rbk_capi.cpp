@@ -2714,11 +2714,15 @@ int apply_unitary(rbk_state* s, const std::vector<cplx>& U, const uint32_t* q, i
       b += len;
     }
     const std::vector<float> w = build_w_split(U, k);
-    if (!s->d_tc_w) {  // once per state: W of the largest k, and the sticky error flag
-      RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&s->d_tc_w), sizeof(float) * rbk::tc_w_split_floats(6)));
-      RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&s->d_tc_flag), sizeof(int)));
+    // Once per state: W of the largest k, and the sticky error flag.  Each on its own, so
+    // that a call in which one could not be had leaves the others to the next.
+    if (!s->d_tc_w) RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&s->d_tc_w), sizeof(float) * rbk::tc_w_split_floats(6)));
+    if (!s->h_tc_flag) {
       RBK_CUDA(cudaMallocHost(reinterpret_cast<void**>(&s->h_tc_flag), sizeof(int)));
       *s->h_tc_flag = 0;
+    }
+    if (!s->d_tc_flag) {
+      RBK_CUDA(cudaMalloc(reinterpret_cast<void**>(&s->d_tc_flag), sizeof(int)));
       RBK_CUDA(cudaMemsetAsync(s->d_tc_flag, 0, sizeof(int), s->stream));
     }
     // Stream order keeps this copy behind the previous unitary's reads of the buffer; the

@@ -178,6 +178,16 @@ int main()
       };
     });
   }
+  // A dense unitary of 5 qubits on the tensor cores.
+  std::vector<double> u(2 * 32 * 32, 0.0);
+  for (int r = 0; r < 32; ++r) u[2 * (33 * r)] = 1.0;
+  const uint32_t qubits[5] = {0, 1, 2, 3, 4};
+  sweep("unitary", [&] {
+    rbk_state* s = nullptr;
+    if (rbk_state_create(n, RBK_C64, 0, 0, &s) != RBK_OK) fail(rbk_last_error());
+    const std::shared_ptr<rbk_state> held(s, rbk_state_destroy);
+    return [&, held] { return rbk_apply_unitary(held.get(), u.data(), qubits, 5); };
+  });
   std::printf("ALL OK\n");
   return 0;
 }
