@@ -16,6 +16,7 @@
 #include "rbk_device.cuh"
 #include "rbk_internal.h"
 #include "rbk_kernels.h"
+#include "rbk_sample_scan.h"
 #include "rbk_small_core.cuh"
 
 namespace rbk {
@@ -2025,18 +2026,17 @@ sample_sums_kernel(const typename ctype<Real>::c* __restrict__ a, uint64_t size,
 }
 
 // Inclusive scan of v[0..count) in place by one block: thread t sums and then
-// rewrites its own run of consecutive values.  At most 2^21 chunks (33 qubits).
+// rewrites its own run of consecutive values (rbk_sample_scan.h).  At most 2^21
+// chunks (33 qubits).
 constexpr int kSampleScanThreads = 1024;
 __global__ void __launch_bounds__(kSampleScanThreads) sample_scan_kernel(double* __restrict__ v, uint64_t count)
 {
-  __shared__ double warp_tot[kSampleScanThreads / 32];
+  __shared__ double warp_tot[kSampleScanThreads / 32], warp_end[kSampleScanThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t per = (count + kSampleScanThreads - 1) / kSampleScanThreads;
   const uint64_t lo = min(count, threadIdx.x * per), hi = min(count, lo + per);
-  double run = 0.0;
-#pragma unroll 8
-  for (uint64_t i = lo; i < hi; ++i) run += v[i];
-  double incl = run;
+  uint64_t last;
+  double incl = scan_run(v, lo, hi, &last);
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const double y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -2046,17 +2046,18 @@ __global__ void __launch_bounds__(kSampleScanThreads) sample_scan_kernel(double*
   __syncthreads();
   double off = 0.0;
   for (int w = 0; w < warp; ++w) off += warp_tot[w];
-  // The start of a run is the end of the one before it, bit for bit, so that the
-  // scanned values never decrease from one thread's run to the next.
-  double before = __shfl_up_sync(0xffffffffu, incl, 1);
-  if (lane == 0) before = 0.0;
-  double acc = off + before;
-  const double end = off + incl;
-#pragma unroll 8
-  for (uint64_t i = lo; i < hi; ++i) {
-    acc += v[i];
-    v[i] = i + 1 == hi ? end : min(acc, end);
+  double end = last > lo ? off + incl : 0.0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end = scan_later(y, end);
   }
+  if (lane == 31) warp_end[warp] = end;
+  __syncthreads();
+  double prev = 0.0;
+  for (int w = 0; w < warp; ++w) prev = scan_later(prev, warp_end[w]);
+  const double y = __shfl_up_sync(0xffffffffu, end, 1);
+  scan_write(v, lo, hi, last, lane > 0 ? scan_later(prev, y) : prev, scan_later(prev, end));
 }
 
 // One warp per sample: events[k] = first index whose prefix sum exceeds r[k].

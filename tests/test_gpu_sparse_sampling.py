@@ -26,3 +26,20 @@ def test_sparse_state_events_vs_oracle(pkg, n):
             ev = s.generate_events(num, 7 + num)
             assert np.array_equal(ev, o.generate_events(num, 7 + num))
             assert np.all(np.abs(a[ev]) > 0)
+
+
+def test_sparse_chunks_vs_oracle(pkg):
+    """24 qubits: four chunks per thread of the scan, 19 of 20 of weight zero."""
+    n = 24
+    rng = np.random.default_rng(n)
+    a = np.zeros((1 << (n - 12), 4096), dtype=np.complex128)
+    chunks = rng.permutation(a.shape[0])[:a.shape[0] // 20]
+    a[chunks[:, None], rng.integers(4096, size=(chunks.size, 3))] = 10.0 ** rng.uniform(-6, 0, (chunks.size, 3))
+    a = a.ravel() / np.linalg.norm(a)
+    with pkg.State(n) as s:
+        s.upload(a)
+        o = oracle.COracle(n)
+        o.set_amplitudes(a)
+        ev = s.generate_events(5000, 3)
+        assert np.array_equal(ev, o.generate_events(5000, 3))
+        assert np.all(np.abs(a[ev]) > 0)
