@@ -26,10 +26,10 @@ class CircuitGate(ctypes.Structure):
 def gate_array(spec):
     """spec: list of (mnemonic, qubits, param_index or None, scale, angles)."""
     arr = (CircuitGate * max(1, len(spec)))()
-    if rbk.marshal():
-        rbk.marshal().fill_gates(ctypes.addressof(arr), spec, GATE)
-        return arr, len(spec)
-    for i, (mnem, qubits, param, scale, angles) in enumerate(spec):
+    count = len(spec)
+
+    def one(i, gate):
+        mnem, qubits, param, scale, angles = gate
         g = arr[i]
         g.kind = GATE[mnem]
         for j, q in enumerate(qubits[:2]):
@@ -38,7 +38,13 @@ def gate_array(spec):
         g.scale = float(scale)
         for j, a in enumerate(angles[:3]):
             g.angles[j] = float(a)
-    return arr, len(spec)
+
+    if rbk.marshal():
+        rbk.marshal().fill_gates(ctypes.addressof(arr), count, spec, GATE, one)
+    else:
+        for i, gate in enumerate(spec):
+            one(i, gate)
+    return arr, count
 
 
 def ansatz_spec(n, layers):

@@ -6,6 +6,9 @@
 // instructions: 426 us, a third of the call); here it is some 0.1 us.
 // fill_gates(): a parametrised circuit as the array of rbk_circuit_gate that
 // the adjoint calls take (960 gates: 558 us in Python).
+// Both take the plain forms only and hand any other to the Python code that
+// converts through ctypes, so that what is accepted, what is refused and with
+// which error do not depend on this module.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -55,215 +58,301 @@ PyObject* py_bind(PyObject*, PyObject* args)
   Py_RETURN_NONE;
 }
 
-// A tuple or list as it is, any other sequence (a numpy row, say) as a new tuple.
-struct as_sequence {
+// A Python object's reference, given back at the end of the scope.
+struct held {
   PyObject* o = nullptr;
-  explicit as_sequence(PyObject* x)
-  {
-    if (!x) return;
-    if (PyTuple_Check(x) || PyList_Check(x)) {
-      Py_INCREF(x);
-      o = x;
-    } else {
-      o = PySequence_Tuple(x);
-    }
-  }
-  as_sequence(const as_sequence&) = delete;
-  ~as_sequence() { Py_XDECREF(o); }
+  explicit held(PyObject* x) : o(x) {}
+  held(const held&) = delete;
+  ~held() { Py_XDECREF(o); }
 };
 
-// Element i of a tuple or list, borrowed; nullptr with IndexError set when there is none.
-PyObject* item(PyObject* seq, Py_ssize_t i)
+// A plain tuple or list; its items, nullptr past the end.
+inline bool plain(PyObject* x) { return PyTuple_CheckExact(x) || PyList_CheckExact(x); }
+inline Py_ssize_t plain_size(PyObject* x) { return PyTuple_CheckExact(x) ? PyTuple_GET_SIZE(x) : PyList_GET_SIZE(x); }
+inline PyObject* plain_item(PyObject* x, Py_ssize_t i)
 {
-  if (!seq) return nullptr;  // an error is set
-  if (PyTuple_Check(seq)) {
-    if (i < PyTuple_GET_SIZE(seq)) return PyTuple_GET_ITEM(seq, i);
-  } else if (PyList_Check(seq)) {
-    if (i < PyList_GET_SIZE(seq)) return PyList_GET_ITEM(seq, i);
-  } else {
-    PyErr_SetString(PyExc_TypeError, "expected a tuple or list");
-    return nullptr;
-  }
-  PyErr_SetString(PyExc_IndexError, "tuple index out of range");
-  return nullptr;
+  if (i >= plain_size(x)) return nullptr;
+  return PyTuple_CheckExact(x) ? PyTuple_GET_ITEM(x, i) : PyList_GET_ITEM(x, i);
 }
 
-bool get_qubit(PyObject* seq, Py_ssize_t i, uint32_t* out)
+// x[i] as Python subscripts it, a new reference; nullptr, with an error set or
+// not, where there is none.  An object of its own class may run any code.
+inline PyObject* subscript(PyObject* x, Py_ssize_t i, bool* foreign)
 {
-  PyObject* o = item(seq, i);
-  if (!o) return false;
-  PyObject* idx = PyNumber_Index(o);
-  if (!idx) return false;
-  *out = static_cast<uint32_t>(PyLong_AsUnsignedLongMask(idx));  // a negative index wraps, and is refused as out of range
-  Py_DECREF(idx);
+  if (plain(x)) {
+    PyObject* o = plain_item(x, i);
+    Py_XINCREF(o);
+    return o;
+  }
+  *foreign = true;
+  const held index(PyLong_FromSsize_t(i));
+  return index.o ? PyObject_GetItem(x, index.o) : nullptr;
+}
+
+// The conversions below return false, with an error set or not, where the value
+// is one for the ctypes calls to judge.
+inline bool as_qubit(PyObject* o, uint32_t* out, bool* foreign)
+{
+  if (PyLong_CheckExact(o)) {
+    *out = static_cast<uint32_t>(PyLong_AsUnsignedLongMask(o));  // a negative index wraps, and is refused as out of range
+    return true;
+  }
+  *foreign = true;
+  if (!PyIndex_Check(o)) return false;
+  const held v(PyNumber_Index(o));
+  if (!v.o) return false;
+  *out = static_cast<uint32_t>(PyLong_AsUnsignedLongMask(v.o));
   return !PyErr_Occurred();
 }
 
-bool get_real(PyObject* seq, Py_ssize_t i, double* out)
+inline bool as_real(PyObject* o, double* out, bool* foreign)
 {
-  PyObject* o = item(seq, i);
-  if (!o) return false;
+  if (PyFloat_CheckExact(o)) {
+    *out = PyFloat_AS_DOUBLE(o);
+    return true;
+  }
+  if (!PyLong_CheckExact(o)) *foreign = true;
   *out = PyFloat_AsDouble(o);
   return !PyErr_Occurred();
 }
 
-// As float(x) takes it: strings of digits too.
-bool get_float(PyObject* seq, Py_ssize_t i, double* out)
+// int(o), where it fits.
+inline bool as_int(PyObject* o, int* out, bool* foreign)
 {
-  PyObject* o = item(seq, i);
-  PyObject* v = o ? PyNumber_Float(o) : nullptr;
-  if (!v) return false;
-  *out = PyFloat_AS_DOUBLE(v);
-  Py_DECREF(v);
-  return true;
-}
-
-// int(value) of element i.
-bool get_int(PyObject* seq, Py_ssize_t i, int* out)
-{
-  PyObject* o = item(seq, i);
-  if (!o) return false;
-  PyObject* v = PyNumber_Long(o);
-  if (!v) return false;
-  const long x = PyLong_AsLong(v);
-  Py_DECREF(v);
+  if (PyLong_CheckExact(o)) {
+    int overflow = 0;
+    *out = static_cast<int>(PyLong_AsLongAndOverflow(o, &overflow));
+    return overflow == 0;
+  }
+  *foreign = true;
+  const held v(PyNumber_Long(o));
+  if (!v.o) return false;
+  const long x = PyLong_AsLong(v.o);
   if (PyErr_Occurred()) return false;
   *out = static_cast<int>(x);
   return true;
 }
 
-// apply(state, ops): every instruction in order; the first failing call's status code, or 0.
+// float(o): strings of digits too.
+inline bool as_float(PyObject* o, double* out, bool* foreign)
+{
+  if (PyFloat_CheckExact(o)) {
+    *out = PyFloat_AS_DOUBLE(o);
+    return true;
+  }
+  if (!PyLong_CheckExact(o)) *foreign = true;
+  const held v(PyNumber_Float(o));
+  if (!v.o) return false;
+  *out = PyFloat_AS_DOUBLE(v.o);
+  return true;
+}
+
+template <auto as, typename T>
+inline bool at(PyObject* x, Py_ssize_t i, T* out, bool* foreign)
+{
+  const held o(subscript(x, i, foreign));
+  return o.o && as(o.o, out, foreign);
+}
+
+// Whether an error other than a conversion's (an interrupt, say) is set; a
+// conversion's is cleared.
+bool hard_error()
+{
+  if (!PyErr_Occurred()) return false;
+  if (!PyErr_ExceptionMatches(PyExc_Exception)) return true;
+  PyErr_Clear();
+  return false;
+}
+
+// The C handle of a State (its attribute h, a c_void_p or None) in *s; 0 with an error set.
+int handle_of(PyObject* state, rbk_state** s)
+{
+  *s = nullptr;
+  const held h(PyObject_GetAttrString(state, "h"));
+  if (!h.o) return 0;
+  if (h.o == Py_None) return 1;
+  const held v(PyObject_GetAttrString(h.o, "value"));
+  if (!v.o) return 0;
+  if (v.o != Py_None) *s = static_cast<rbk_state*>(PyLong_AsVoidPtr(v.o));
+  return !PyErr_Occurred();
+}
+
+// One instruction.  1: called, with its status in *rc; 0: not of the plain form
+// (or one that the ctypes calls refuse, whose error they raise).
+int apply_plain(PyObject* state, rbk_state* s, PyObject* op, int* rc, bool* foreign)
+{
+  if (!plain(op) || plain_size(op) != 3 || !PyUnicode_CheckExact(plain_item(op, 0))) return 0;
+  const held name_o(Py_NewRef(plain_item(op, 0))), q_o(Py_NewRef(plain_item(op, 1))), p_o(Py_NewRef(plain_item(op, 2)));
+  PyObject *q = q_o.o, *p = p_o.o;
+  Py_ssize_t length = 0;
+  const char* name = PyUnicode_AsUTF8AndSize(name_o.o, &length);
+  if (!name || std::strlen(name) != static_cast<size_t>(length)) return 0;
+  uint32_t a = 0, b = 0;
+  double x = 0, y = 0, z = 0;
+  int n = 0;
+  const uint32_t* none = nullptr;
+  // Foreign code may have closed the state.
+  auto usable = [&] { return !*foreign || (handle_of(state, &s) && s); };
+  auto qubit = [&](Py_ssize_t i, uint32_t* out) { return at<as_qubit>(q, i, out, foreign); };
+  auto real = [&](Py_ssize_t i, double* out) { return at<as_real>(p, i, out, foreign); };
+#define RBK_CALL(expr) { if (!usable()) return 0; Py_BEGIN_ALLOW_THREADS *rc = (expr); Py_END_ALLOW_THREADS return 1; }
+  if (!std::strcmp(name, "U3")) {
+    if (real(0, &x) && real(1, &y) && real(2, &z) && qubit(0, &a)) RBK_CALL(A.phase_shift3(s, x, y, z, a, none, 0))
+  } else if (!std::strcmp(name, "CNOT")) {
+    if (qubit(1, &b) && qubit(0, &a)) RBK_CALL(A.pauli_x(s, b, &a, 1))
+  } else if (!std::strcmp(name, "H")) {
+    if (qubit(0, &a)) RBK_CALL(A.hadamard(s, a, none, 0))
+  } else if (!std::strcmp(name, "X")) {
+    if (qubit(0, &a)) RBK_CALL(A.pauli_x(s, a, none, 0))
+  } else if (!std::strcmp(name, "Y")) {
+    if (qubit(0, &a)) RBK_CALL(A.pauli_y(s, a, none, 0))
+  } else if (!std::strcmp(name, "Z")) {
+    if (qubit(0, &a)) RBK_CALL(A.pauli_z(s, &a, 1))
+  } else if (!std::strcmp(name, "U1")) {
+    if (real(0, &x) && qubit(0, &a)) RBK_CALL(A.phase_shift(s, x, &a, 1))
+  } else if (!std::strcmp(name, "U2")) {
+    if (real(0, &x) && real(1, &y) && qubit(0, &a)) RBK_CALL(A.phase_shift2(s, x, y, a, none, 0))
+  } else if (!std::strcmp(name, "CZ")) {
+    uint32_t qs[2];
+    if (qubit(0, &qs[0]) && qubit(1, &qs[1])) RBK_CALL(A.pauli_z(s, qs, 2))
+  } else if (!std::strcmp(name, "U")) {
+    uint32_t qs[2];
+    if (at<as_int>(p, 0, &n, foreign) && qubit(0, &qs[0]) && qubit(1, &qs[1])) RBK_CALL(A.phase_shift_k(s, n, qs, 2))
+  } else if (!std::strcmp(name, "EY")) {
+    if (real(0, &x) && qubit(0, &a)) RBK_CALL(A.exp_y(s, x, a, none, 0))
+  } else if (!std::strcmp(name, "EZ")) {
+    if (real(0, &x) && qubit(0, &a)) RBK_CALL(A.exp_z(s, x, a, none, 0))
+  } else if (!std::strcmp(name, "EX")) {
+    if (real(0, &x) && qubit(0, &a)) RBK_CALL(A.exp_x(s, x, a, none, 0))
+  } else if (!std::strcmp(name, "SWAP")) {
+    if (qubit(0, &a) && qubit(1, &b)) RBK_CALL(A.swap(s, a, b, none, 0))
+  } else if (!std::strcmp(name, "BEGIN FUSION")) {
+    RBK_CALL(A.begin_fusion(s))
+  } else if (!std::strcmp(name, "END FUSION")) {
+    RBK_CALL(A.end_fusion(s))
+  }
+#undef RBK_CALL
+  return 0;
+}
+
+// apply(state, ops, one): every instruction in order; the first failing call's
+// status code, or 0.  Instructions of the plain form -- a tuple or list of a known
+// mnemonic, qubits and parameters that convert -- go straight to the C ABI; one(op)
+// takes any other.  The handle is read again wherever Python code may have run.
 PyObject* py_apply(PyObject*, PyObject* args)
 {
-  PyObject *handle, *ops;
-  if (!PyArg_ParseTuple(args, "OO", &handle, &ops)) return nullptr;
+  PyObject *state, *ops, *one;
+  if (!PyArg_ParseTuple(args, "OOO", &state, &ops, &one)) return nullptr;
   if (!bound) {
     PyErr_SetString(PyExc_RuntimeError, "entry points not bound");
     return nullptr;
   }
-  rbk_state* s = static_cast<rbk_state*>(PyLong_AsVoidPtr(handle));
-  if (PyErr_Occurred()) return nullptr;
-  PyObject* seq = PySequence_Fast(ops, "instructions must be a sequence");
-  if (!seq) return nullptr;
+  const bool list = plain(ops);
+  const held it(list ? nullptr : PyObject_GetIter(ops));
+  if (!list && !it.o) return nullptr;
+  rbk_state* s = nullptr;
+  bool foreign = true;
   int rc = 0;
-  bool ok = true;
-  for (Py_ssize_t k = 0; ok && rc == 0 && k < PySequence_Fast_GET_SIZE(seq); ++k) {
-    // References are held: a call below runs without the interpreter's lock.
-    const as_sequence held(PySequence_Fast_GET_ITEM(seq, k));
-    PyObject* op = held.o;
-    if (!op || PySequence_Fast_GET_SIZE(op) != 3) {
-      if (op) PyErr_SetString(PyExc_ValueError, "an instruction is (mnemonic, qubits, params)");
-      ok = false;
+  for (Py_ssize_t k = 0; rc == 0; ++k) {
+    PyObject* item = list ? plain_item(ops, k) : PyIter_Next(it.o);
+    if (!item) {
+      if (PyErr_Occurred()) return nullptr;
       break;
     }
-    const as_sequence qubits(item(op, 1)), params(item(op, 2));
-    PyObject *q = qubits.o, *p = params.o;
-    if (!q || !p) {
-      ok = false;
-      break;
-    }
-    const char* name = PyUnicode_Check(item(op, 0)) ? PyUnicode_AsUTF8(item(op, 0)) : nullptr;
-    uint32_t a = 0, b = 0;
-    double x = 0, y = 0, z = 0;
-    int n = 0;
-#define RBK_CALL(expr) { Py_BEGIN_ALLOW_THREADS rc = (expr); Py_END_ALLOW_THREADS }
-    const uint32_t* none = nullptr;
-    if (!name) {
-      PyErr_Clear();
-      PyErr_Format(PyExc_ValueError, "unsupported instruction %S", item(op, 0));
-      ok = false;
-    } else if (!std::strcmp(name, "U3")) {
-      if ((ok = get_real(p, 0, &x) && get_real(p, 1, &y) && get_real(p, 2, &z) && get_qubit(q, 0, &a))) RBK_CALL(A.phase_shift3(s, x, y, z, a, none, 0))
-    } else if (!std::strcmp(name, "CNOT")) {
-      if ((ok = get_qubit(q, 1, &b) && get_qubit(q, 0, &a))) RBK_CALL(A.pauli_x(s, b, &a, 1))
-    } else if (!std::strcmp(name, "H")) {
-      if ((ok = get_qubit(q, 0, &a))) RBK_CALL(A.hadamard(s, a, none, 0))
-    } else if (!std::strcmp(name, "X")) {
-      if ((ok = get_qubit(q, 0, &a))) RBK_CALL(A.pauli_x(s, a, none, 0))
-    } else if (!std::strcmp(name, "Y")) {
-      if ((ok = get_qubit(q, 0, &a))) RBK_CALL(A.pauli_y(s, a, none, 0))
-    } else if (!std::strcmp(name, "Z")) {
-      if ((ok = get_qubit(q, 0, &a))) RBK_CALL(A.pauli_z(s, &a, 1))
-    } else if (!std::strcmp(name, "U1")) {
-      if ((ok = get_real(p, 0, &x) && get_qubit(q, 0, &a))) RBK_CALL(A.phase_shift(s, x, &a, 1))
-    } else if (!std::strcmp(name, "U2")) {
-      if ((ok = get_real(p, 0, &x) && get_real(p, 1, &y) && get_qubit(q, 0, &a))) RBK_CALL(A.phase_shift2(s, x, y, a, none, 0))
-    } else if (!std::strcmp(name, "CZ")) {
-      uint32_t qs[2];
-      if ((ok = get_qubit(q, 0, &qs[0]) && get_qubit(q, 1, &qs[1]))) RBK_CALL(A.pauli_z(s, qs, 2))
-    } else if (!std::strcmp(name, "U")) {
-      uint32_t qs[2];
-      if ((ok = get_int(p, 0, &n) && get_qubit(q, 0, &qs[0]) && get_qubit(q, 1, &qs[1]))) RBK_CALL(A.phase_shift_k(s, n, qs, 2))
-    } else if (!std::strcmp(name, "EY")) {
-      if ((ok = get_real(p, 0, &x) && get_qubit(q, 0, &a))) RBK_CALL(A.exp_y(s, x, a, none, 0))
-    } else if (!std::strcmp(name, "EZ")) {
-      if ((ok = get_real(p, 0, &x) && get_qubit(q, 0, &a))) RBK_CALL(A.exp_z(s, x, a, none, 0))
-    } else if (!std::strcmp(name, "EX")) {
-      if ((ok = get_real(p, 0, &x) && get_qubit(q, 0, &a))) RBK_CALL(A.exp_x(s, x, a, none, 0))
-    } else if (!std::strcmp(name, "SWAP")) {
-      if ((ok = get_qubit(q, 0, &a) && get_qubit(q, 1, &b))) RBK_CALL(A.swap(s, a, b, none, 0))
-    } else if (!std::strcmp(name, "BEGIN FUSION")) {
-      RBK_CALL(A.begin_fusion(s))
-    } else if (!std::strcmp(name, "END FUSION")) {
-      RBK_CALL(A.end_fusion(s))
-    } else {
-      PyErr_Format(PyExc_ValueError, "unsupported instruction %s", name);
-      ok = false;
-    }
-#undef RBK_CALL
+    if (list) Py_INCREF(item);
+    const held op(item);  // held: a call below runs without the interpreter's lock
+    if (!list) foreign = true;
+    if (foreign && !handle_of(state, &s)) return nullptr;
+    foreign = false;
+    if (s && apply_plain(state, s, op.o, &rc, &foreign)) continue;
+    if (hard_error()) return nullptr;
+    const held r(PyObject_CallOneArg(one, op.o));
+    if (!r.o) return nullptr;
+    foreign = true;
   }
-  Py_DECREF(seq);
-  return ok ? PyLong_FromLong(rc) : nullptr;
+  return PyLong_FromLong(rc);
 }
 
-// fill_gates(address, spec, kinds): spec's (mnemonic, qubits, param, scale, angles)
-// as rbk_circuit_gate records at `address` (room for len(spec)); kinds: {mnemonic: code}.
+// x[:n] as Python slices it: a tuple or list of which the first n items count.  A new reference.
+inline PyObject* first_of(PyObject* x, Py_ssize_t n)
+{
+  if (plain(x)) return Py_NewRef(x);
+  const held part(PySequence_GetSlice(x, 0, n));
+  return part.o ? PySequence_Tuple(part.o) : nullptr;
+}
+
+// One gate of the plain form in *r; false otherwise.
+bool gate_plain(PyObject* g, PyObject* kinds, rbk_circuit_gate* r)
+{
+  if (!plain(g) || plain_size(g) != 5) return false;
+  const held name(Py_NewRef(plain_item(g, 0))), q_o(Py_NewRef(plain_item(g, 1))), param(Py_NewRef(plain_item(g, 2))),
+    scale(Py_NewRef(plain_item(g, 3))), angles_o(Py_NewRef(plain_item(g, 4)));
+  PyObject* kind = PyDict_GetItemWithError(kinds, name.o);
+  if (!kind) return false;
+  std::memset(r, 0, sizeof(*r));
+  bool foreign = false;
+  int v = 0;
+  if (!as_int(kind, &v, &foreign)) return false;
+  r->kind = v;
+  const held q(first_of(q_o.o, 2));
+  if (!q.o) return false;
+  for (Py_ssize_t j = 0; j < 2 && j < plain_size(q.o); ++j) {
+    if (!at<as_int>(q.o, j, &v, &foreign)) return false;
+    r->qubits[j] = v;
+  }
+  r->param = -1;
+  if (param.o != Py_None) {
+    if (!as_int(param.o, &v, &foreign)) return false;
+    r->param = v;
+  }
+  if (!as_float(scale.o, &r->scale, &foreign)) return false;
+  const held angles(first_of(angles_o.o, 3));
+  if (!angles.o) return false;
+  for (Py_ssize_t j = 0; j < 3 && j < plain_size(angles.o); ++j)
+    if (!at<as_float>(angles.o, j, &r->angles[j], &foreign)) return false;
+  return true;
+}
+
+// fill_gates(address, count, spec, kinds, one): spec's (mnemonic, qubits, param, scale,
+// angles) as rbk_circuit_gate records at `address`, where `count` have room; kinds:
+// {mnemonic: code}.  one(i, gate) takes gates that are not of the plain form, and
+// any past the room.
 PyObject* py_fill_gates(PyObject*, PyObject* args)
 {
-  PyObject *address, *spec, *kinds;
-  if (!PyArg_ParseTuple(args, "OOO!", &address, &spec, &PyDict_Type, &kinds)) return nullptr;
+  PyObject *address, *spec, *kinds, *one;
+  Py_ssize_t count;
+  if (!PyArg_ParseTuple(args, "OnOO!O", &address, &count, &spec, &PyDict_Type, &kinds, &one)) return nullptr;
   rbk_circuit_gate* out = static_cast<rbk_circuit_gate*>(PyLong_AsVoidPtr(address));
   if (PyErr_Occurred()) return nullptr;
-  PyObject* seq = PySequence_Fast(spec, "a circuit must be a sequence");
-  if (!seq) return nullptr;
-  for (Py_ssize_t k = 0; k < PySequence_Fast_GET_SIZE(seq); ++k) {
-    const as_sequence held(PySequence_Fast_GET_ITEM(seq, k));
-    PyObject* g = held.o;
-    if (!g || PySequence_Fast_GET_SIZE(g) != 5) {
-      if (g) PyErr_SetString(PyExc_ValueError, "a gate is (mnemonic, qubits, param, scale, angles)");
+  const bool list = plain(spec);
+  const held it(list ? nullptr : PyObject_GetIter(spec));
+  if (!list && !it.o) return nullptr;
+  for (Py_ssize_t k = 0;; ++k) {
+    PyObject* item = list ? plain_item(spec, k) : PyIter_Next(it.o);
+    if (!item) {
+      if (PyErr_Occurred()) return nullptr;
       break;
     }
+    if (list) Py_INCREF(item);
+    const held g(item);
     rbk_circuit_gate r;
-    std::memset(&r, 0, sizeof(r));
-    PyObject* kind = PyDict_GetItemWithError(kinds, item(g, 0));
-    if (!kind) {
-      if (!PyErr_Occurred()) PyErr_SetObject(PyExc_KeyError, item(g, 0));
-      break;
+    if (k < count && gate_plain(g.o, kinds, &r)) {
+      out[k] = r;
+      continue;
     }
-    r.kind = static_cast<int32_t>(PyLong_AsLong(kind));
-    const as_sequence qubits(item(g, 1)), turns(item(g, 4));
-    PyObject *q = qubits.o, *angles = turns.o;
-    if (!q || !angles) break;
-    int v = 0;
-    bool ok = true;
-    for (Py_ssize_t j = 0; ok && j < 2 && j < PySequence_Fast_GET_SIZE(q); ++j)
-      if ((ok = get_int(q, j, &v))) r.qubits[j] = v;
-    r.param = -1;
-    if (ok && item(g, 2) != Py_None && (ok = get_int(g, 2, &v))) r.param = v;
-    ok = ok && get_float(g, 3, &r.scale);
-    for (Py_ssize_t j = 0; ok && j < 3 && j < PySequence_Fast_GET_SIZE(angles); ++j) ok = get_float(angles, j, &r.angles[j]);
-    if (!ok) break;
-    out[k] = r;
+    if (hard_error()) return nullptr;
+    const held index(PyLong_FromSsize_t(k));
+    if (!index.o) return nullptr;
+    const held done(PyObject_CallFunctionObjArgs(one, index.o, g.o, nullptr));
+    if (!done.o) return nullptr;
   }
-  Py_DECREF(seq);
-  if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }
 
 PyMethodDef methods[] = {
   {"bind", py_bind, METH_VARARGS, "bind(addresses): the C ABI's entry points"},
-  {"apply", py_apply, METH_VARARGS, "apply(state, ops): status code of the first failing call, or 0"},
-  {"fill_gates", py_fill_gates, METH_VARARGS, "fill_gates(address, spec, kinds)"},
+  {"apply", py_apply, METH_VARARGS, "apply(state, ops, one): status code of the first failing call, or 0"},
+  {"fill_gates", py_fill_gates, METH_VARARGS, "fill_gates(address, count, spec, kinds, one)"},
   {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_marshal", "Argument conversion of the binding", -1, methods, nullptr, nullptr, nullptr, nullptr};

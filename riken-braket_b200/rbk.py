@@ -341,43 +341,47 @@ class State:
     def apply(self, ops):
         """Applies bra instruction tuples (see circuits.py)."""
         if type(self) is State and marshal():  # a subclass may have its own gate methods
-            _check(_native.apply(self.h.value, ops if isinstance(ops, (list, tuple)) else list(ops)))
+            _check(_native.apply(self, ops, self._apply_one))
             return
-        for mnem, q, p in ops:
-            if mnem == "H":
-                self.hadamard(q[0])
-            elif mnem == "X":
-                self.pauli_x(q[0])
-            elif mnem == "Y":
-                self.pauli_y(q[0])
-            elif mnem == "Z":
-                self.pauli_z(q[0])
-            elif mnem == "U1":
-                self.phase_shift(p[0], q[0])
-            elif mnem == "U2":
-                self.u2(p[0], p[1], q[0])
-            elif mnem == "U3":
-                self.u3(p[0], p[1], p[2], q[0])
-            elif mnem == "CNOT":
-                self.pauli_x(q[1], controls=(q[0],))
-            elif mnem == "CZ":
-                self.pauli_z(q[0], q[1])
-            elif mnem == "U":
-                self.controlled_phase_shift_k(int(p[0]), q[0], q[1])
-            elif mnem == "EY":
-                self.exponential_pauli_y(p[0], q[0])
-            elif mnem == "EZ":
-                self.exponential_pauli_z(p[0], q[0])
-            elif mnem == "EX":
-                self.exponential_pauli_x(p[0], q[0])
-            elif mnem == "SWAP":
-                self.swap(q[0], q[1])
-            elif mnem == "BEGIN FUSION":
-                self.begin_fusion()
-            elif mnem == "END FUSION":
-                self.end_fusion()
-            else:
-                raise ValueError(f"unsupported instruction {mnem}")
+        for op in ops:
+            self._apply_one(op)
+
+    def _apply_one(self, op):
+        mnem, q, p = op
+        if mnem == "H":
+            self.hadamard(q[0])
+        elif mnem == "X":
+            self.pauli_x(q[0])
+        elif mnem == "Y":
+            self.pauli_y(q[0])
+        elif mnem == "Z":
+            self.pauli_z(q[0])
+        elif mnem == "U1":
+            self.phase_shift(p[0], q[0])
+        elif mnem == "U2":
+            self.u2(p[0], p[1], q[0])
+        elif mnem == "U3":
+            self.u3(p[0], p[1], p[2], q[0])
+        elif mnem == "CNOT":
+            self.pauli_x(q[1], controls=(q[0],))
+        elif mnem == "CZ":
+            self.pauli_z(q[0], q[1])
+        elif mnem == "U":
+            self.controlled_phase_shift_k(int(p[0]), q[0], q[1])
+        elif mnem == "EY":
+            self.exponential_pauli_y(p[0], q[0])
+        elif mnem == "EZ":
+            self.exponential_pauli_z(p[0], q[0])
+        elif mnem == "EX":
+            self.exponential_pauli_x(p[0], q[0])
+        elif mnem == "SWAP":
+            self.swap(q[0], q[1])
+        elif mnem == "BEGIN FUSION":
+            self.begin_fusion()
+        elif mnem == "END FUSION":
+            self.end_fusion()
+        else:
+            raise ValueError(f"unsupported instruction {mnem}")
 
     # -- further gate families ---------------------------------------------
     def x_rotation_half_pi(self, t, controls=(), adjoint=False):
