@@ -116,6 +116,18 @@ int record_small(rbk_batch* b)
   return b->set.fetch(b->stream);
 }
 
+// Whether the engine's sweep refuses what the planned instance asks for
+// (rbk_adjoint_gradient: phase exponents above n, more than 128 strings or 64 flip
+// patterns).
+bool sweep_refuses(const rbk_batch_instance& I, const rbk::sa_program& P)
+{
+  for (int k = 0; k < I.num_gates; ++k)
+    if (I.gates[k].kind == RBK_GATE_U && std::abs(I.gates[k].angles[0]) >= I.num_qubits + 1) return true;
+  int flips = P.terms.empty() ? 0 : 1;
+  for (size_t t = 1; t < P.terms.size(); ++t) flips += P.terms[t].flip != P.terms[t - 1].flip ? 1 : 0;
+  return P.terms.size() > static_cast<size_t>(rbk::kMaxSumTerms) || flips > rbk::kMaxSumGroups;
+}
+
 int sync_bounded(cudaStream_t s)
 {
   const char* env = std::getenv("RBK_TIMEOUT_S");
@@ -230,8 +242,13 @@ extern "C" int rbk_batch_create(int precision, int device, int num_instances, co
         continue;
       }
       b->programs.emplace_back();
-      if (!rbk::sa_plan(I.num_qubits, I.gates, I.num_gates, I.num_terms, I.strings, I.coeffs, b->programs.back()))
-        return fail(RBK_ERR_INVALID, "Pauli strings use the characters I, X, Y, Z");
+      const bool planned = rbk::sa_plan(I.num_qubits, I.gates, I.num_gates, I.num_terms, I.strings, I.coeffs, b->programs.back());
+      if (!planned && I.num_qubits <= small_limit) return fail(RBK_ERR_INVALID, "Pauli strings use the characters I, X, Y, Z");
+      if (I.num_qubits > small_limit && (!planned || sweep_refuses(I, b->programs.back()))) {
+        b->programs.pop_back();  // the sweep refuses it when the batch runs
+        b->large.push_back(i);
+        continue;
+      }
       b->programs.back().theta_begin = b->param_begin.back();
       b->set_index.push_back(i);
       ++(I.num_qubits <= small_limit ? b->stats.num_small : b->stats.num_large);
