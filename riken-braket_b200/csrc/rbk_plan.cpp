@@ -375,13 +375,11 @@ void fold_trailing_x(const plan_params& p, dev_pass& out, dev_phase& dp, int& op
 // the products once, instead of running every gate over the registers.
 // The members are rewritten in the run's own form: all the gate's bits in
 // creg / cthr / cout (controls and target alike), the factor in (m[2], m[3]).
-// They are sorted by accumulator -- no register bit, register bit 0, ..., R-1,
-// then two or more register bits -- and the header's dout holds the class sizes,
-// one byte each in that order (the last class takes the rest of `run`).  The
-// kernel's accumulators go by the register bits beyond those that all members
-// share (the header's creg): the class sizes by these, in the same order, are
-// the bytes of the header's m[0], and the rest of the run multiplies amplitudes
-// directly.  The gates of a run commute, so their order is free.
+// They are sorted by accumulator, which goes by the register bits beyond those
+// that all members share (the header's creg): none, register bit 0, ..., R-1, then
+// two or more.  The bytes of the header's m[0] are the class sizes in that order;
+// the rest of the run multiplies amplitudes directly.  The gates of a run commute,
+// so their order is free.
 // A diagonal gate diag(d0, d1) with d0 != 1 (EZ: d0 = e^{i theta}) joins a run
 // as two members: d0 on its controls alone (an empty condition: every
 // amplitude) and d1 / d0 on its controls and target.  Members with the same
@@ -467,32 +465,23 @@ void group_phase_runs(const plan_params& p, dev_pass& out, dev_phase& dp, int& o
       }
     }
     if (j - i >= shortest && headers_left > 0 && !members.empty()) {
-      auto cls = [&](const dev_op& g) {
-        const int c = __builtin_popcount(g.creg);
-        return c == 0 ? 0 : c == 1 ? 1 + __builtin_ctz(g.creg) : 1 + p.R;
-      };
       // Register bits of every member (the QFT's phases behind one Hadamard share
       // its qubit), and the class by the others: none, one, or several.
       uint32_t common = (1u << p.R) - 1;
       for (const dev_op& g : members) common &= g.creg;
-      auto sub = [&](const dev_op& g) {
+      auto cls = [&](const dev_op& g) {
         const uint32_t rest = g.creg & ~common;
         const int c = __builtin_popcount(rest);
         return c == 0 ? 0 : c == 1 ? 1 + __builtin_ctz(rest) : 1 + p.R;
       };
-      std::stable_sort(members.begin(), members.end(), [&](const dev_op& x, const dev_op& y) {
-        return cls(x) != cls(y) ? cls(x) < cls(y) : sub(x) < sub(y);
-      });
+      std::stable_sort(members.begin(), members.end(), [&](const dev_op& x, const dev_op& y) { return cls(x) < cls(y); });
       dev_op h{};
       h.kind = OPK_PHASES;
       h.run = static_cast<uint32_t>(members.size());
       h.code = op_code(OPK_PHASES, 0, true, 0);
       uint64_t sizes = 0;
-      for (const dev_op& g : members) {
-        const int c = cls(g), c2 = sub(g);
-        if (c <= p.R) h.dout += 1ull << (8 * c);
-        if (c2 <= p.R) sizes += 1ull << (8 * c2);
-      }
+      for (const dev_op& g : members)
+        if (const int c = cls(g); c <= p.R) sizes += 1ull << (8 * c);
       h.creg = common;
       std::memcpy(&h.m[0], &sizes, sizeof(sizes));
       grouped.push_back(h);

@@ -150,24 +150,45 @@ static void run_pass(std::vector<cplx>& st, const plan_params& p, const dev_pass
           if (op.code != want_code || op.code >= kNumOpCodes || op.treg >= R) { std::fprintf(stderr, "bad dispatch code\n"); std::exit(8); }
           if (op.kind == OPK_PHASES) {  // a run header: the run's gates follow, each a factor on the amplitudes whose bits are all one
             if (op.run < 1 || o + static_cast<int>(op.run) >= D.op_end) { std::fprintf(stderr, "bad phase run\n"); std::exit(14); }
-            // class sizes (no register bit, register bit 0 .. R-1; the rest: two or more register bits)
+            // As the kernel runs it: the class sizes in m[0] (no register bit beyond the common ones of
+            // the header, register bit 0 .. R-1; the rest: two or more) choose the accumulator, and
+            // each amplitude that has the common bits takes the product of its accumulators.
+            uint64_t sizes;
+            std::memcpy(&sizes, &op.m[0], sizeof(sizes));
             int bound[9], sum = 0;
-            for (int c = 0; c <= R; ++c) { sum += static_cast<int>((op.dout >> (8 * c)) & 0xff); bound[c] = sum; }
-            if (sum > static_cast<int>(op.run) || (op.dout >> (8 * (R + 1))) != 0) { std::fprintf(stderr, "bad phase run classes\n"); std::exit(18); }
+            for (int c = 0; c <= R; ++c) { sum += static_cast<int>((sizes >> (8 * c)) & 0xff); bound[c] = sum; }
+            if (sum > static_cast<int>(op.run) || (sizes >> (8 * (R + 1))) != 0 || op.creg >= (1u << R) || op.cthr || op.cout ||
+                op.dreg || op.dthr || op.dout) {
+              std::fprintf(stderr, "bad phase run classes\n");
+              std::exit(18);
+            }
+            cplx all{1.0, 0.0}, by[8];
+            for (int c = 0; c < R; ++c) by[c] = all;
             for (int k = 1; k <= static_cast<int>(op.run); ++k) {
               const dev_op& g = P.ops[o + k];
               int c = 0;
               while (c <= R && k - 1 >= bound[c]) ++c;  // the class member k - 1 belongs to
-              const int nr = __builtin_popcount(g.creg);
-              const bool ok_class = c == 0 ? nr == 0 : c <= R ? g.creg == (1u << (c - 1)) : nr >= 2;
-              if (g.kind != OPK_DIAG || g.dreg || g.dthr || g.dout || g.creg >= (1u << R) || !ok_class) {
+              const uint32_t rest = g.creg & ~op.creg;
+              const int nr = __builtin_popcount(rest);
+              const bool ok_class = c == 0 ? nr == 0 : c <= R ? rest == (1u << (c - 1)) : nr >= 2;
+              if (g.kind != OPK_DIAG || g.dreg || g.dthr || g.dout || g.creg >= (1u << R) || (g.creg & op.creg) != op.creg || !ok_class) {
                 std::fprintf(stderr, "phase run holds a gate out of its form or class\n");
                 std::exit(15);
               }
               if ((uint32_t(tid) & g.cthr) != g.cthr || (base & g.cout) != g.cout) continue;
               const cplx d{g.m[2], g.m[3]};
-              for (int i = 0; i < NR; ++i)
-                if ((uint32_t(i) & g.creg) == g.creg) a[i] *= d;
+              if (c == 0) all *= d;
+              else if (c <= R) by[c - 1] *= d;
+              else
+                for (int i = 0; i < NR; ++i)
+                  if ((uint32_t(i) & g.creg) == g.creg) a[i] *= d;
+            }
+            for (int i = 0; i < NR; ++i) {
+              if ((uint32_t(i) & op.creg) != op.creg) continue;
+              cplx f = all;
+              for (int b = 0; b < R; ++b)
+                if (((i & ~op.creg) >> b) & 1) f *= by[b];
+              a[i] *= f;
             }
             o += static_cast<int>(op.run);
             continue;
