@@ -49,3 +49,48 @@ def test_small_states_vs_oracle(pkg, precision, n):
             s.apply(ops)
             assert np.abs(s.spins() - o.spins()).max() <= tol
             assert np.abs(s.amplitudes().astype(np.complex128) - o.amplitudes()).max() <= tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,n", [(p, n) for p in (0, 1) for n in (1, 2, 3, 4, 9, 10, 11, 12)])
+def test_one_phase_programs_vs_oracle(pkg, precision, n):
+    """One register phase of 1 to 9 gates: up to 8 run straight from HBM, 9 through shared memory.
+    Targets on at most three qubits, controls and phases on any; tolerances as above."""
+    import oracle
+
+    tol = 1e-12 if precision == 0 else 2e-5
+    rng = np.random.default_rng(50 + n)
+    init = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    init /= np.linalg.norm(init)
+    for count in (1, 2, 7, 8, 9):
+        for _ in range(6):
+            targets = [int(q) for q in rng.permutation(n)[:3]]
+            ops = []
+            for _ in range(count):
+                t, c = targets[int(rng.integers(len(targets)))], int(rng.integers(n))
+                x = [float(v) for v in rng.uniform(-3, 3, 3)]
+                pick = int(rng.integers(9))
+                ops.append([("U3", (t,), tuple(x)), ("H", (t,), ()), ("Y", (t,), ()), ("EY", (t,), (x[0],)), ("U1", (c,), (x[0],)),
+                            ("Z", (c,), ()), ("EZ", (c,), (x[0],)), ("CNOT", (c, t), ()) if c != t else ("X", (t,), ()),
+                            ("CZ", (c, t), ()) if c != t else ("X", (t,), ())][pick])
+            o = oracle.COracle(n)
+            o.set_amplitudes(init)
+            o.apply(ops)
+            with pkg.State(n, precision) as s:
+                s.upload(init)
+                s.apply(ops)
+                assert np.abs(s.amplitudes().astype(np.complex128) - o.amplitudes()).max() <= tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 11, 12, 13])
+def test_gates_launched_one_by_one_vs_oracle(pkg, n):
+    import oracle
+
+    ops = pkg.circuits.random_circuit(n, 60, seed=n)
+    o = oracle.COracle(n)
+    o.apply(ops)
+    with pkg.State(n) as s:
+        s.set_deferred(False)
+        s.apply(ops)
+        assert np.abs(s.amplitudes() - o.amplitudes()).max() <= 1e-12
