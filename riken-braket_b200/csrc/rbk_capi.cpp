@@ -525,7 +525,7 @@ int observe_all(rbk_state* s, uint64_t flips, bool z, const std::vector<diag_ter
   if (int rc = flush(s)) return rc;  // the layout map is final only after the queued gates ran
   const bool c128 = s->precision == RBK_C128;
   const int n = s->n, RB = rbk::kObserveRegBits, KT = rbk::kObserveTileBits;
-  if (n < KT) {
+  if (n < KT || (n <= rbk::kObserveSmallBits && diag.size() <= size_t(rbk::kMaxPauliTerms))) {
     for (size_t first = 0; first == 0 || first < diag.size(); first += rbk::kMaxPauliTerms) {
       rbk::pauli_terms t{};
       for (size_t k = first; k < diag.size() && t.count < rbk::kMaxPauliTerms; ++k) {

@@ -607,51 +607,51 @@ observe_kernel(const typename ctype<Real>::c* __restrict__ a, int n, const __gri
   }
 }
 
-// launch_observe_small: the state in shared memory, one warp per output, no
-// partial sums and no second launch.
-constexpr int kSmallThreads = 512;
+// launch_observe_small: one block per sum, each reading the state from L2, no
+// partial sums and no second launch.  The sums of a state in one CTA's shared
+// memory, a warp for each, took two rounds of 16 warps and ended at 11 qubits; with
+// two observe_kernel launches spins of 12 qubits in complex<float> took 44.8 us,
+// 31 here (35 with one tile of 2^12 amplitudes); energies of 11 and fewer gain too.
+constexpr int kSmallThreads = 256;
 template <typename Real>
 __global__ void __launch_bounds__(kSmallThreads)
 observe_small_kernel(const typename ctype<Real>::c* __restrict__ a, int n, const __grid_constant__ pauli_terms T,
                      double* __restrict__ out)
 {
-  using C = typename ctype<Real>::c;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* s = reinterpret_cast<C*>(smem_raw);
   const uint32_t size = 1u << n;
-  for (uint32_t i = threadIdx.x; i < size; i += blockDim.x) s[i] = a[i];
+  const int w = blockIdx.x;
+  double v[2] = {0.0, 0.0};
+  if (w < n) {  // x_b of bit b = w
+    for (uint32_t k = threadIdx.x; k < size / 2; k += kSmallThreads) {
+      const uint32_t i = uint32_t(insert_zero(k, w));
+      const auto x = a[i], y = a[i | (1u << w)];
+      v[0] += double(x.x) * double(y.x) + double(x.y) * double(y.y);
+      v[1] += double(x.x) * double(y.y) - double(x.y) * double(y.x);
+    }
+  } else {  // the plain sum (n), the sum over bit b set (n + 1 + b), the diagonal strings (2 n + 1)
+    const uint32_t need = w > n && w <= 2 * n ? 1u << (w - n - 1) : 0u;
+    for (uint32_t i = threadIdx.x; i < size; i += kSmallThreads) {
+      if ((i & need) != need) continue;
+      const auto x = a[i];
+      const double p = double(x.x) * double(x.x) + double(x.y) * double(x.y);
+      double f = 1.0;
+      if (w == 2 * n + 1) {
+        f = 0.0;
+        for (int t = 0; t < T.count; ++t) f += (__popc(i & uint32_t(T.sign[t])) & 1) ? -T.w[t][0] : T.w[t][0];
+      }
+      v[0] += p * f;
+    }
+  }
+  __shared__ double red[kSmallThreads / 32][2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double re = warp_sum(v[0]), im = warp_sum(v[1]);
+  if (lane == 0) { red[warp][0] = re; red[warp][1] = im; }
   __syncthreads();
-  const uint32_t lane = threadIdx.x & 31;
-  const int warps = kSmallThreads / 32;
-  // Work items: x_b of bit b (item b), the plain sum (item n), the sum over bit b set (n + 1 + b), the diagonal strings.
-  for (int w = threadIdx.x >> 5; w < 2 * n + 2; w += warps) {
-    double re = 0.0, im = 0.0;
-    if (w < n) {
-      for (uint32_t v = lane; v < size / 2; v += 32) {
-        const uint32_t i = uint32_t(insert_zero(v, w));
-        const C x = s[i], y = s[i | (1u << w)];
-        re += double(x.x) * double(y.x) + double(x.y) * double(y.y);
-        im += double(x.x) * double(y.y) - double(x.y) * double(y.x);
-      }
-    } else {
-      const uint32_t need = w > n && w <= 2 * n ? 1u << (w - n - 1) : 0u;
-      for (uint32_t i = lane; i < size; i += 32) {
-        if ((i & need) != need) continue;
-        const double p = double(s[i].x) * double(s[i].x) + double(s[i].y) * double(s[i].y);
-        double f = 1.0;
-        if (w == 2 * n + 1) {
-          f = 0.0;
-          for (int t = 0; t < T.count; ++t) f += (__popc(i & uint32_t(T.sign[t])) & 1) ? -T.w[t][0] : T.w[t][0];
-        }
-        re += p * f;
-      }
-    }
-    re = warp_sum(re);
-    im = warp_sum(im);
-    if (lane == 0) {
-      if (w < n) { out[2 * w] = re; out[2 * w + 1] = im; }
-      else out[n + w] = re;
-    }
+  if (threadIdx.x < 2) {
+    double s = 0.0;
+    for (int k = 0; k < kSmallThreads / 32; ++k) s += red[k][threadIdx.x];
+    if (w < n) out[2 * w + threadIdx.x] = s;
+    else if (threadIdx.x == 0) out[n + w] = s;
   }
 }
 
@@ -785,8 +785,8 @@ cudaError_t launch_observe(const void* state, int n, const observe_group& g, dou
 template <typename Real>
 cudaError_t launch_observe_small(const void* state, int n, const pauli_terms& terms, double* out, cudaStream_t stream)
 {
-  if (n < 1 || n >= 8 + observe_shape::RB || terms.count < 0 || terms.count > kMaxPauliTerms) return cudaErrorInvalidValue;
-  observe_small_kernel<Real><<<1, kSmallThreads, sizeof(typename ctype<Real>::c) << n, stream>>>(
+  if (n < 1 || n > kObserveSmallBits || terms.count < 0 || terms.count > kMaxPauliTerms) return cudaErrorInvalidValue;
+  observe_small_kernel<Real><<<2 * n + 2, kSmallThreads, 0, stream>>>(
     static_cast<const typename ctype<Real>::c*>(state), n, terms, out);
   return cudaGetLastError();
 }

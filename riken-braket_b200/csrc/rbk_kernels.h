@@ -134,8 +134,9 @@ struct observe_group {
 int observe_width(const observe_group& g, int n);
 template <typename Real> cudaError_t launch_observe(const void* state, int n, const observe_group& g, double* partials, double* out,
                                                     cudaStream_t stream);
-// The same for a state smaller than the tile (n < kObserveTileBits), in one CTA: every x_b, the
+// The same for a small state (n <= kObserveSmallBits), in one launch: every x_b, the
 // 1 + n sums of |a_j|^2, and the diagonal sum of `terms` (real weights), in that order.
+constexpr int kObserveSmallBits = 12;
 template <typename Real> cudaError_t launch_observe_small(const void* state, int n, const pauli_terms& terms, double* out,
                                                           cudaStream_t stream);
 

@@ -46,3 +46,19 @@ def test_expectation_and_spins_vs_numpy(pkg, precision, n):
         assert abs(s.expectation(terms[:n]) - sum(c * pauli_value(wide, t) for t, c in terms[:n])) <= 1e-13 * scale
         spins = np.array([[0.5 * pauli_value(wide, one(c, q)).real for c in "XYZ"] for q in range(n)])
         assert np.abs(s.spins() - spins).max() <= 1e-13
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n,count", [(11, 64), (12, 1), (12, 63), (12, 64), (12, 65), (13, 64)])
+def test_diagonal_strings_around_the_small_launch(pkg, precision, n, count):
+    """The sizes and numbers of strings where one launch for a small state ends."""
+    rng = np.random.default_rng(7 * n + count)
+    a = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    a = (a / np.linalg.norm(a)).astype(np.complex128 if precision == 0 else np.complex64)
+    wide = a.astype(np.complex128)
+    strings = {"".join(rng.choice(list("IZ"), n)) for _ in range(2 * count)}
+    terms = [(t, float(w)) for t, w in zip(sorted(strings)[:count], rng.standard_normal(count))]
+    with pkg.State(n, precision) as s:
+        s.upload(a)
+        want = sum(c * pauli_value(wide, t) for t, c in terms)
+        assert abs(s.expectation(terms) - want) <= 1e-13 * sum(abs(c) for _, c in terms) * float(np.vdot(wide, wide).real)
