@@ -30,6 +30,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <set>
 #include <string>
 #include <thread>
 #include <vector>
@@ -269,12 +270,17 @@ extern "C" int rbk_batch_create(int precision, int device, int num_instances, co
     b->stats.num_large += static_cast<int>(b->large.size());
     if (!b->programs.empty()) {
       b->d_theta.reset(dalloc<double>(np));
-      for (int k = 0; k + 1 < rbk::sa_set::kClasses; ++k) {
+      // A side stream for each size class after the first, and an event more.  Those of
+      // all six classes whatever the sizes made creating a batch of one class 1 ms longer
+      // (four instances of 12 qubits: 5.4 ms, now 4.5 to 4.9).
+      std::set<int> classes;
+      for (const auto& P : b->programs) classes.insert(rbk::sa_set::size_class(P.n));
+      for (size_t k = 1; k < classes.size(); ++k) {
         cudaStream_t q;
         if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess) return fail(RBK_ERR_CUDA, "stream");
         b->side.push_back(q);
       }
-      for (int k = 0; k < rbk::sa_set::kClasses; ++k) {
+      for (size_t k = 0; k < classes.size(); ++k) {
         cudaEvent_t ev;
         if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return fail(RBK_ERR_CUDA, "event");
         b->events.push_back(ev);

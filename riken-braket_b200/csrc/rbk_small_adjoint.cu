@@ -34,7 +34,6 @@ constexpr int kSaPhaseOps = 48;  // ops of one phase, staged in shared memory tw
 constexpr int kSaPhaseSlots = 8;  // overlaps of one phase: a column of partial sums per thread each, staged twice
 constexpr int kSaRegs = kSmallSlots;
 constexpr int kSaLocalBits = 12;  // amplitudes a CTA holds of each state
-constexpr int kSaClassBits = 10;  // instances of fewer qubits share the launch of this size
 
 struct sa_args {
   const sa_inst* inst;
@@ -602,7 +601,7 @@ int sa_set::assign(int precision, const std::vector<const sa_program*>& programs
     terms += P.terms.size();
     slots_ += I.num_slots;
     // an overlap per CTA, the energy per warp
-    partial += size_t(cluster_of(P.n)) * (size_t(I.num_slots) + size_t(threads_of(std::max(kSaClassBits, P.n), kSaThreads) / 32));
+    partial += size_t(cluster_of(P.n)) * (size_t(I.num_slots) + size_t(threads_of(size_class(P.n), kSaThreads) / 32));
     insts_.push_back(I);
   }
   if (ops > size_t(INT32_MAX) || terms > size_t(INT32_MAX)) return sa_fail(RBK_ERR_UNSUPPORTED, "batch: too many gates");
@@ -670,12 +669,11 @@ int sa_set::launch(const double* d_theta, int max_threads, cudaStream_t stream, 
   A.partial = d_partial_;
   A.energy = d_out_;
   A.overlaps = d_out_ + insts_.size();
-  // Classes of one launch shape: 15, 14, 13, 12, 11 and at most 10 qubits.
   size_t used = 0;
   for (size_t i = 0; i < insts_.size();) {
-    const int cls = std::max(kSaClassBits, insts_[i].n), n = insts_[i].n;  // the first is the largest of its class
+    const int cls = size_class(insts_[i].n), n = insts_[i].n;  // the first is the largest of its class
     size_t j = i;
-    while (j < insts_.size() && std::max(kSaClassBits, insts_[j].n) == cls) ++j;
+    while (j < insts_.size() && size_class(insts_[j].n) == cls) ++j;
     cudaStream_t on = stream;
     if (i > 0 && used < side.size()) {
       on = side[used];

@@ -65,7 +65,8 @@ public:
   int fetch(cudaStream_t stream);
   const double* energies() const { return h_out_; }
   const double* overlaps(int program) const { return h_out_ + insts_.size() + slot_begin_[static_cast<size_t>(program)]; }
-  static constexpr int kClasses = 6;  // launches of different shape that one set can need
+  // Instances of one size class share a launch: 15, 14, 13, 12, 11 and at most 10 qubits.
+  static int size_class(int n) { return n > 10 ? n : 10; }
 
 private:
   int precision_ = 0, slots_ = 0;
