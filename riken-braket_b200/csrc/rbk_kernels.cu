@@ -2082,7 +2082,8 @@ sample_sums_kernel(const typename ctype<Real>::c* __restrict__ a, uint64_t size,
 constexpr int kSampleScanThreads = 1024;
 __global__ void __launch_bounds__(kSampleScanThreads) sample_scan_kernel(double* __restrict__ v, uint64_t count)
 {
-  __shared__ double warp_tot[kSampleScanThreads / 32], warp_end[kSampleScanThreads / 32];
+  static_assert(kSampleScanThreads == 32 * 32, "a lane for every warp");
+  __shared__ double warp_tot[32], warp_end[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t per = (count + kSampleScanThreads - 1) / kSampleScanThreads;
   const uint64_t lo = min(count, threadIdx.x * per), hi = min(count, lo + per);
@@ -2095,9 +2096,15 @@ __global__ void __launch_bounds__(kSampleScanThreads) sample_scan_kernel(double*
   }
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
-  double off = 0.0;
-  for (int w = 0; w < warp; ++w) off += warp_tot[w];
-  double end = last > lo ? off + incl : 0.0;
+  // Every warp scans the warps' sums (and below their ends): lane w has those of warps 0 .. w.
+  double sums = warp_tot[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, sums, o);
+    if (lane >= o) sums += y;
+  }
+  const double off = __shfl_sync(0xffffffffu, sums, max(warp - 1, 0));
+  double end = last > lo ? (warp > 0 ? off + incl : incl) : 0.0;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const double y = __shfl_up_sync(0xffffffffu, end, o);
@@ -2105,8 +2112,14 @@ __global__ void __launch_bounds__(kSampleScanThreads) sample_scan_kernel(double*
   }
   if (lane == 31) warp_end[warp] = end;
   __syncthreads();
-  double prev = 0.0;
-  for (int w = 0; w < warp; ++w) prev = scan_later(prev, warp_end[w]);
+  double ends = warp_end[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xffffffffu, ends, o);
+    if (lane >= o) ends = scan_later(y, ends);
+  }
+  double prev = __shfl_sync(0xffffffffu, ends, max(warp - 1, 0));
+  if (warp == 0) prev = 0.0;
   const double y = __shfl_up_sync(0xffffffffu, end, 1);
   scan_write(v, lo, hi, last, lane > 0 ? scan_later(prev, y) : prev, scan_later(prev, end));
 }

@@ -22,11 +22,13 @@ static void scan(std::vector<double>& v)
     for (int t = 0; t < kThreads; ++t)
       if ((t & 31) >= o) incl[t] += was[t - o];
   }
-  for (int t = 0; t < kThreads; ++t) {
-    double off = 0.0;
-    for (int w = 0; w < t / 32; ++w) off += incl[32 * w + 31];
-    end[t] = last[t] > lo(t) ? off + incl[t] : 0.0;
+  std::vector<double> sums(32);
+  for (int w = 0; w < 32; ++w) sums[w] = incl[32 * w + 31];
+  for (int o = 1; o < 32; o <<= 1) {
+    const std::vector<double> was(sums);
+    for (int w = o; w < 32; ++w) sums[w] += was[w - o];
   }
+  for (int t = 0; t < kThreads; ++t) end[t] = last[t] > lo(t) ? (t >= 32 ? sums[t / 32 - 1] + incl[t] : incl[t]) : 0.0;
   for (int o = 1; o < 32; o <<= 1) {
     const std::vector<double> was(end);
     for (int t = 0; t < kThreads; ++t)
