@@ -94,6 +94,7 @@ struct rbk_batch {
   ~rbk_batch()
   {
     cudaSetDevice(device);
+    if (stream) cudaStreamSynchronize(stream);  // a call that ended early may have left its launches
     for (auto& pool : pools)
       for (auto& kv : pool) rbk::adjoint_workspace_destroy(kv.second);
     if (exec) cudaGraphExecDestroy(exec);
@@ -398,7 +399,11 @@ extern "C" int rbk_batch_run(rbk_batch* b, const double* theta, double* energies
       for (int t = 1; t < b->workers; ++t) threads.emplace_back(work, t);
       work(0);
       for (auto& t : threads) t.join();
-      if (first_rc.load() != RBK_OK) return fail(first_rc.load(), "batch: " + err);
+      if (first_rc.load() != RBK_OK) {
+        // The launches still read and write the batch's buffers.
+        if (!b->programs.empty()) sync_bounded(b->stream);
+        return fail(first_rc.load(), "batch: " + err);
+      }
     }
     if (!b->programs.empty()) {
       if (int rc = sync_bounded(b->stream)) return rc;
