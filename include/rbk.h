@@ -216,7 +216,8 @@ int rbk_shor_box(rbk_state* s, uint32_t num_exponent_qubits, uint64_t divisor, u
  * the basis index is qubits[i].  complex<float> states with k = 5 or 6
  * (and n >= k + 7) run on the tensor cores as 3xTF32 split-precision GEMMs with
  * FP32 accumulation (tcgen05, accumulator in TMEM); other cases on CUDA cores,
- * with the qubits where they lie.
+ * up to 6 qubits with the qubits where they lie, more after relabelling passes
+ * that move them onto the low physical bits.
  * No counterpart in ket beyond the fused blocks below; k <= 10. */
 int rbk_apply_unitary(rbk_state* s, const double* u, const uint32_t* qubits, int k);
 /* 0 (default): BEGIN/END FUSION blocks run gate by gate inside the fused passes.
@@ -263,7 +264,10 @@ int rbk_state_seed(rbk_state* s, uint64_t seed);
  * ket::generate_events does (ket/include/ket/generate_events.hpp:18-66):
  * uniform_real_distribution(0, total) and upper_bound over the inclusive prefix
  * sums.  seed < 0 uses (and advances) the state's generator; otherwise a fresh
- * generator built from seed.  Unlike the reference, the state is left intact. */
+ * generator built from seed.  Unlike the reference, the state is left intact.
+ * The sums take 2^n / 16 bytes of device memory and each event 16; the state keeps
+ * a workspace of up to 40 MB (29 qubits) until it is destroyed, a larger one is the
+ * call's own.  rbk_measure uses the same. */
 int rbk_generate_events(rbk_state* s, int num_events, int64_t seed, uint64_t* events);
 /* ket::measure (ket/include/ket/measure.hpp:16-46): sample one index with the
  * state's generator; the state becomes that basis state. */
@@ -321,13 +325,14 @@ int rbk_adjoint_gradient(int num_qubits, int precision, int device, const rbk_ci
 /* ---- batches of parametrised circuits (no counterpart in the reference) -----
  * Energies and adjoint gradients of many independent circuits of uneven size,
  * each with its own parameters and observable (same conventions as
- * rbk_adjoint_gradient).  Instances of up to 15 qubits run in
- * one launch per size class, replayed from a CUDA graph, one CTA (n <= 12 in
- * c128, n <= 13 in c64) or one cluster of CTAs per instance with both state
- * vectors in shared memory; the CTA size is chosen by timing the candidates at
- * rbk_batch_create.  Larger instances run through
- * rbk_adjoint_gradient.  Parameters and gradients are concatenated in instance
- * order. */
+ * rbk_adjoint_gradient).  Instances of up to 15 qubits run in one launch per size
+ * class, replayed from a CUDA graph, one CTA (n <= 12) or one cluster of 2, 4 or 8
+ * CTAs per instance with both state vectors in shared memory; the CTA size is
+ * chosen by timing the candidates at rbk_batch_create.  Larger instances run
+ * through rbk_adjoint_gradient.  Above 12 qubits (13 in complex<float>) what
+ * rbk_adjoint_gradient refuses is refused by rbk_batch_run; below there is no limit
+ * on phase exponents, strings and X/Y patterns.  Parameters and gradients are
+ * concatenated in instance order. */
 typedef struct rbk_batch rbk_batch;
 typedef struct rbk_batch_instance {
   int32_t num_qubits;
@@ -339,10 +344,10 @@ typedef struct rbk_batch_instance {
   const double* coeffs;  /* num_terms (re, im) */
 } rbk_batch_instance;
 typedef struct rbk_batch_stats {
-  int num_small;       /* instances in the persistent launch */
-  int num_large;       /* instances through rbk_adjoint_gradient */
+  int num_small;       /* instances of up to 12 qubits (complex<float>: 13) */
+  int num_large;       /* the others: up to 15 qubits in clusters, above through rbk_adjoint_gradient */
   int threads;         /* CTA size picked by the autotuner */
-  float small_ms;      /* device time of the persistent launch when tuned */
+  float small_ms;      /* device time of the launches for up to 15 qubits when tuned */
   double last_run_ms;  /* host wall time of the last rbk_batch_run */
 } rbk_batch_stats;
 int rbk_batch_create(int precision, int device, int num_instances, const rbk_batch_instance* instances, rbk_batch** out);
@@ -357,8 +362,9 @@ int rbk_batch_tuned_shape(const rbk_batch* batch, int num_qubits, int* shape);
 int rbk_batch_destroy(rbk_batch* batch);
 
 /* The same sweep on a context that keeps its two state vectors and buffers
- * between calls (optimiser loops): create once per qubit count and precision,
- * then rbk_adjoint_run with the arguments of rbk_adjoint_gradient. */
+ * between calls (optimiser loops; 8 MB of partial sums beside the states from 11
+ * qubits on): create once per qubit count and precision, then rbk_adjoint_run with
+ * the arguments of rbk_adjoint_gradient. */
 typedef struct rbk_adjoint_ctx rbk_adjoint_ctx;
 int rbk_adjoint_create(int num_qubits, int precision, int device, rbk_adjoint_ctx** out);
 int rbk_adjoint_run(rbk_adjoint_ctx* ctx, const rbk_circuit_gate* gates, int num_gates, const double* theta,

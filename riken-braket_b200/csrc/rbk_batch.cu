@@ -1,12 +1,11 @@
 // rbk_batch.cu -- energies and adjoint gradients of many parametrised circuits
 // of uneven size in one call (rbk_batch_* of include/rbk.h).
 //
-// Instances whose two state vectors fit the shared memory of one CTA (n <= 12
-// for complex<double>, n <= 13 for complex<float>) or of one cluster (up to 15
-// qubits) run in one set of launches (rbk_small_adjoint.cu), one launch per
-// size class on streams of their own, which do the whole job of every instance
-// and are captured with their copies in a CUDA graph that every parameter
-// vector replays.  The CTA size is picked by an autotuner that times the
+// Instances whose two state vectors fit the shared memory of one CTA (up to 12
+// qubits) or of one cluster (up to 15) run in one set of launches
+// (rbk_small_adjoint.cu), one launch per size class on streams of their own, which
+// do the whole job of every instance and are captured with their copies in a CUDA
+// graph that every parameter vector replays.  The CTA size is picked by an autotuner that times the
 // candidates on the batch's own instances.  Larger instances run through the
 // engine's adjoint sweep (rbk_adjoint_gradient) on worker threads, with the
 // fused passes' tile shape (their fusion width) picked per qubit count by a

@@ -1,7 +1,8 @@
 // rbk_small_adjoint.h -- energies and adjoint gradients of circuits whose two
 // state vectors fit the shared memory of one CTA or of one cluster of CTAs.
-// The host plans a circuit once (its register phases do not depend on the
-// parameters); a launch then does the whole job of every instance.
+// The host plans a circuit (its register phases do not depend on the parameters:
+// a batch plans when it is created, a single gradient at every call); a launch then
+// does the whole job of every instance.
 #pragma once
 
 #include <cuda_runtime.h>
