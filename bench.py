@@ -156,6 +156,14 @@ def sample_blocks(ops):
     return out
 
 
+REFERENCE_LIB = os.path.join(ROOT, "oracle", "_ref", "libketref_fast.so")
+
+
+def reference_missing():
+    """Why the reference's release build cannot run here, or None."""
+    return None if os.path.exists(REFERENCE_LIB) else "oracle/_ref/libketref_fast.so is not built (needs the reference's sources)"
+
+
 class CpuReference:
     """The reference's own ket/bra code, release build (oracle/_ref/libketref_fast.so)."""
 
@@ -178,6 +186,8 @@ def cpu_sample(ops, threads, budget_s, n=N_QUBITS):
     sample_blocks() in order (the ones the reference arm's timed steps start
     with), until budget_s of CPU time is spent.  Returns (passes, seconds,
     description)."""
+    if reference_missing():
+        return None, None, reference_missing()
     need = (16 << n) * 1.1
     if host_mem_available() < need:
         return None, None, f"host has {host_mem_available() / 2**30:.0f} GiB free, a {n}-qubit state needs {need / 2**30:.0f} GiB"
@@ -306,7 +316,7 @@ def run_gpu(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_kind,
                      "traffic": traffic.get("bytes_per_launch") if traffic else None,
-                     "kernel": "rbk::tile_pass_kernel<double>"},
+                     "kernel": "rbk::straight_pass_kernel<double>"},
         "cpu_baseline": cpu,
         "e2e": {"value": e2e_value, "unit": "GB/s", "h2d_bytes_per_step": int(e2e_passes * desc_bytes),
                 "d2h_bytes_per_step": 8 * 3 * N_QUBITS, "circuit_ms": e2e_max / args.steps * 1e3,
@@ -399,6 +409,9 @@ def run_reference(args):
     ops = C.brick(N_QUBITS, DEPTH, seed=SEED, fuse_k=FUSE_K)
     bytes_pass = 2 * (1 << N_QUBITS) * 16
     threads = os.cpu_count() or 1
+    if reference_missing():
+        print(json.dumps({"impl": "reference", "unavailable": reference_missing()}))
+        return
     need = (16 << N_QUBITS) * 1.1
     if host_mem_available() < need:
         print(json.dumps({"impl": "reference", "unavailable": f"host RAM: {host_mem_available() / 2**30:.0f} GiB free, "
