@@ -16,6 +16,17 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200); runs through the C ABI of librbk.so")
 
 
+# Modules and tests that fail without the reference's own build.
+NEED_REFERENCE = {"test_gpu_bra_b200", "test_inner_product_pauli_vs_reference", "test_pauliss_hamiltonian_energy_full_precision"}
+
+
+def pytest_collection_modifyitems(items):
+    """Where the reference is not built, the tests that need it run after all others,
+    so that a run that stops at its first failure has run those."""
+    if not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libketref.so")):
+        items.sort(key=lambda i: i.module.__name__ in NEED_REFERENCE or getattr(i, "originalname", "") in NEED_REFERENCE)
+
+
 @pytest.fixture(scope="session")
 def pkg():
     return load_package()
